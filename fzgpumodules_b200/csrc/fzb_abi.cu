@@ -520,9 +520,7 @@ int fzb_rze_decode(const void* d_in, uint64_t in_bytes, uint64_t orig_bytes, voi
     a.orig_bytes = (uint32_t)orig_bytes;
     a.bytes_out = static_cast<uint8_t*>(d_out);
     a.err = w.err;
-    const int smem = kChunkBytes * 2 + 16 + 2048 + 256 + 32;
-    CK(cudaFuncSetAttribute(rze_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    rze_decode_kernel<<<(unsigned)nch, kThreads, smem, s>>>(a);
+    rze_decode_kernel<<<(unsigned)nch, kThreads, 0, s>>>(a);
     CK(cudaGetLastError());
     return FZB_OK;
 }
@@ -577,9 +575,6 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
                                 a.cap, (uint32_t)nch, w.ostart, w.err));
         }
         CK(cudaGetLastError());
-        const int smem = 2 * kChunkBytes + 16 + 2048 + 256 + 32 + 4 * kChunkCodes;
-        CK(cudaFuncSetAttribute(fused_inverse_3d_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                smem));
         if (nx >= 32 && !(flags_env() & 4)) {
             int dev = 0, sms = 148;
             cudaGetDevice(&dev);
@@ -587,6 +582,9 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
             TraceScope ts(s, "lq3d_inv_slab");
             if (launch_lq3d_inv_slab(a, (unsigned)sms, s) != 0) return FZB_E_CUDA;
         } else {
+            const int smem = 4 * kChunkCodes;
+            static SmemAttr attr;
+            CK(ensure_dyn_smem(attr, (const void*)fused_inverse_3d_kernel, smem));
             dim3 grid(g.ny / R, (g.nz + 7) / 8, 1);
             TraceScope ts(s, "fused_inverse_3d");
             fused_inverse_3d_kernel<<<grid, kThreads, smem, s>>>(a);
@@ -609,13 +607,10 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
         }
     }
     a.codes = w.codes;
-    const int smem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
-    CK(cudaFuncSetAttribute(rze_decode_codes_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                            smem));
     {
         TraceScope ts(s, "rze_decode_bitunshuffle");
         const uint64_t lim = a.gate ? 4ull * (uint64_t)sm_count() : nch;
-        rze_decode_codes_kernel<<<(unsigned)std::min<uint64_t>(nch, lim), kThreads, smem, s>>>(a);
+        rze_decode_codes_kernel<<<(unsigned)std::min<uint64_t>(nch, lim), kThreads, 0, s>>>(a);
     }
     CK(cudaGetLastError());
     rc = exact_inverse(a, g, s);

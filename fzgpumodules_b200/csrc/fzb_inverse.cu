@@ -2,7 +2,7 @@
 // (bytes, or bytes + Bitshuffle inverse -> codes), outlier scatter, the
 // exact tile-local Lorenzo inverse (1-D/2-D/3-D) and the fused single-pass
 // RZE -> Bitshuffle -> 3-D Lorenzo inverse.
-#include "fzb_kernels.cuh"
+#include "fzb_rzedec.cuh"
 
 namespace fzb {
 
@@ -164,93 +164,58 @@ __global__ void outlier_ranges_kernel(const uint32_t* __restrict__ idx, const ui
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
-__device__ __forceinline__ RzeDecSmem dec_smem(uint8_t* base, uint32_t* ws) {
-    RzeDecSmem sm;
-    sm.C = base;
-    sm.S = reinterpret_cast<uint32_t*>(base + kChunkBytes + 16);
-    sm.bm1 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16);
-    sm.bm2 = base + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = base + 2 * kChunkBytes + 16 + 2048 + 256;
-    sm.ws = ws;
-    return sm;
+// Decodes chunk c of a.rze into x (see rze_decode_words); returns its original size.
+__device__ __forceinline__ int decode_chunk(const InvArgs& a, uint32_t c, RzeDecSmem& sm, uint32_t (&x)[16]) {
+    const int osz = (c + 1 < a.n_chunks) ? kChunkBytes : (int)(a.orig_bytes - c * (uint32_t)kChunkBytes);
+    rze_decode_words(a.rze, a.rze_bytes, a.in_off[c], reinterpret_cast<const uint32_t*>(a.rze + 8)[c], osz, sm, a.err,
+                     x);
+    return osz;
 }
-constexpr int kDecSmemBytes = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
 
-__device__ __forceinline__ bool chunk_src(const InvArgs& a, uint32_t c, uint32_t* e, int* osz,
-                                          const uint8_t** src) {
-    *e = reinterpret_cast<const uint32_t*>(a.rze + 8)[c];
-    *osz = (c + 1 < a.n_chunks) ? kChunkBytes : (int)(a.orig_bytes - c * (uint32_t)kChunkBytes);
-    const uint64_t off = a.in_off[c];
-    *src = a.rze + off;
-    return off + (*e & 0x7fffffffu) <= a.rze_bytes;
+// Stores a chunk's words x[b] = word (15 - b) * 256 + t: coalesced 4-byte
+// stores when dst is 4-byte aligned; bytes for the rest and the ragged end.
+__device__ __forceinline__ void store_words(uint8_t* dst, int osz, const uint32_t (&x)[16]) {
+    const bool al = (reinterpret_cast<uintptr_t>(dst) & 3u) == 0;
+#pragma unroll
+    for (int b = 0; b < 16; b++) {
+        const int p = 4 * ((15 - b) * 256 + (int)threadIdx.x);
+        if (al && p + 4 <= osz) {
+            *reinterpret_cast<uint32_t*>(dst + p) = x[b];
+        } else {
+#pragma unroll
+            for (int k = 0; k < 4; k++)
+                if (p + k < osz) dst[p + k] = (uint8_t)(x[b] >> (8 * k));
+        }
+    }
 }
 
 // Plain RZE decode: one CTA per chunk, decoded bytes to bytes_out.
-__global__ void __launch_bounds__(kThreads) rze_decode_kernel(InvArgs a) {
-    extern __shared__ float4 smraw[];
-    __shared__ uint32_t s_ws[16];
+__global__ void __launch_bounds__(kThreads, 4) rze_decode_kernel(InvArgs a) {
+    __shared__ RzeDecSmem sm;
+    rze_decode_init(sm);
     const uint32_t c = blockIdx.x;
-    const RzeDecSmem sm = dec_smem(reinterpret_cast<uint8_t*>(smraw), s_ws);
-    uint32_t e;
-    int osz;
-    const uint8_t* src;
-    if (!chunk_src(a, c, &e, &osz, &src)) {
-        if (threadIdx.x == 0) atomicOr(a.err, kErrMalformed);
-        e = 2;  // decode as zeros
-    }
-    rze_decode_chunk(src, e, osz, sm, a.err);
-    uint8_t* dst = a.bytes_out + (size_t)c * kChunkBytes;
-    if (osz == kChunkBytes && (reinterpret_cast<uintptr_t>(dst) & 15) == 0) {
-        const uint4* s4 = reinterpret_cast<const uint4*>(sm.S);
-        uint4* d4 = reinterpret_cast<uint4*>(dst);
-        for (int i = threadIdx.x; i < kChunkBytes / 16; i += kThreads) d4[i] = s4[i];
-    } else {
-        const uint8_t* Sb = reinterpret_cast<const uint8_t*>(sm.S);
-        for (int i = threadIdx.x; i < osz; i += kThreads) dst[i] = Sb[i];
-    }
+    uint32_t x[16];
+    const int osz = decode_chunk(a, c, sm, x);
+    store_words(a.bytes_out + (size_t)c * kChunkBytes, osz, x);
 }
 
 // RZE decode + Bitshuffle inverse: one CTA per chunk (grid-stride over the
 // chunks when the grid is smaller), codes to a.codes.
-__global__ void __launch_bounds__(kThreads) rze_decode_codes_kernel(InvArgs a) {
-    extern __shared__ float4 smraw[];
-    __shared__ uint32_t s_ws[16];
+__global__ void __launch_bounds__(kThreads, 4) rze_decode_codes_kernel(InvArgs a) {
+    __shared__ RzeDecSmem sm;
     if (inv_gated_off(a)) return;
-    const RzeDecSmem sm = dec_smem(reinterpret_cast<uint8_t*>(smraw), s_ws);
+    rze_decode_init(sm);
     for (uint32_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
-        uint32_t e;
-        int osz;
-        const uint8_t* src;
-        if (!chunk_src(a, c, &e, &osz, &src)) {
-            if (threadIdx.x == 0) atomicOr(a.err, kErrMalformed);
-            e = 2;
-        }
-        rze_decode_chunk(src, e, osz, sm, a.err);
-        const int t = threadIdx.x;
-        if (osz == kChunkBytes) {
-            uint32_t x[16];
-            if (a.shuffled) {
+        uint32_t x[16];
+        const int osz = decode_chunk(a, c, sm, x);
+        if (osz == kChunkBytes && a.shuffled) {
+            uint32_t w[16];
+            codes_from_planes(x, w);
+            uint4* d4 = reinterpret_cast<uint4*>(a.codes + (size_t)c * kChunkCodes + 32 * threadIdx.x);
 #pragma unroll
-                for (int b = 0; b < 16; b++) x[b] = sm.S[(15 - b) * 256 + t];
-                transpose16x2(x);
-                uint32_t rw[16];
-#pragma unroll
-                for (int l = 0; l < 8; l++) rw[l] = __byte_perm(x[2 * l], x[2 * l + 1], 0x5410);
-#pragma unroll
-                for (int l = 8; l < 16; l++) rw[l] = __byte_perm(x[2 * l - 16], x[2 * l - 15], 0x7632);
-#pragma unroll
-                for (int l = 0; l < 16; l++) x[l] = rw[l];
-            } else {
-#pragma unroll
-                for (int l = 0; l < 16; l++) x[l] = sm.S[16 * t + l];
-            }
-            uint4* d4 = reinterpret_cast<uint4*>(a.codes + (size_t)c * kChunkCodes + 32 * t);
-#pragma unroll
-            for (int v = 0; v < 4; v++) d4[v] = make_uint4(x[4 * v], x[4 * v + 1], x[4 * v + 2], x[4 * v + 3]);
-        } else {  // tail block: stored unshuffled
-            uint8_t* dst = reinterpret_cast<uint8_t*>(a.codes) + (size_t)c * kChunkBytes;
-            const uint8_t* Sb = reinterpret_cast<const uint8_t*>(sm.S);
-            for (int i = t; i < osz; i += kThreads) dst[i] = Sb[i];
+            for (int v = 0; v < 4; v++) d4[v] = make_uint4(w[4 * v], w[4 * v + 1], w[4 * v + 2], w[4 * v + 3]);
+        } else {  // a tail block is stored unshuffled
+            store_words(reinterpret_cast<uint8_t*>(a.codes) + (size_t)c * kChunkBytes, osz, x);
         }
         __syncthreads();  // the shared buffers are reused by the next chunk
     }
@@ -459,11 +424,10 @@ __device__ __forceinline__ int dswz(int m) {  // swizzled float index in D
 
 __global__ void __launch_bounds__(kThreads, 2) fused_inverse_3d_kernel(InvArgs a) {
     extern __shared__ float4 smraw[];
-    __shared__ uint32_t s_ws[16];
+    __shared__ RzeDecSmem sm;
     if (*a.err & (kErrUnsorted | kErrMalformed)) return;
-    uint8_t* base = reinterpret_cast<uint8_t*>(smraw);
-    const RzeDecSmem sm = dec_smem(base, s_ws);
-    float* D = reinterpret_cast<float*>(base + kDecSmemBytes);
+    rze_decode_init(sm);
+    float* D = reinterpret_cast<float*>(smraw);
     const int t = threadIdx.x;
     const uint32_t nx = a.nx, R = kChunkCodes / nx, slabs = a.ny / R;
     const uint32_t s = blockIdx.x, zt = blockIdx.y;
@@ -485,18 +449,9 @@ __global__ void __launch_bounds__(kThreads, 2) fused_inverse_3d_kernel(InvArgs a
     const uint32_t z0 = zt * 8, z1 = min(z0 + 8, a.nz);
     for (uint32_t z = z0; z < z1; z++) {
         const uint32_t c = z * slabs + s;
-        uint32_t e;
-        int osz;
-        const uint8_t* src;
-        if (!chunk_src(a, c, &e, &osz, &src)) {
-            if (t == 0) atomicOr(a.err, kErrMalformed);
-            e = 2;
-        }
-        rze_decode_chunk(src, e, osz, sm, a.err);
         {   // Bitshuffle inverse + code -> float delta, thread t owns codes 32t..
             uint32_t x[16];
-#pragma unroll
-            for (int b = 0; b < 16; b++) x[b] = sm.S[(15 - b) * 256 + t];
+            decode_chunk(a, c, sm, x);
             transpose16x2(x);
             float4* D4 = reinterpret_cast<float4*>(D);
 #pragma unroll

@@ -27,7 +27,7 @@
 
 #include "../../include/fzb.h"
 #include "fzb_common.cuh"
-#include "fzb_kernels.cuh"
+#include "fzb_rzedec.cuh"
 
 namespace fzb {
 namespace {
@@ -231,43 +231,30 @@ __device__ __forceinline__ float pfpl_value(uint32_t c, float ebx2, float log2eb
 }
 
 template <bool REL>
-__global__ void __launch_bounds__(kThreads, 3) pfpl_decode_kernel(PDec a) {
-    extern __shared__ float4 smraw[];
+__global__ void __launch_bounds__(kThreads, 4) pfpl_decode_kernel(PDec a) {
+    __shared__ RzeDecSmem sm;
     __shared__ uint32_t s_ws[16];
+    rze_decode_init(sm);
     const int t = threadIdx.x;
     const uint32_t c = blockIdx.x;
-    uint8_t* base = reinterpret_cast<uint8_t*>(smraw);
-    RzeDecSmem sm;
-    sm.C = base;
-    sm.S = reinterpret_cast<uint32_t*>(base + kChunkBytes + 16);
-    sm.bm1 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16);
-    sm.bm2 = base + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = base + 2 * kChunkBytes + 16 + 2048 + 256;
-    sm.ws = s_ws;
-    uint32_t e = reinterpret_cast<const uint32_t*>(a.rze + 8)[c];
     const int osz = (c + 1 < a.n_chunks) ? kChunkBytes : (int)(a.orig_bytes - c * (uint32_t)kChunkBytes);
-    const uint64_t off = a.in_off[c];
-    if (off + (e & 0x7fffffffu) > a.rze_bytes) {
-        if (t == 0) atomicOr(a.err, kErrMalformed);
-        e = 2;  // decode as zeros
-    }
-    rze_decode_chunk(a.rze + off, e, osz, sm, a.err);
     const uint32_t cnt = (uint32_t)osz / 4;
     const uint32_t e0 = 16u * t;
     uint32_t d[16];
-    if (osz == kChunkBytes) {
+    {
         uint32_t x[16];
+        rze_decode_words(a.rze, a.rze_bytes, a.in_off[c], reinterpret_cast<const uint32_t*>(a.rze + 8)[c], osz, sm,
+                         a.err, x);
+        if (osz == kChunkBytes) {
+            codes_from_planes(x, d);
+        } else {  // a tail block is stored unshuffled: its words in order, through shared memory
+            __syncthreads();
 #pragma unroll
-        for (int b = 0; b < 16; b++) x[b] = sm.S[(15 - b) * 256 + t];
-        transpose16x2(x);
+            for (int b = 0; b < 16; b++) sm.C[(15 - b) * 256 + t] = x[b];
+            __syncthreads();
 #pragma unroll
-        for (int l = 0; l < 8; l++) {
-            d[l] = __byte_perm(x[2 * l], x[2 * l + 1], 0x5410);
-            d[8 + l] = __byte_perm(x[2 * l], x[2 * l + 1], 0x7632);
+            for (int k = 0; k < 16; k++) d[k] = (e0 + k < cnt) ? sm.C[16 * t + k] : 0u;
         }
-    } else {
-#pragma unroll
-        for (int k = 0; k < 16; k++) d[k] = (e0 + k < cnt) ? sm.S[16 * t + k] : 0u;
     }
     // negabinary, then the chunk's inclusive prefix sum
     uint32_t run = 0;
@@ -490,8 +477,8 @@ int fzb_pfpl_decompress(const void* d_rze, uint64_t rze_bytes, const float* d_ov
     a.err = err;
     {
         TraceScope ts(s, "pfpl_decode");
-        if (eb_mode == FZB_REL) pfpl_decode_kernel<true><<<nch, kThreads, kPSmem, s>>>(a);
-        else pfpl_decode_kernel<false><<<nch, kThreads, kPSmem, s>>>(a);
+        if (eb_mode == FZB_REL) pfpl_decode_kernel<true><<<nch, kThreads, 0, s>>>(a);
+        else pfpl_decode_kernel<false><<<nch, kThreads, 0, s>>>(a);
         if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
     }
     if (cap) {

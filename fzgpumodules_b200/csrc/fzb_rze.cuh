@@ -1,4 +1,5 @@
-// fzb_rze.cuh -- block-level RZE chunk encoder/decoder (256 threads).
+// fzb_rze.cuh -- block-level RZE chunk encoder (256 threads; the decoder is in
+// fzb_rzedec.cuh).
 //
 // Format of one chunk (modules/coders/rze/rze_stage.cu:324-445):
 //   [nonzero bytes][non-repeated bm1 bytes][non-repeated bm2 bytes]
@@ -211,118 +212,6 @@ __device__ __forceinline__ void copy_out_bytes(uint8_t* dst, const uint8_t* src,
         const uint8_t* p = s + 4 * i;
         dw[i] = (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
     }
-}
-
-struct RzeDecSmem {
-    uint8_t* C;     // >= kChunkBytes + 8: staged compressed chunk
-    uint32_t* S;    // 4096 words: decoded chunk bytes
-    uint32_t* bm1;  // 512 words
-    uint8_t* bm2;   // 256 bytes
-    uint8_t* bm3;   // 32 bytes
-    uint32_t* ws;   // 16 words
-};
-
-// Decodes one chunk (header word `e`, `osz` original bytes) from global
-// `src` into sm.S (bytes past osz zeroed).  Sets kErrMalformed on an
-// inconsistent chunk (and leaves zeros).  Ends with a barrier.
-__device__ static void rze_decode_chunk(const uint8_t* __restrict__ src, uint32_t e, int osz,
-                                 const RzeDecSmem& sm, uint32_t* err) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t comp = e & 0x7fffffffu;
-    uint8_t* Sb = reinterpret_cast<uint8_t*>(sm.S);
-    if (e & 0x80000000u) {  // raw chunk: copy the original bytes
-        const int n = min((int)comp, osz);
-        if (n != osz && t == 0) atomicOr(err, kErrMalformed);
-        for (int i = t; i < kChunkBytes; i += kThreads) Sb[i] = (i < n) ? src[i] : 0;
-        __syncthreads();
-        return;
-    }
-    if (comp <= 2) {  // all-zero chunk
-        for (int i = t; i < kChunkBytes / 4; i += kThreads) sm.S[i] = 0;
-        __syncthreads();
-        return;
-    }
-    if (comp > (uint32_t)kChunkBytes || comp < 7u) {
-        if (t == 0) atomicOr(err, kErrMalformed);
-        for (int i = t; i < kChunkBytes / 4; i += kThreads) sm.S[i] = 0;
-        __syncthreads();
-        return;
-    }
-    // stage the compressed bytes (aligned word loads, unaligned start)
-    {
-        const uintptr_t s0 = reinterpret_cast<uintptr_t>(src);
-        const uintptr_t a0 = s0 & ~(uintptr_t)3;
-        const uint32_t lead = (uint32_t)(s0 - a0);
-        const uint32_t nw = (lead + comp + 3) >> 2;
-        const uint32_t* sw = reinterpret_cast<const uint32_t*>(a0);
-        for (uint32_t i = t; i < nw; i += kThreads) {
-            uint32_t v = __ldg(sw + i);
-#pragma unroll
-            for (int b = 0; b < 4; b++) {
-                int32_t pos = (int32_t)(4 * i + b) - (int32_t)lead;
-                if (pos >= 0 && pos < (int32_t)comp) sm.C[pos] = (uint8_t)(v >> (8 * b));
-            }
-        }
-    }
-    __syncthreads();
-    const int b1 = (osz + 7) >> 3, b2 = (b1 + 7) >> 3, b3 = (b2 + 7) >> 3;
-    const int bm4_start = (int)comp - 6;
-    const uint32_t bm4 = (uint32_t)sm.C[bm4_start] | ((uint32_t)sm.C[bm4_start + 1] << 8) |
-                         ((uint32_t)sm.C[bm4_start + 2] << 16) | ((uint32_t)sm.C[bm4_start + 3] << 24);
-    const int s3 = bm4_start - __popc(bm4);
-    bool bad = s3 < 0;
-    // bm3 from bm4: byte l = data3[rank(l)-1] if any set bit at <= l
-    if (warp == 0) {
-        uint32_t r = __popc(bm4 & (0xffffffffu >> (31 - lane)));
-        uint32_t v = (r && lane < b3 && !bad) ? sm.C[s3 + (int)r - 1] : 0u;
-        sm.bm3[lane] = (uint8_t)v;
-        uint32_t pc = __popc(v);
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) pc += __shfl_xor_sync(0xffffffffu, pc, d);
-        if (lane == 0) sm.ws[12] = pc;
-    }
-    __syncthreads();
-    const int s2 = s3 - (int)sm.ws[12];
-    bad = bad || s2 < 0;
-    // bm2 from bm3: thread t produces bm2 byte t from bm3 bit t
-    {
-        const uint32_t* b3w = reinterpret_cast<const uint32_t*>(sm.bm3);
-        uint32_t r = 0;
-        for (int k = 0; k < (t >> 5); k++) r += __popc(b3w[k]);
-        r += __popc(b3w[t >> 5] & (0xffffffffu >> (31 - lane)));
-        uint32_t v = (r && t < b2 && !bad) ? sm.C[s2 + (int)r - 1] : 0u;
-        sm.bm2[t] = (uint8_t)v;
-        uint32_t n2;
-        const uint32_t ex = block_excl_scan((uint32_t)__popc(v), sm.ws, &n2);
-        const int s1 = s2 - (int)n2;
-        bad = bad || s1 < 0;
-        // bm1 from bm2: thread t produces bm1 bytes 8t..8t+7 from bm2 byte t
-        uint64_t M = 0;
-#pragma unroll
-        for (int k = 0; k < 8; k++) {
-            uint32_t rk = ex + __popc(v & (0xffu >> (7 - k)));
-            uint32_t byte = (rk && (8 * t + k) < b1 && !bad) ? sm.C[s1 + (int)rk - 1] : 0u;
-            M |= (uint64_t)byte << (8 * k);
-        }
-        // level-1 zero elimination: bytes 64t..64t+63 from bits of M
-        uint32_t nzT;
-        uint32_t pos = block_excl_scan((uint32_t)__popcll(M), sm.ws, &nzT);
-        bad = bad || ((int)nzT != s1);
-        if (bad) M = 0;
-#pragma unroll
-        for (int i = 0; i < 16; i++) {
-            uint32_t nib = (uint32_t)(M >> (4 * i)) & 15u;
-            uint32_t wv = 0;
-            while (nib) {
-                int b = __ffs(nib) - 1;
-                nib &= nib - 1;
-                wv |= (uint32_t)sm.C[pos++] << (8 * b);
-            }
-            sm.S[16 * t + i] = wv;
-        }
-    }
-    if (bad && t == 0) atomicOr(err, kErrMalformed);
-    __syncthreads();
 }
 
 }  // namespace fzb

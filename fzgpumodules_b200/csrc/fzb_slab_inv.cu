@@ -31,102 +31,20 @@
 // equal.  Chunks that carry outliers are checked: |d|, |x prefix| and
 // |xy prefix| must stay below 2^21, else kErrInexact is raised and the host
 // reruns the exact kernels.
-#include "fzb_slab.cuh"
+#include "fzb_rzedec.cuh"
 
 namespace fzb {
 namespace {
 
-constexpr int kCBytes = kChunkBytes + 64;  // one staged chunk (+ lead bytes and a slack word)
 constexpr size_t kInvSmem = kSmemAlign + kStageBytes + 2 * kCBytes + 2048 + 256 + 1024;
 constexpr float kExact = 2097152.0f;       // 2^21
 constexpr int kInvCtasPerSm = 3;           // 80 registers a thread, 3 x 73 KB of shared memory an SM
 
-// Expansion selectors: __byte_perm(v, 0, kExpandInit[m]) moves the low
-// popc(m) bytes of v to the byte positions flagged in the 4-bit mask m.
-__constant__ uint32_t kExpandInit[16] = {
-    0x4444, 0x4440, 0x4404, 0x4410, 0x4044, 0x4140, 0x4104, 0x4210,
-    0x0444, 0x1440, 0x1404, 0x2410, 0x1044, 0x2140, 0x2104, 0x3210};
-
-__device__ __forceinline__ void cp_async4(uint32_t* dst, const uint32_t* src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async16s(uint32_t* dst, const void* src) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;" ::: "memory"); }
-
-// Stages chunk c's payload (from the 16-byte boundary at or below its first
-// byte when the stream is 16-byte aligned, else the 4-byte one) into Cw.
-// Returns the header word in e, the first byte's offset from that boundary in
-// lead, and ok = the payload lies inside the stream.
+// stage_payload of chunk c; its header word in e.
 __device__ __forceinline__ void stage_chunk(const InvArgs& a, uint32_t c, uint32_t* Cw, uint32_t& e,
                                             uint32_t& lead, bool& ok) {
     e = reinterpret_cast<const uint32_t*>(a.rze + 8)[c];
-    const uint64_t off = a.in_off[c];
-    const uint32_t comp = e & 0x7fffffffu;
-    ok = off + comp <= a.rze_bytes;
-    const uint8_t* src = a.rze + (ok ? off : 0);
-    const uint32_t ncopy = ok ? min(comp, (uint32_t)kChunkBytes) : 0u;
-    const uint8_t* end = a.rze + a.rze_bytes;
-    if ((reinterpret_cast<uintptr_t>(a.rze) & 15u) == 0) {
-        // a 16-byte aligned stream: 16-byte copies from the 16-byte boundary
-        // at or below the first byte (never below the stream's start)
-        lead = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 15u);
-        const uint32_t ng = (lead + ncopy + 15) >> 4;
-        const uint8_t* g0 = src - lead;
-        for (uint32_t i = threadIdx.x; i < ng; i += kThreads) {
-            const uint8_t* p = g0 + 16u * i;
-            if (p + 16 <= end) {
-                cp_async16s(Cw + 4u * i, p);
-            } else {  // the stream's last bytes: only those inside it
-#pragma unroll
-                for (int w = 0; w < 4; w++) {
-                    uint32_t v = 0;
-                    for (int b = 0; b < 4; b++)
-                        if (p + 4 * w + b < end) v |= (uint32_t)p[4 * w + b] << (8 * b);
-                    Cw[4u * i + w] = v;
-                }
-            }
-        }
-        cp_async_commit();
-        return;
-    }
-    lead = (uint32_t)(reinterpret_cast<uintptr_t>(src) & 3u);
-    const uint32_t nw = (lead + ncopy + 3) >> 2;
-    const uint32_t* gw = reinterpret_cast<const uint32_t*>(src - lead);
-    for (uint32_t i = threadIdx.x; i < nw; i += kThreads) {
-        const uint8_t* p = reinterpret_cast<const uint8_t*>(gw + i);
-        if (p + 4 <= end) {
-            cp_async4(Cw + i, gw + i);
-        } else {  // last word of the stream: only the bytes inside it
-            uint32_t v = 0;
-            for (int b = 0; b < 4; b++)
-                if (p + b < end) v |= (uint32_t)p[b] << (8 * b);
-            Cw[i] = v;
-        }
-    }
-    cp_async_commit();
-}
-
-// 4 bytes of the staged chunk starting at payload byte q (lead included).
-__device__ __forceinline__ uint32_t staged_word(const uint32_t* Cw, uint32_t q) {
-    return __funnelshift_r(Cw[q >> 2], Cw[(q >> 2) + 1], 8u * (q & 3u));
-}
-
-__device__ __forceinline__ uint32_t staged_byte(const uint32_t* Cw, uint32_t q) {
-    return (Cw[q >> 2] >> (8u * (q & 3u))) & 0xffu;
-}
-
-// Packed code pair -> two biased 16-bit values u = s + 32768 (s the signed
-// delta): zigzag inverse (zigzag.h:80-84) or plain int16.
-template <bool ZZ>
-__device__ __forceinline__ uint32_t biased_pair(uint32_t x) {
-    if (ZZ) {
-        const uint32_t nb = 0x80008000u - (x & 0x00010001u);  // per half: bit0 ? 0x7fff : 0x8000
-        return ((x >> 1) & 0x7fff7fffu) ^ nb;
-    }
-    return x ^ 0x80008000u;
+    stage_payload(a.rze, a.rze_bytes, a.in_off[c], e, Cw, lead, ok);
 }
 
 }  // namespace
