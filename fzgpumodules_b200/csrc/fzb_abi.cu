@@ -289,35 +289,30 @@ int sm_count() {
     return sms;
 }
 
-// zero(out) + scatter + tile kernels (the exact path).  Every kernel walks
-// its tiles grid-stride: one tile per CTA normally; when the launch is gated
-// on the device status (a.gate) the grids are a few CTAs per SM, so a gate
-// that says "not needed" costs a few microseconds.
+// The outlier records of the Lorenzo inverse, in the workspace's n_total + 64
+// words `big` (a bit an element, three words a tile of at least 8 elements or
+// of the whole field).
+void outlier_records(InvArgs& a, const Work& w, const Geometry& g) {
+    uint64_t bits = 0;
+    a.ozero = lq_inverse_outlier_words((int)g.ndim, g.nx, g.ny, g.nz, &bits);
+    a.obits = w.big;
+    a.otiles = w.big + bits;
+}
+
+// Outliers, then the tile kernels (the exact path); a.obits (null when there is
+// no outlier list) is zeroed and the outputs past the field are zero.  When the
+// launch is gated on the device status (a.gate) the grids are a few CTAs per SM
+// walking their tiles, so a gate that says "not needed" costs a few microseconds.
 int exact_inverse(const InvArgs& a, const Geometry& g, cudaStream_t s) {
-    const uint32_t lim = a.gate ? 2u * (uint32_t)sm_count() : 0xffffffffu;
-    auto grid = [&](uint64_t tiles) { return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(tiles, lim)); };
-    if (a.gate) {
-        TraceScope ts(s, "zero_out");
-        zero_out_kernel<<<grid(((uint64_t)a.n_total + 1023) / 1024), 256, 0, s>>>(a);
-        CK(cudaGetLastError());
-    } else {
-        CK(cudaMemsetAsync(a.out, 0, sizeof(float) * (size_t)a.n_total, s));
-    }
-    if (a.cap) {
-        TraceScope ts(s, "scatter_outliers");
-        scatter_outliers_kernel<<<std::min(grid((a.cap + 255) / 256), 4096u), 256, 0, s>>>(a);
+    const uint32_t lim = a.gate ? 4u * (uint32_t)sm_count() : 0x7fffffffu;
+    if (a.obits) {
+        TraceScope ts(s, "mark_outliers");
+        const uint64_t want = std::min<uint64_t>((a.cap + 255ull) / 256u, std::min(lim, 4096u));
+        mark_outliers_kernel<<<(unsigned)want, 256, 0, s>>>(a);
         CK(cudaGetLastError());
     }
     TraceScope ts(s, "lq_inverse");
-    if (g.ndim == 1) {
-        lq_inverse_1d_kernel<<<grid((g.nfield + 1023) / 1024), 256, 0, s>>>(a);
-    } else if (g.ndim == 2) {
-        lq_inverse_2d_kernel<<<grid((uint64_t)((g.nx + 31) / 32) * ((g.ny + 31) / 32)), 128, 0, s>>>(a);
-    } else {
-        lq_inverse_3d_kernel<<<grid((uint64_t)((g.nx + 31) / 32) * ((g.ny + 7) / 8) * ((g.nz + 7) / 8)), 256, 0, s>>>(a);
-    }
-    CK(cudaGetLastError());
-    return FZB_OK;
+    return launch_lq_inverse(a, (int)g.ndim, lim, s) == 0 ? FZB_OK : FZB_E_CUDA;
 }
 
 int read_status(const Work& w, cudaStream_t s, uint32_t* bits) {
@@ -410,6 +405,11 @@ int lq_inverse_common(const uint16_t* d_codes, const float* d_err, const uint32_
     a.abs_eb_src = d_abs_eb;
     a.zigzag = zigzag;
     a.out = d_out;
+    if (cap) {
+        outlier_records(a, w, g);
+        CK(cudaMemsetAsync(a.obits, 0, 4 * (size_t)a.ozero, s));
+    }
+    if (n_total > g.nfield) CK(cudaMemsetAsync(d_out + g.nfield, 0, sizeof(float) * (n_total - g.nfield), s));
     return exact_inverse(a, g, s);
 }
 }  // namespace
@@ -607,6 +607,7 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
         }
     }
     a.codes = w.codes;
+    if (cap) outlier_records(a, w, g);
     {
         TraceScope ts(s, "rze_decode_bitunshuffle");
         const uint64_t lim = a.gate ? 4ull * (uint64_t)sm_count() : nch;

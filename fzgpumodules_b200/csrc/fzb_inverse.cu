@@ -1,6 +1,5 @@
 // fzb_inverse.cu -- inverse kernels: RZE stream prepass, chunk decode
-// (bytes, or bytes + Bitshuffle inverse -> codes), outlier scatter, the
-// exact tile-local Lorenzo inverse (1-D/2-D/3-D) and the fused single-pass
+// (bytes, or bytes + Bitshuffle inverse -> codes) and the fused single-pass
 // RZE -> Bitshuffle -> 3-D Lorenzo inverse.
 #include "fzb_rzedec.cuh"
 
@@ -200,13 +199,20 @@ __global__ void __launch_bounds__(kThreads, 4) rze_decode_kernel(InvArgs a) {
 }
 
 // RZE decode + Bitshuffle inverse: one CTA per chunk (grid-stride over the
-// chunks when the grid is smaller), codes to a.codes.
+// chunks when the grid is smaller), codes to a.codes.  It also clears the
+// outlier records (a.obits, when set) and the outputs past the field, which the
+// Lorenzo inverse that follows expects.
 __global__ void __launch_bounds__(kThreads, 4) rze_decode_codes_kernel(InvArgs a) {
     __shared__ RzeDecSmem sm;
     if (inv_gated_off(a)) return;
     rze_decode_init(sm);
+    if (a.obits)
+        for (uint64_t i = (uint64_t)blockIdx.x * kThreads + threadIdx.x; i < a.ozero; i += (uint64_t)gridDim.x * kThreads)
+            a.obits[i] = 0u;
     for (uint32_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
         uint32_t x[16];
+        const uint32_t e = c * (uint32_t)kChunkCodes + 32u * threadIdx.x;  // this thread's first element
+        for (uint32_t i = max(e, a.nfield); i < min(e + 32u, a.n_total); i++) a.out[i] = 0.0f;
         const int osz = decode_chunk(a, c, sm, x);
         if (osz == kChunkBytes && a.shuffled) {
             uint32_t w[16];
@@ -218,191 +224,6 @@ __global__ void __launch_bounds__(kThreads, 4) rze_decode_codes_kernel(InvArgs a
             store_words(reinterpret_cast<uint8_t*>(a.codes) + (size_t)c * kChunkBytes, osz, x);
         }
         __syncthreads();  // the shared buffers are reused by the next chunk
-    }
-}
-
-// Zeroes the n_total outputs (the exact path's first step; a kernel rather
-// than a memset so that it can be gated).
-__global__ void zero_out_kernel(InvArgs a) {
-    if (inv_gated_off(a)) return;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < a.n_total;
-         i += (uint64_t)gridDim.x * blockDim.x)
-        a.out[i] = 0.0f;
-}
-
-// out must be zeroed; writes each outlier's delta at its index
-// (lorenzo_quant_kernels.cuh:23-40).
-__global__ void scatter_outliers_kernel(InvArgs a) {
-    if (inv_gated_off(a)) return;
-    const uint32_t n = min(*a.out_count, a.cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = a.out_idx[i];
-        if (k < a.n_total) a.out[k] = a.out_err[i];
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Exact inverse kernels.  `out` holds the scattered outlier deltas (zero
-// elsewhere); each tile is reconstructed with the reference's add tree.
-// ---------------------------------------------------------------------------
-
-// 1-D: 1024-element tiles, thread t owns elements 4t..4t+3
-// (lorenzo_quant.cu:155-244).
-__global__ void __launch_bounds__(256) lq_inverse_1d_kernel(InvArgs a) {
-    __shared__ float s_w[8];
-    if (inv_gated_off(a)) return;
-    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const float ebx2 = inv_ebx2(a);
-    const bool zz = a.zigzag != 0;
-    const uint32_t ntiles = (a.nfield + 1023) / 1024;
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint64_t base = (uint64_t)tile * 1024 + 4 * t;
-        float v[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint64_t g = base + i;
-            v[i] = (g < a.nfield) ? __fadd_rn(a.out[g], decode_code(a.codes[g], zz)) : 0.0f;
-        }
-#pragma unroll
-        for (int i = 1; i < 4; i++) v[i] = __fadd_rn(v[i], v[i - 1]);
-        float ts = v[3];
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            float n = __shfl_up_sync(0xffffffffu, ts, d);
-            if ((int)lane >= d) ts = __fadd_rn(ts, n);
-        }
-        float pre = __shfl_up_sync(0xffffffffu, ts, 1);
-        if (lane > 0) {
-#pragma unroll
-            for (int i = 0; i < 4; i++) v[i] = __fadd_rn(v[i], pre);
-        }
-        if (lane == 31) s_w[warp] = v[3];
-        __syncthreads();
-        if (warp > 0) {
-            float w[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) w[i] = s_w[i];
-            // Hillis-Steele over the 8 warp totals, evaluated as a tree
-#pragma unroll
-            for (int d = 1; d < 8; d <<= 1)
-#pragma unroll
-                for (int i = 7; i >= 1; i--)
-                    if (i >= d) w[i] = __fadd_rn(w[i], w[i - d]);
-            const float add = w[warp - 1];
-#pragma unroll
-            for (int i = 0; i < 4; i++) v[i] = __fadd_rn(v[i], add);
-        }
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            const uint64_t g = base + i;
-            if (g < a.nfield) a.out[g] = __fmul_rn(v[i], ebx2);
-        }
-        __syncthreads();  // s_w is rewritten by the next tile
-    }
-}
-
-// 2-D: 32x32 tiles, 128 threads = 32 x 4 row groups of 8
-// (lorenzo_quant_nd.cu:112-190).
-__global__ void __launch_bounds__(128) lq_inverse_2d_kernel(InvArgs a) {
-    __shared__ float s_tot[4][32];
-    if (inv_gated_off(a)) return;
-    const uint32_t lx = threadIdx.x & 31, wy = threadIdx.x >> 5;
-    const float ebx2 = inv_ebx2(a);
-    const bool zz = a.zigzag != 0;
-    const uint32_t tx = (a.nx + 31) / 32, ntiles = tx * ((a.ny + 31) / 32);
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t gx = (tile % tx) * 32 + lx, gy0 = (tile / tx) * 32 + wy * 8;
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t gy = gy0 + i;
-            v[i] = 0.0f;
-            if (gx < a.nx && gy < a.ny) {
-                const uint64_t g = (uint64_t)gy * a.nx + gx;
-                v[i] = __fadd_rn(a.out[g], decode_code(a.codes[g], zz));
-            }
-        }
-#pragma unroll
-        for (int i = 1; i < 8; i++) v[i] = __fadd_rn(v[i], v[i - 1]);
-        s_tot[wy][lx] = v[7];
-        __syncthreads();
-        if (wy > 0) {
-            const float t0 = s_tot[0][lx];
-            const float t1 = __fadd_rn(t0, s_tot[1][lx]);
-            const float add = (wy == 1) ? t0 : (wy == 2) ? t1 : __fadd_rn(t1, s_tot[2][lx]);
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = __fadd_rn(v[i], add);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                float n = __shfl_up_sync(0xffffffffu, v[i], d);
-                if ((int)lx >= d) v[i] = __fadd_rn(v[i], n);
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t gy = gy0 + i;
-            if (gx < a.nx && gy < a.ny) a.out[(uint64_t)gy * a.nx + gx] = __fmul_rn(v[i], ebx2);
-        }
-        __syncthreads();  // s_tot is rewritten by the next tile
-    }
-}
-
-// 3-D: one CTA per 32x8x8 brick (four 8x8x8 tiles); thread (x, z) scans y
-// sequentially and x as an 8-lane Hillis-Steele, then thread (x, y) runs the
-// z Hillis-Steele tree in registers (lorenzo_quant_nd.cu:281-364).
-__global__ void __launch_bounds__(256) lq_inverse_3d_kernel(InvArgs a) {
-    __shared__ float V[8][8][33];  // [z][y][x]
-    if (inv_gated_off(a)) return;
-    const uint32_t lx = threadIdx.x & 31, lz = threadIdx.x >> 5;
-    const float ebx2 = inv_ebx2(a);
-    const bool zz = a.zigzag != 0;
-    const uint32_t tx = (a.nx + 31) / 32, ty = (a.ny + 7) / 8, ntiles = tx * ty * ((a.nz + 7) / 8);
-    for (uint32_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const uint32_t bx = tile % tx, by = (tile / tx) % ty, bz = tile / (tx * ty);
-        const uint32_t gx = bx * 32 + lx, gy0 = by * 8, gz = bz * 8 + lz;
-        float v[8];
-#pragma unroll
-        for (int y = 0; y < 8; y++) {
-            v[y] = 0.0f;
-            const uint32_t gy = gy0 + y;
-            if (gx < a.nx && gy < a.ny && gz < a.nz) {
-                const uint64_t g = ((uint64_t)gz * a.ny + gy) * a.nx + gx;
-                v[y] = __fadd_rn(a.out[g], decode_code(a.codes[g], zz));
-            }
-        }
-#pragma unroll
-        for (int y = 1; y < 8; y++) v[y] = __fadd_rn(v[y], v[y - 1]);
-        const uint32_t sx = lx & 7;
-#pragma unroll
-        for (int y = 0; y < 8; y++) {
-#pragma unroll
-            for (int d = 1; d < 8; d <<= 1) {
-                float n = __shfl_up_sync(0xffffffffu, v[y], d, 8);
-                if ((int)sx >= d) v[y] = __fadd_rn(v[y], n);
-            }
-            V[lz][y][lx] = v[y];
-        }
-        __syncthreads();
-        const uint32_t ly = lz;  // second phase: thread (x, y)
-        float w[8];
-#pragma unroll
-        for (int z = 0; z < 8; z++) w[z] = V[z][ly][lx];
-#pragma unroll
-        for (int d = 1; d < 8; d <<= 1)
-#pragma unroll
-            for (int z = 7; z >= 1; z--)
-                if (z >= d) w[z] = __fadd_rn(w[z], w[z - d]);
-        const uint32_t gy = gy0 + ly;
-#pragma unroll
-        for (int z = 0; z < 8; z++) {
-            const uint32_t gzz = bz * 8 + z;
-            if (gx < a.nx && gy < a.ny && gzz < a.nz)
-                a.out[((uint64_t)gzz * a.ny + gy) * a.nx + gx] = __fmul_rn(w[z], ebx2);
-        }
-        __syncthreads();  // V is rewritten by the next brick
     }
 }
 

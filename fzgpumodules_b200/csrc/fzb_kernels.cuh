@@ -119,6 +119,9 @@ struct InvArgs {
     int zigzag;
     int shuffled;                 // full chunks are bitshuffled (ew = 2)
     float* out;
+    uint32_t* obits;              // Lorenzo inverse: one bit per element with an outlier (null: none)
+    uint32_t* otiles;             // with obits: three words a tile (fzb_lqinv.cu), right after the bitmap
+    uint64_t ozero;               // words of both, zeroed before the outliers are marked
     uint32_t* err;
     // device-resident error bound: when set, kernels take 2 * *abs_eb_src
     // (the compressor's eb state) instead of ebx2
@@ -244,11 +247,11 @@ __global__ void outlier_ranges_kernel(const uint32_t* idx, const uint32_t* count
                                       uint32_t n_chunks, uint32_t* ostart, uint32_t* err);
 __global__ void rze_decode_kernel(InvArgs a);
 __global__ void rze_decode_codes_kernel(InvArgs a);
-__global__ void scatter_outliers_kernel(InvArgs a);
-__global__ void zero_out_kernel(InvArgs a);
-__global__ void lq_inverse_1d_kernel(InvArgs a);
-__global__ void lq_inverse_2d_kernel(InvArgs a);
-__global__ void lq_inverse_3d_kernel(InvArgs a);
+// Lorenzo inverse from codes (fzb_lqinv.cu): marks the outliers, then
+// reconstructs the tiles with at most `max_grid` CTAs.
+__global__ void mark_outliers_kernel(InvArgs a);
+int launch_lq_inverse(const InvArgs& a, int ndim, unsigned max_grid, cudaStream_t s);
+uint64_t lq_inverse_outlier_words(int ndim, uint32_t nx, uint32_t ny, uint32_t nz, uint64_t* bit_words);
 __global__ void fused_inverse_3d_kernel(InvArgs a);
 // Persistent slab inverse (fzb_slab_inv.cu) for nx >= 32; same results.
 int launch_lq3d_inv_slab(const InvArgs& a, unsigned sms, cudaStream_t s);  // persistent grid: 3 CTAs per SM

@@ -1,0 +1,57 @@
+"""The tile-local Lorenzo inverse from codes against the oracle, bit for bit:
+extents around the tile and load sizes, codes at 16-, 4- and 2-byte alignment,
+codes small and over the whole 16-bit range (the integer sums and the
+reference's add trees), and outliers that are integral, huge, fractional or
+not finite."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+DIMS = [(1, 1, 1), (7, 1, 1), (1023, 1, 1), (1025, 1, 1), (5000, 1, 1),
+        (31, 33, 1), (32, 32, 1), (40, 7, 1), (333, 65, 1), (8, 200, 1),
+        (7, 9, 3), (8, 8, 8), (33, 17, 9), (64, 10, 21), (130, 5, 40)]
+
+
+def _run(cuda, dims, codes, err, idx, zigzag, shift):
+    from fzgpumodules_b200 import kernels as K
+    n = codes.size
+    room = torch.zeros(n + shift, dtype=torch.int16, device=cuda)
+    room[shift:] = torch.from_numpy(codes.view(np.int16)).to(cuda)
+    abs_eb = np.float32(0.0123)
+    cap = max(len(err), 1)
+    e = torch.from_numpy(err if len(err) else np.zeros(1, np.float32)).to(cuda)
+    i = torch.from_numpy((idx if len(idx) else np.zeros(1, np.uint32)).view(np.int32)).to(cuda)
+    cnt = torch.tensor([len(err)], dtype=torch.int32, device=cuda)
+    y = K.lq_inverse(room[shift:].view(torch.uint16), e, i, cnt, cap, dims, float(abs_eb), zigzag)
+    ref = O.lq_inv(codes, err, idx, dims, np.float32(2) * abs_eb, zigzag)
+    got = y.cpu().numpy()
+    # equal bits, but for a NaN's payload, which IEEE 754 leaves to the machine
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    fine = ~np.isnan(ref)
+    assert np.array_equal(got.view(np.uint32)[fine], ref.view(np.uint32)[fine])
+
+
+@pytest.mark.parametrize("kind", ["small", "full", "integral", "huge", "fraction", "special"])
+@pytest.mark.parametrize("dims", DIMS)
+def test_inverse_edges(cuda, dims, kind):
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n + len(kind))
+    err, idx = np.zeros(0, np.float32), np.zeros(0, np.uint32)
+    codes = rng.integers(0, 65536 if kind == "full" else 200, n).astype(np.uint16)
+    if kind not in ("small", "full"):
+        idx = np.sort(rng.choice(n, max(1, n // 50), replace=False)).astype(np.uint32)
+        err = rng.integers(-60000, 60000, idx.size).astype(np.float32)
+        if kind == "huge":
+            err *= np.float32(1000)
+        if kind == "fraction":
+            err += np.float32(0.5)
+        if kind == "special":
+            err[0] = np.inf
+            err[-1] = np.nan if idx.size > 1 else np.inf
+        codes[idx] = 0
+    for zigzag, shift in ((True, 0), (False, 0), (True, 1), (True, 2)):
+        _run(cuda, dims, codes, err, idx, zigzag, shift)
