@@ -561,9 +561,11 @@ __device__ __forceinline__ uint32_t hf_emit(HfBits& r, const HfDecTables& t, uin
     return used;
 }
 
-__global__ void __launch_bounds__(kHfDecThreads, 2)
-    hf_decode_kernel(const uint8_t* __restrict__ blob, uint64_t blob_bytes, uint64_t n, uint32_t bklen_expect,
-                     uint16_t* __restrict__ out, uint32_t* err) {
+// CTA `cta` of `nctas` decoding one blob; fail() reports a malformed one.
+template <class Fail>
+__device__ __forceinline__ void hf_decode_blob(const uint8_t* __restrict__ blob, uint64_t blob_bytes, uint64_t n,
+                                               uint32_t bklen_expect, uint16_t* __restrict__ out, uint32_t cta,
+                                               uint32_t nctas, Fail fail) {
     __shared__ uint32_t s_first[32];
     __shared__ int s_entry[32];
     __shared__ uint32_t s_next;  // the CTA's next partition (or group of 32), in its own numbering
@@ -584,7 +586,7 @@ __global__ void __launch_bounds__(kHfDecThreads, 2)
                     e2 == e1 + 256 + 2 * bklen && e3 == e2 + 4 * pardeg && e4 == e3 + 4 * pardeg &&
                     e4 <= e5 && e5 <= blob_bytes;
     if (!ok) {
-        if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(err, kErrMalformed);
+        if (threadIdx.x == 0 && cta == 0) fail();
         return;
     }
     const int* rb = reinterpret_cast<const int*>(blob + e1);
@@ -670,7 +672,7 @@ __global__ void __launch_bounds__(kHfDecThreads, 2)
         // one partition per lane, 32 per take from the counter
         while (true) {
             uint32_t g = 0;
-            if (lane == 0) g = blockIdx.x + atomicAdd(&s_next, 1u) * gridDim.x;
+            if (lane == 0) g = cta + atomicAdd(&s_next, 1u) * nctas;
             g = __shfl_sync(~0u, g, 0);
             if (g >= (pardeg + 31) / 32) break;
             const uint32_t p = 32 * g + lane;
@@ -694,13 +696,13 @@ __global__ void __launch_bounds__(kHfDecThreads, 2)
                 }
             }
         }
-        if (bad) atomicOr(err, kErrMalformed);
+        if (bad) fail();
         return;
     }
 
     while (true) {
         uint32_t p = 0;
-        if (lane == 0) p = blockIdx.x + atomicAdd(&s_next, 1u) * gridDim.x;
+        if (lane == 0) p = cta + atomicAdd(&s_next, 1u) * nctas;
         p = __shfl_sync(~0u, p, 0);
         if (p >= pardeg) break;
         const uint32_t nbit = __ldg(nbits_g + p);
@@ -824,7 +826,34 @@ __global__ void __launch_bounds__(kHfDecThreads, 2)
         }
         __syncwarp();
     }
-    if (bad) atomicOr(err, kErrMalformed);
+    if (bad) fail();
+}
+
+__global__ void __launch_bounds__(kHfDecThreads, 2)
+    hf_decode_kernel(const uint8_t* __restrict__ blob, uint64_t blob_bytes, uint64_t n, uint32_t bklen_expect,
+                     uint16_t* __restrict__ out, uint32_t* err) {
+    hf_decode_blob(blob, blob_bytes, n, bklen_expect, out, blockIdx.x, gridDim.x,
+                   [&] { atomicOr(err, kErrMalformed); });
+}
+
+// The Huffman chunks of a selector container (fzb_select_dec.cu): a CTA takes
+// every gridDim.x-th chunk and decodes those with the Huffman tag.
+__global__ void __launch_bounds__(kHfDecThreads, 2) sel_hf_decode_kernel(SelDec a) {
+    if (*a.state == 0u) return;
+    for (uint32_t c = blockIdx.x; c < a.nch; c += gridDim.x) {
+        if (sel_tag(a, c) != 3u) continue;
+        const uint32_t sz = sel_size(a, c);
+        const uint64_t off = 4ull * a.offs[c];
+        if (off + sz > a.in_bytes) continue;  // reported by the offsets kernel
+        if (sz < 128u) {
+            if (threadIdx.x == 0) sel_fail(a, c, kSelMalformed);
+            continue;
+        }
+        const uint64_t c0 = (uint64_t)c * kSelCodes;
+        hf_decode_blob(a.in + off, sz, min((uint64_t)kSelCodes, a.n - c0), (uint32_t)kSelBk, a.out + c0, 0u, 1u,
+                       [&] { sel_fail(a, c, kSelMalformed); });
+        __syncthreads();  // the tables are rebuilt for the next chunk
+    }
 }
 
 int launch_hf_histogram(const uint16_t* in, uint64_t n, uint32_t bklen, uint32_t* freq, int sms,
@@ -880,6 +909,14 @@ int launch_hf_encode(const uint16_t* in, uint64_t n, const uint32_t* bk4, uint32
                                  (const uint32_t*)slots, (const uint32_t*)par_nbit, (const uint32_t*)par_ncell,
                                  (const uint32_t*)par_entry, pardeg, sublen, out_nbit, out_nbit + pardeg, bitstream,
                                  ctrl, reinterpret_cast<uint32_t*>(out + 24));
+}
+
+int launch_sel_hf_decode(const SelDec& a, int sms, cudaStream_t s) {
+    static SmemAttr attr;
+    const cudaError_t e = ensure_dyn_smem(attr, (const void*)sel_hf_decode_kernel, (int)kHfDecSmem);
+    if (e != cudaSuccess) return (int)e;
+    sel_hf_decode_kernel<<<min(2u * (uint32_t)sms, a.nch), kHfDecThreads, kHfDecSmem, s>>>(a);
+    return (int)cudaGetLastError();
 }
 
 int launch_hf_decode(const uint8_t* blob, uint64_t blob_bytes, uint64_t n, uint32_t bklen,

@@ -341,6 +341,32 @@ struct SelArgs {
     uint8_t* tags;           // nchunks
 };
 
+// Decoding a selector container (fzb_select_dec.cu): every chunk at once.
+struct SelDec {
+    const uint8_t* in;
+    uint64_t in_bytes;
+    uint64_t n;
+    uint32_t nch;
+    uint16_t* out;
+    uint32_t* state;  // 1 once the container's header is found good (zeroed before)
+    uint32_t* fault;  // ~(chunk * 4 + cause) of the first faulty chunk, 0 for none (zeroed before)
+    uint32_t* offs;   // nch: payload offsets in 4-byte words
+};
+constexpr uint32_t kSelMalformed = 1, kSelInvalid = 2;
+
+__device__ __forceinline__ uint32_t sel_tag(const SelDec& a, uint32_t c) { return a.in[16 + c]; }
+__device__ __forceinline__ uint32_t sel_param(const SelDec& a, uint32_t c) {
+    return a.in[16 + ((a.nch + 3u) & ~3u) + c];
+}
+__device__ __forceinline__ uint32_t sel_size(const SelDec& a, uint32_t c) {
+    return reinterpret_cast<const uint32_t*>(a.in + 16 + 2 * (size_t)((a.nch + 3u) & ~3u))[c];
+}
+__device__ __forceinline__ void sel_fail(const SelDec& a, uint32_t c, uint32_t cause) {
+    atomicMax(a.fault, ~(4u * c + cause));
+}
+int launch_sel_decode(const SelDec& a, cudaStream_t s);
+int launch_sel_hf_decode(const SelDec& a, int sms, cudaStream_t s);
+
 int launch_sel_features(const uint16_t* codes, uint64_t n, float* feats, cudaStream_t s);
 int launch_sel_coders(const SelArgs& a, uint32_t nchunks, unsigned coder_mask, cudaStream_t s);
 int launch_sel_choose(const SelArgs& a, uint32_t nchunks, int mode, const float* pred, cudaStream_t s);

@@ -5,7 +5,6 @@
 
 #include <cstdint>
 #include <cstring>
-#include <vector>
 
 #include "../../include/fzb.h"
 #include "fzb_kernels.cuh"
@@ -186,56 +185,34 @@ int fzb_sel_encode(const uint16_t* d_codes, uint64_t n, int mode, const float* d
     return FZB_OK;
 }
 
-// Host-driven decoder: reads the container header, then decodes every
-// chunk with its coder's decoder into d_codes (n codes).
+// Decodes every chunk with its coder's decoder into d_codes (n codes), all
+// chunks at once on the device; the one host wait reads the outcome.
 int fzb_sel_decode(const void* d_in, uint64_t in_bytes, uint16_t* d_codes, uint64_t n, void* d_work,
                    size_t work_bytes, void* stream) {
     if (!d_in || !d_codes || n == 0 || n >= (1ull << 31) || in_bytes < 16) return FZB_E_INVALID;
     const uint64_t nch = sel_chunks(n);
     const size_t need = fzb_workspace_bytes(kSelCodes, 0) + 2 * kSelBytes + 256;
-    if (!d_work || work_bytes < need) return FZB_E_WORKSPACE;
+    if (!d_work || work_bytes < need || need < 256 + 4 * nch) return FZB_E_WORKSPACE;
+    if (in_bytes < 16 + 2 * ((nch + 3) & ~3ull) + 4 * nch) return FZB_E_MALFORMED;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const uint8_t* in = static_cast<const uint8_t*>(d_in);
-    uint32_t h[4];
-    CK(cudaMemcpyAsync(h, in, 16, cudaMemcpyDeviceToHost, s));
+    uint32_t* ctrl = static_cast<uint32_t*>(d_work);  // word 0: device status, 1: state, 2: fault
+    CK(cudaMemsetAsync(ctrl, 0, 256, s));
+    SelDec a{};
+    a.in = static_cast<const uint8_t*>(d_in);
+    a.in_bytes = in_bytes;
+    a.n = n;
+    a.nch = (uint32_t)nch;
+    a.out = d_codes;
+    a.state = ctrl + 1;
+    a.fault = ctrl + 2;
+    a.offs = ctrl + 64;
+    if (launch_sel_decode(a, s) != 0) return FZB_E_CUDA;
+    uint32_t h[2];
+    CK(cudaMemcpyAsync(h, ctrl + 1, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
-    if (h[0] != 0x43535A46u || h[1] != nch || h[2] != (uint32_t)n || h[3] != (uint32_t)kSelCodes)
-        return FZB_E_MALFORMED;
-    const uint64_t pad = (nch + 3) & ~3ull;
-    const uint64_t hdr = 16 + 2 * pad + 4 * nch;
-    if (in_bytes < hdr) return FZB_E_MALFORMED;
-    std::vector<uint8_t> meta(hdr);
-    CK(cudaMemcpyAsync(meta.data(), in, hdr, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
-    const uint8_t* tags = meta.data() + 16;
-    const uint8_t* params = tags + pad;
-    const uint32_t* sizes = reinterpret_cast<const uint32_t*>(params + pad);
-    uint8_t* ws = static_cast<uint8_t*>(d_work);
-    uint8_t* tmp = ws + a256(fzb_workspace_bytes(kSelCodes, 0));  // 64 KiB staging
-    const size_t wsz = fzb_workspace_bytes(kSelCodes, 0);
-    uint64_t off = hdr;
-    for (uint64_t c = 0; c < nch; c++) {
-        const uint32_t cnt = (uint32_t)((n - c * kSelCodes) < (uint64_t)kSelCodes ? n - c * kSelCodes : kSelCodes);
-        const uint32_t sz = sizes[c];
-        if (off + sz > in_bytes) return FZB_E_MALFORMED;
-        uint16_t* dst = d_codes + c * kSelCodes;
-        int rc = FZB_OK;
-        switch (tags[c]) {
-            case 0:  // RZE stream of the bitshuffled chunk
-                rc = fzb_rze_decode(in + off, sz, 2ull * cnt, tmp, ws, wsz, stream);
-                if (!rc) rc = fzb_bitshuffle(tmp, 2ull * cnt, kChunkBytes, 2, 1, dst, stream);
-                break;
-            case 1: rc = fzb_rle_decode(in + off, cnt, 2, dst, ws, wsz, stream); break;
-            case 2: rc = fzb_bitpack_decode(in + off, cnt, 2, params[c], dst, stream); break;
-            case 3: rc = fzb_huff_decode(in + off, sz, cnt, kSelBk, dst, ws, wsz, stream); break;
-            default: return FZB_E_MALFORMED;
-        }
-        if (rc) return rc;
-        const int st = fzb_workspace_status(ws, stream);
-        if (st) return st;
-        off += (sz + 3) & ~3u;
-    }
-    return FZB_OK;
+    if (!h[0]) return FZB_E_MALFORMED;
+    if (!h[1]) return FZB_OK;
+    return (~h[1] & 3u) == kSelInvalid ? FZB_E_INVALID : FZB_E_MALFORMED;
 }
 
 int fzb_mlp_forward(const float* d_params, const float* d_x, float* d_y, uint32_t batch, void* stream) {
