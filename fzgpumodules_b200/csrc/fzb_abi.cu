@@ -34,7 +34,7 @@ struct Work {
     float* ostage_err;
     uint32_t* ostage_idx;
     uint64_t ostage_cap;
-    uint32_t* big;      // n_total u32 (RLE run starts / offsets)
+    uint32_t* big;      // n_total u32 (outlier bitmaps, RLE tile records)
     uint32_t* tiles;    // per-4096-element tile scratch
     uint32_t* total;    // device scalar
     unsigned int* done; // last-block counter
@@ -667,7 +667,7 @@ int fzb_rle_decode(const void* d_in, uint64_t n, int elem, void* d_out, void* d_
     cudaStream_t s = S(stream);
     CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));
     return launch_rle_decode(static_cast<const uint8_t*>(d_in), (uint32_t)n, elem, d_out, w.big,
-                             w.tiles, w.total, w.err, s) == 0 ? FZB_OK : FZB_E_CUDA;
+                             w.total, w.err, s) == 0 ? FZB_OK : FZB_E_CUDA;
 }
 
 int fzb_bitpack_encode(const void* d_in, uint64_t n, int elem, int nbits, void* d_out,

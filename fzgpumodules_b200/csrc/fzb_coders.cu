@@ -16,16 +16,9 @@ constexpr int kScanTile = 4096;  // elements per CTA in the scan passes
 
 // ---------------------------------------------------------------------------
 // Exclusive scan of u32 values, three passes: tile sums, one-CTA scan of
-// the tile sums, tile scan + offset.  The source is either a plain array
-// (count given or read from *cptr) or the run-length array of an RLE stream
-// (count and position read from the stream's header on the device).
+// the tile sums, tile scan + offset.  The count is given or read from *cptr.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ const uint32_t* scan_src(const ScanSrc& a, uint32_t* cnt) {
-    if (a.rle) {
-        const uint32_t R = *reinterpret_cast<const uint32_t*>(a.rle);
-        *cnt = min(R, a.n);
-        return reinterpret_cast<const uint32_t*>(a.rle + 4 + ((R * (uint32_t)a.elem + 3u) & ~3u));
-    }
     *cnt = a.cptr ? min(*a.cptr, a.n) : a.n;
     return a.base;
 }
@@ -112,181 +105,274 @@ int launch_scan_u32(const ScanSrc& a, uint32_t* out, uint32_t* tile_scratch, uin
 }
 
 // ---------------------------------------------------------------------------
-// RLE encode.  Pass 1 counts run starts per 4096-element tile; the tile
-// counts are scanned; pass 2 writes each run's value and start position;
-// pass 3 turns start positions into lengths.
+// RLE encode.  Pass 1 counts the runs that start in each 4096-element tile and
+// notes the first start; the counts are scanned; pass 2 compacts a tile's runs
+// in shared memory and writes their values and lengths in order (the last run
+// of a tile ends at the first start of the next tile that has one).
+//
+// Bound by HBM: the input is read twice (2 B an element, the second time
+// mostly from L2) and sizeof(T) + 4 B written a run.  Before, each thread
+// wrote its 16 elements' runs one by one, with their starts, and a third
+// kernel turned starts into lengths: 6.5 M elements in nearly as many runs took
+// 9.6 + 65 + 15 us, now 4 + 17.
 // ---------------------------------------------------------------------------
+
+// The tile's elements 16t .. 16t + 15 (t the thread) and their run-start bits.
 template <typename T>
-__device__ __forceinline__ uint32_t run_starts16(const T* __restrict__ in, uint32_t n, uint32_t b,
+__device__ __forceinline__ uint32_t run_starts16(const T* __restrict__ in, uint32_t n, uint32_t b, bool vec,
                                                  T (&v)[16]) {
+    constexpr int kQ = 16 * sizeof(T) / 16;  // 16-byte granules a thread
+    union {
+        uint4 q[kQ];
+        T e[16];
+    } u;
+    if (vec && b + 16 <= n) {
+#pragma unroll
+        for (int i = 0; i < kQ; i++) u.q[i] = __ldg(reinterpret_cast<const uint4*>(in + b) + i);
+    } else {
+#pragma unroll
+        for (int i = 0; i < 16; i++) u.e[i] = b + i < n ? in[b + i] : T(0);
+    }
+    T prev = (b > 0 && b <= n) ? __ldg(in + b - 1) : T(0);
     uint32_t m = 0;
-    T prev = (b > 0 && b - 1 < n) ? in[b - 1] : T(0);
 #pragma unroll
     for (int i = 0; i < 16; i++) {
-        const uint32_t k = b + i;
-        v[i] = (k < n) ? in[k] : T(0);
-        const bool start = (k < n) && (k == 0 || v[i] != prev);
-        m |= (start ? 1u : 0u) << i;
+        v[i] = u.e[i];
+        m |= ((v[i] != prev || b + i == 0) ? 1u : 0u) << i;
         prev = v[i];
     }
-    return m;
+    return b + 16 <= n ? m : b < n ? m & ((1u << (n - b)) - 1u) : 0u;
 }
 
 template <typename T>
-__global__ void __launch_bounds__(256) rle_count_kernel(const T* __restrict__ in, uint32_t n,
-                                                        uint32_t* __restrict__ tcnt) {
-    T v[16];
-    const uint32_t m = run_starts16(in, n, blockIdx.x * kScanTile + threadIdx.x * 16, v);
-    uint32_t s = __popc(m);
-#pragma unroll
-    for (int d = 16; d >= 1; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    __shared__ uint32_t w[8];
-    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t t = 0;
-        for (int i = 0; i < 8; i++) t += w[i];
-        tcnt[blockIdx.x] = t;
-    }
-}
-
-template <typename T>
-__global__ void __launch_bounds__(256) rle_emit_kernel(const T* __restrict__ in, uint32_t n,
-                                                       const uint32_t* __restrict__ toff,
-                                                       uint8_t* __restrict__ out,
-                                                       uint32_t* __restrict__ starts) {
-    __shared__ uint32_t ws[16];
+__global__ void __launch_bounds__(256) rle_count_kernel(const T* __restrict__ in, uint32_t n, int vec,
+                                                        uint32_t* __restrict__ tcnt, uint32_t* __restrict__ tfirst) {
+    __shared__ uint32_t w[8], f[8];
     T v[16];
     const uint32_t b = blockIdx.x * kScanTile + threadIdx.x * 16;
-    const uint32_t m = run_starts16(in, n, b, v);
-    uint32_t tot;
-    uint32_t r = toff[blockIdx.x] + block_excl_scan(__popc(m), ws, &tot);
-    T* values = reinterpret_cast<T*>(out + 4);
-#pragma unroll
-    for (int i = 0; i < 16; i++) {
-        if ((m >> i) & 1u) {
-            values[r] = v[i];
-            starts[r] = b + i;
-            r++;
+    const uint32_t m = run_starts16(in, n, b, vec != 0, v);
+    const uint32_t s = __reduce_add_sync(0xffffffffu, __popc(m));
+    const uint32_t first = __reduce_min_sync(0xffffffffu, m ? b + __ffs(m) - 1 : 0xffffffffu);
+    if ((threadIdx.x & 31) == 0) {
+        w[threadIdx.x >> 5] = s;
+        f[threadIdx.x >> 5] = first;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t t = 0, g = 0xffffffffu;
+        for (int i = 0; i < 8; i++) {
+            t += w[i];
+            g = min(g, f[i]);
         }
+        tcnt[blockIdx.x] = t;
+        tfirst[blockIdx.x] = g;
     }
 }
 
 template <typename T>
-__global__ void rle_lengths_kernel(const uint32_t* __restrict__ runs_ptr, uint32_t n,
-                                   const uint32_t* __restrict__ starts, uint8_t* __restrict__ out,
-                                   unsigned long long* __restrict__ out_size) {
-    const uint32_t R = *runs_ptr;
+__global__ void __launch_bounds__(256) rle_emit_kernel(const T* __restrict__ in, uint32_t n, int vec,
+                                                       const uint32_t* __restrict__ toff,
+                                                       const uint32_t* __restrict__ tfirst,
+                                                       const uint32_t* __restrict__ total, uint8_t* __restrict__ out,
+                                                       unsigned long long* __restrict__ out_size) {
+    __shared__ uint32_t ws[16];
+    __shared__ uint32_t s_start[kScanTile + 1];
+    __shared__ T s_val[kScanTile];
+    const uint32_t R = *total, t = threadIdx.x;
     const uint32_t vbytes = R * (uint32_t)sizeof(T), valigned = (vbytes + 3u) & ~3u;
+    T* values = reinterpret_cast<T*>(out + 4);
     uint32_t* lens = reinterpret_cast<uint32_t*>(out + 4 + valigned);
-    const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint32_t r = tid; r < R; r += gridDim.x * blockDim.x)
-        lens[r] = ((r + 1 < R) ? starts[r + 1] : n) - starts[r];
-    if (tid == 0) {
+    if (blockIdx.x == 0 && t == 0) {
         reinterpret_cast<uint32_t*>(out)[0] = R;
         for (uint32_t i = vbytes; i < valigned; i++) out[4 + i] = 0;
         *out_size = 4ull + valigned + 4ull * R;
     }
+    const uint32_t r0 = toff[blockIdx.x];
+    const uint32_t r1 = blockIdx.x + 1 < gridDim.x ? toff[blockIdx.x + 1] : R;
+    if (r0 == r1) return;
+    T v[16];
+    const uint32_t b = blockIdx.x * kScanTile + t * 16;
+    const uint32_t m = run_starts16(in, n, b, vec != 0, v);
+    uint32_t tot;
+    uint32_t r = block_excl_scan(__popc(m), ws, &tot);
+#pragma unroll
+    for (int i = 0; i < 16; i++) {
+        if ((m >> i) & 1u) {
+            s_start[r] = b + i;
+            s_val[r] = v[i];
+            r++;
+        }
+    }
+    if (t == 0) {  // the first start after the tile: of the first later tile with more runs before its end
+        uint32_t next = n;
+        if (r1 < R) {
+            uint32_t lo = blockIdx.x + 1, hi = gridDim.x - 1;  // tile lo .. hi holds run r1
+            while (lo < hi) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (toff[mid + 1] > r1) hi = mid;
+                else lo = mid + 1;
+            }
+            next = tfirst[lo];
+        }
+        s_start[tot] = next;
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < tot; i += 256) {
+        values[r0 + i] = s_val[i];
+        lens[r0 + i] = s_start[i + 1] - s_start[i];
+    }
 }
 
 // ---------------------------------------------------------------------------
-// RLE decode: scan of run lengths, then each 4096-element output tile
-// gathers the runs that overlap it into shared memory and every element
-// binary-searches its run there.
+// RLE decode.  The run lengths are summed per 1024 runs and the sums scanned;
+// then each 4096-element output tile finds its first tile of runs, scans the
+// lengths of the tiles of runs that overlap it and fills its part of shared
+// memory: short runs by their own thread, longer ones by the whole block.
+//
+// Bound by HBM (lengths read twice, 4 B a run; values and output once).  It
+// replaced a scan that wrote every run's offset and a binary search for every
+// element: the same stream took 5 + 37 + 50 us, now 5 + 32.
 // ---------------------------------------------------------------------------
+constexpr uint32_t kRunTile = 1024;
+
+// Exclusive scan over 256 threads of values up to `top` (below 2^31), the sums
+// saturating at it (a malformed stream's lengths may add up past 32 bits).
+__device__ __forceinline__ uint32_t block_excl_scan_sat(uint32_t v, uint32_t top, uint32_t* ws, uint32_t* total) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    uint32_t inc = v;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t o = __shfl_up_sync(0xffffffffu, inc, d);
+        if (lane >= (uint32_t)d) inc = min(inc + o, top);
+    }
+    uint32_t ex = __shfl_up_sync(0xffffffffu, inc, 1);
+    if (lane == 0) ex = 0;
+    if (lane == 31) ws[warp] = inc;
+    __syncthreads();
+    uint32_t base = 0, all = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < 8; w++) {
+        if (w == warp) base = all;
+        all = min(all + ws[w], top);
+    }
+    *total = all;
+    return min(base + ex, top);
+}
+
+__device__ __forceinline__ uint32_t rle_runs(const uint8_t* in, uint32_t n) {
+    return min(*reinterpret_cast<const uint32_t*>(in), n);  // at most n runs in a valid stream
+}
+__device__ __forceinline__ const uint32_t* rle_lens(const uint8_t* in, uint32_t elem) {
+    const uint32_t R = *reinterpret_cast<const uint32_t*>(in);
+    return reinterpret_cast<const uint32_t*>(in + 4 + ((R * elem + 3u) & ~3u));
+}
+
+// Sum of each tile of runs, a warp a tile.
+__global__ void __launch_bounds__(256) rle_sums_kernel(const uint8_t* __restrict__ in, uint32_t n, uint32_t elem,
+                                                       uint32_t* __restrict__ tsum, uint32_t ntiles) {
+    const uint32_t R = rle_runs(in, n), lane = threadIdx.x & 31u;
+    const uint32_t* lens = rle_lens(in, elem);
+    for (uint32_t tile = blockIdx.x * 8 + (threadIdx.x >> 5); tile < ntiles; tile += gridDim.x * 8) {
+        uint32_t s = 0;
+        const uint32_t b = tile * kRunTile;
+#pragma unroll 8
+        for (uint32_t i = b + lane; i < b + kRunTile; i += 32)
+            if (i < R) s += lens[i];
+        s = __reduce_add_sync(0xffffffffu, s);
+        if (lane == 0) tsum[tile] = s;
+    }
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256) rle_expand_kernel(const uint8_t* __restrict__ in,
-                                                         const uint32_t* __restrict__ offs,
-                                                         uint32_t n, T* __restrict__ out,
-                                                         uint32_t* err) {
-    __shared__ uint32_t s_off[kScanTile + 2];
-    __shared__ T s_val[kScanTile + 2];
-    __shared__ uint32_t s_nr;
-    const uint32_t R = min(*reinterpret_cast<const uint32_t*>(in), n);
+                                                         const uint32_t* __restrict__ toff,
+                                                         const uint32_t* __restrict__ total, uint32_t n,
+                                                         T* __restrict__ out, uint32_t* err) {
+    constexpr uint32_t kLong = 64;  // runs from this length on are filled by the whole block
+    __shared__ __align__(16) T s_out[kScanTile];
+    __shared__ uint32_t ws[16], s_long[kScanTile / kLong + 2], s_nlong;
+    const uint32_t R = rle_runs(in, n), t = threadIdx.x;
+    const uint32_t* lens = rle_lens(in, sizeof(T));
     const T* values = reinterpret_cast<const T*>(in + 4);
     const uint32_t t0 = blockIdx.x * kScanTile, t1 = min(n, t0 + kScanTile);
-    if (t0 >= n) return;
-    if (R == 0) {
-        if (threadIdx.x == 0) atomicOr(err, kErrMalformed);
-        for (uint32_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) out[i] = T(0);
-        return;
+    if (blockIdx.x == 0 && t == 0 && (R == 0 || *total != n)) atomicOr(err, kErrMalformed);
+    // the last tile of runs starting at or before t0
+    uint32_t lo = 0, hi = (R + kRunTile - 1) / kRunTile;
+    while (lo + 1 < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (toff[mid] <= t0) lo = mid;
+        else hi = mid;
     }
-    // last run whose start <= t0: every round all threads probe evenly spaced
-    // starts and the count of starts <= t0 narrows the range about blockDim-fold
-    uint32_t lo = 0, hi = R;
-    while (hi - lo > 1) {
-        const uint32_t step = (hi - lo + blockDim.x - 1) / blockDim.x;
-        const uint32_t p = lo + threadIdx.x * step;
-        const int c = __syncthreads_count(p < hi && offs[p] <= t0);
-        const uint32_t nlo = lo + (uint32_t)(c > 0 ? c - 1 : 0) * step;
-        hi = min(hi, lo + (uint32_t)(c > 0 ? c : 1) * step);
-        lo = nlo;
-    }
-    // the runs overlapping the tile: at most kScanTile + 1 from r0
-    const uint32_t r0 = lo, win = min(R - r0, (uint32_t)kScanTile + 1);
-    if (threadIdx.x == 0) s_nr = 0;
+    uint32_t pos = R ? toff[lo] : t1;  // output position of the tile of runs
+    for (uint32_t i = t; i < kScanTile; i += 256) s_out[i] = T(0);
+    if (t == 0) s_nlong = 0;
     __syncthreads();
-    uint32_t mine = 0;
-    for (uint32_t i = threadIdx.x; i < win; i += blockDim.x) {
-        const uint32_t o = offs[r0 + i];
-        s_off[i] = o;
-        s_val[i] = values[r0 + i];
-        mine += o < t1;
-    }
-    if (mine) atomicAdd(&s_nr, mine);
-    __syncthreads();
-    const uint32_t nr = s_nr;
-    if (nr == 0) {
-        for (uint32_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) out[i] = T(0);
-        return;
-    }
-    for (uint32_t i = t0 + threadIdx.x; i < t1; i += blockDim.x) {
-        uint32_t lo = 0, hi = nr;
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (s_off[mid] <= i) lo = mid;
-            else hi = mid;
+    for (uint32_t r0 = lo * kRunTile; r0 < R && pos < t1; r0 += kRunTile) {
+        uint32_t len[4], sum = 0;
+        T val[4];
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t r = r0 + 4 * t + k;
+            len[k] = r < R ? min(lens[r], n) : 0u;
+            val[k] = r < R ? values[r] : T(0);
+            sum = min(sum + len[k], n);
         }
-        out[i] = s_val[lo];
+        uint32_t tot;
+        uint32_t e = min(pos + block_excl_scan_sat(sum, n, ws, &tot), n);
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            const uint32_t a0 = max(e, t0), a1 = min(min(e + len[k], n), t1);
+            e = min(e + len[k], n);
+            if (a0 >= a1) continue;
+            if (a1 - a0 < kLong) {
+                for (uint32_t i = a0; i < a1; i++) s_out[i - t0] = val[k];
+            } else {
+                const uint32_t q = atomicAdd(&s_nlong, 1u);  // at most kScanTile / kLong of them
+                s_long[q] = (a0 - t0) | (a1 - t0) << 16;
+                s_out[a0 - t0] = val[k];
+            }
+        }
+        __syncthreads();
+        for (uint32_t q = 0; q < s_nlong; q++) {
+            const uint32_t a0 = s_long[q] & 0xffffu, a1 = s_long[q] >> 16;
+            const T v = s_out[a0];
+            for (uint32_t i = a0 + 1 + t; i < a1; i += 256) s_out[i] = v;
+        }
+        __syncthreads();
+        if (t == 0) s_nlong = 0;
+        pos = min(pos + tot, n);
     }
+    __syncthreads();
+    for (uint32_t i = t0 + t; i < t1; i += 256) out[i] = s_out[i - t0];
 }
 
 template <typename T>
 int launch_rle_encode_t(const T* in, uint32_t n, uint8_t* out, unsigned long long* out_size,
-                        uint32_t* tcnt, uint32_t* starts, uint32_t* runs_total, cudaStream_t s) {
+                        uint32_t* tcnt, uint32_t* tfirst, uint32_t* runs_total, cudaStream_t s) {
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
-    rle_count_kernel<T><<<ntiles, 256, 0, s>>>(in, n, tcnt);
+    const int vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
+    rle_count_kernel<T><<<ntiles, 256, 0, s>>>(in, n, vec, tcnt, tfirst);
     scan_tile_offsets<<<1, 1024, 0, s>>>(tcnt, ntiles, runs_total);
-    rle_emit_kernel<T><<<ntiles, 256, 0, s>>>(in, n, tcnt, out, starts);
-    rle_lengths_kernel<T><<<592, 256, 0, s>>>(runs_total, n, starts, out, out_size);
+    rle_emit_kernel<T><<<ntiles, 256, 0, s>>>(in, n, vec, tcnt, tfirst, runs_total, out, out_size);
     return (int)cudaGetLastError();
 }
 
 int launch_rle_encode(const void* in, uint32_t n, int elem, uint8_t* out, unsigned long long* out_size,
-                      uint32_t* tcnt, uint32_t* starts, uint32_t* runs_total, cudaStream_t s) {
-    if (elem == 1) return launch_rle_encode_t<uint8_t>((const uint8_t*)in, n, out, out_size, tcnt, starts, runs_total, s);
-    if (elem == 2) return launch_rle_encode_t<uint16_t>((const uint16_t*)in, n, out, out_size, tcnt, starts, runs_total, s);
-    return launch_rle_encode_t<uint32_t>((const uint32_t*)in, n, out, out_size, tcnt, starts, runs_total, s);
+                      uint32_t* tcnt, uint32_t* tfirst, uint32_t* runs_total, cudaStream_t s) {
+    if (elem == 1) return launch_rle_encode_t<uint8_t>((const uint8_t*)in, n, out, out_size, tcnt, tfirst, runs_total, s);
+    if (elem == 2) return launch_rle_encode_t<uint16_t>((const uint16_t*)in, n, out, out_size, tcnt, tfirst, runs_total, s);
+    return launch_rle_encode_t<uint32_t>((const uint32_t*)in, n, out, out_size, tcnt, tfirst, runs_total, s);
 }
 
-// Run lengths must add up to n; checked on the device.
-__global__ void rle_check_total(const uint32_t* __restrict__ total, uint32_t n, uint32_t* err) {
-    if (*total != n) atomicOr(err, kErrMalformed);
-}
-
-int launch_rle_decode(const uint8_t* in, uint32_t n, int elem, void* out, uint32_t* offs,
-                      uint32_t* tile_scratch, uint32_t* total, uint32_t* err, cudaStream_t s) {
-    ScanSrc a{};
-    a.rle = in;
-    a.elem = elem;
-    a.n = n;  // at most n runs in a valid stream
-    int rc = launch_scan_u32(a, offs, tile_scratch, total, s);
-    if (rc) return rc;
-    rle_check_total<<<1, 1, 0, s>>>(total, n, err);
+int launch_rle_decode(const uint8_t* in, uint32_t n, int elem, void* out, uint32_t* tsum, uint32_t* total,
+                      uint32_t* err, cudaStream_t s) {
+    const uint32_t nrt = (n + kRunTile - 1) / kRunTile;  // tiles of runs, at most n runs
+    rle_sums_kernel<<<min((nrt + 7) / 8, 1184u), 256, 0, s>>>(in, n, (uint32_t)elem, tsum, nrt);
+    scan_tile_offsets<<<1, 1024, 0, s>>>(tsum, nrt, total);
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (elem == 1) rle_expand_kernel<uint8_t><<<ntiles, 256, 0, s>>>(in, offs, n, (uint8_t*)out, err);
-    else if (elem == 2) rle_expand_kernel<uint16_t><<<ntiles, 256, 0, s>>>(in, offs, n, (uint16_t*)out, err);
-    else rle_expand_kernel<uint32_t><<<ntiles, 256, 0, s>>>(in, offs, n, (uint32_t*)out, err);
+    if (elem == 1) rle_expand_kernel<uint8_t><<<ntiles, 256, 0, s>>>(in, tsum, total, n, (uint8_t*)out, err);
+    else if (elem == 2) rle_expand_kernel<uint16_t><<<ntiles, 256, 0, s>>>(in, tsum, total, n, (uint16_t*)out, err);
+    else rle_expand_kernel<uint32_t><<<ntiles, 256, 0, s>>>(in, tsum, total, n, (uint32_t*)out, err);
     return (int)cudaGetLastError();
 }
 

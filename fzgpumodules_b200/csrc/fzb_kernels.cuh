@@ -256,14 +256,11 @@ __global__ void fused_inverse_3d_kernel(InvArgs a);
 // Persistent slab inverse (fzb_slab_inv.cu) for nx >= 32; same results.
 int launch_lq3d_inv_slab(const InvArgs& a, unsigned sms, cudaStream_t s);  // persistent grid: 3 CTAs per SM
 
-// Exclusive scan of u32 values (fzb_coders.cu).  The source is a plain
-// array (count given, or read from *cptr on the device) or the run-length
-// array of an RLE stream.
+// Exclusive scan of u32 values (fzb_coders.cu), the count given or read from
+// *cptr on the device.
 struct ScanSrc {
-    const uint32_t* base;     // plain array
+    const uint32_t* base;
     const uint32_t* cptr;     // optional device count
-    const uint8_t* rle;       // RLE stream instead of base
-    int elem;                 // RLE value width
     uint32_t n;               // upper bound of the count
 };
 int launch_scan_u32(const ScanSrc& a, uint32_t* out, uint32_t* tile_scratch, uint32_t* total,
@@ -271,9 +268,9 @@ int launch_scan_u32(const ScanSrc& a, uint32_t* out, uint32_t* tile_scratch, uin
 
 // RLE and Bitpack (fzb_coders.cu); return cudaError_t values.
 int launch_rle_encode(const void* in, uint32_t n, int elem, uint8_t* out, unsigned long long* out_size,
-                      uint32_t* tcnt, uint32_t* starts, uint32_t* runs_total, cudaStream_t s);
-int launch_rle_decode(const uint8_t* in, uint32_t n, int elem, void* out, uint32_t* offs,
-                      uint32_t* tile_scratch, uint32_t* total, uint32_t* err, cudaStream_t s);
+                      uint32_t* tcnt, uint32_t* tfirst, uint32_t* runs_total, cudaStream_t s);
+int launch_rle_decode(const uint8_t* in, uint32_t n, int elem, void* out, uint32_t* tsum, uint32_t* total,
+                      uint32_t* err, cudaStream_t s);
 int launch_bitpack_encode(const void* in, uint64_t n, int elem, int nbits, uint8_t* nbits_dev,
                           uint8_t* out, unsigned long long* out_size, uint32_t* pmax,
                           unsigned int* done, cudaStream_t s);
