@@ -460,8 +460,8 @@ __global__ void __launch_bounds__(256) sel_bitpack_kernel(SelArgs s) {
 
 // ---------------------------------------------------------------------------
 // Coder 3: Huffman (bklen 1024).  Histogram (CTA per chunk), canonical
-// codebook (one warp per chunk; lane 0 replays the reference's heap
-// construction, the warp gathers leaves and canonizes), coarse encode into
+// codebook (one warp per chunk replays the reference's heap construction,
+// gathers leaves and canonizes), coarse encode into
 // the PHF blob.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) sel_hf_hist_kernel(SelArgs s) {
@@ -487,11 +487,14 @@ __global__ void __launch_bounds__(256) sel_hf_hist_kernel(SelArgs s) {
     else if (t == 0) s.sizes[(size_t)c * kSelCoders + 3] = 0;
 }
 
-// Book for one chunk (one warp).  Lane 0 replays the reference's heap
+// Book for one chunk (one warp).  The warp replays the reference's heap
 // construction exactly (same keys, same sift rules, the first popped node
 // becomes the right child); each merge records the parent of the two merged
 // nodes, and one pass from the root down turns the parents into depths (the
-// code lengths of the reference's tree walk).  The leaf gather and the
+// code lengths of the reference's tree walk).  The merges are a serial chain, so
+// its length is the time: five levels of a sift are decided at once, a lane a
+// node (300 books of up to 1024 symbols: 700 us with one lane sifting level by
+// level, 455 so).  The leaf gather and the
 // canonical codebook are warp-parallel.  Dynamic shared memory (8 KB, so
 // about 25 chunks run per SM): the heap (later the per-symbol lengths), then
 // the parent/depth array.
@@ -538,71 +541,88 @@ __global__ void __launch_bounds__(32) sel_hf_book_kernel(SelArgs s) {
         if (fq[g]) par[leafbase[g] + __popc(nzmask[g] & lt)] = (uint16_t)fq[g];
     __syncwarp();
 
-    if (lane == 0) {
-        // binary min-heap, 1-indexed, of keys freq << 11 | node id (freq <=
-        // 32768, ids < 2048; comparisons look at the frequency only):
-        // insertion stops at a parent whose frequency is <= the new node's;
-        // removal sinks the moved node, taking the right child only when
-        // strictly smaller and swapping only when strictly larger
-        int hs = 0;
-        auto push = [&](uint32_t key) {
-            const uint32_t kf = key >> 11;
-            int i = ++hs;
-            while (i > 1) {
-                const int p = i >> 1;
-                const uint32_t kp = hk[p];
-                if ((kp >> 11) <= kf) break;
-                hk[i] = kp;
-                i = p;
-            }
-            hk[i] = key;
-        };
-        auto pop = [&]() -> uint32_t {
-            const uint32_t top = hk[1];
-            const uint32_t moved = hk[hs];
-            hs--;
-            const uint32_t mf = moved >> 11;
-            int i = 1;
-            while (2 * i <= hs) {
-                const uint2 kk = *reinterpret_cast<const uint2*>(hk + 2 * i);  // both children
-                int ch = 2 * i;
-                uint32_t kc = kk.x;
-                if (ch + 1 <= hs && (kk.y >> 11) < (kc >> 11)) {
-                    ch++;
-                    kc = kk.y;
-                }
-                if (mf > (kc >> 11)) {
-                    hk[i] = kc;
-                    i = ch;
-                } else {
-                    break;
-                }
-            }
-            hk[i] = moved;
-            return top;
-        };
-        for (int i = 0; i < leaves; i++) push(((uint32_t)par[i] << 11) | (uint32_t)i);
-        int nn = leaves;
-        while (hs > 1) {  // the first popped node becomes the right child
-            const uint32_t kr = pop();
-            const uint32_t kl = pop();
+    // binary min-heap, 1-indexed, of keys freq << 11 | node id (freq <=
+    // 32768, ids < 2048; comparisons look at the frequency only): insertion
+    // stops at a parent whose frequency is <= the new node's; removal sinks
+    // the moved node, taking the right child only when strictly smaller and
+    // swapping only when strictly larger.
+    int hs = 0;
+    auto push = [&](uint32_t key) {
+        const int i = ++hs;
+        const int up = i >> (lane < 30u ? lane + 1 : 30u);  // lane j: ancestor j + 1
+        const uint32_t kp = up ? hk[up] : 0u;
+        const uint32_t above = __ballot_sync(full, up != 0 && (kp >> 11) > (key >> 11));
+        const uint32_t cnt = (uint32_t)__ffs(~above) - 1;  // ancestors that move down one level
+        if (lane < cnt) hk[i >> lane] = kp;
+        if (lane == 0) hk[i >> cnt] = key;
+        __syncwarp();
+    };
+    // lane l = 1 .. 31 stands for node l of a five-level subtree (its children
+    // 2l, 2l + 1): with every lane's choice of child and its comparison with the
+    // moved key, the lanes on the sinking path know it from their ancestors'
+    const uint32_t dl = lane ? 31u - __clz(lane) : 0u;
+    uint32_t amask = 0, aexp = 0;  // ancestors' lanes, and which of them lead here by the right child
+    for (uint32_t l = lane; l > 1; l >>= 1) {
+        amask |= 1u << (l >> 1);
+        aexp |= (l & 1u) << (l >> 1);
+    }
+    auto pop = [&]() -> uint32_t {
+        const uint32_t top = hk[1], moved = hk[hs], mf = moved >> 11;
+        hs--;
+        int i = 1;
+        while (true) {
+            const int P = (i << dl) + (int)(lane - (1u << dl));
+            const bool in = lane != 0 && 2 * P <= hs;
+            const uint2 kk = in ? *reinterpret_cast<const uint2*>(hk + 2 * P) : make_uint2(0u, 0u);
+            const bool right = in && 2 * P + 1 <= hs && (kk.y >> 11) < (kk.x >> 11);
+            const uint32_t kc = right ? kk.y : kk.x;
+            const bool sink = in && mf > (kc >> 11);
+            const uint32_t choice = __ballot_sync(full, right), sinks = __ballot_sync(full, sink);
+            const bool move = sink && (choice & amask) == aexp && (sinks & amask) == amask;
+            const uint32_t moves = __ballot_sync(full, move);  // the path's lanes, the last the deepest
+            if (move) hk[P] = kc;
+            if (!moves) break;
+            const uint32_t D = 31u - __clz(moves), dd = 31u - __clz(D);
+            i = 2 * ((i << dd) + (int)(D - (1u << dd))) + (int)((choice >> D) & 1u);
+            if (dd < 4u) break;
+        }
+        if (lane == 0) hk[i] = moved;
+        __syncwarp();
+        return top;
+    };
+    for (int i = 0; i < leaves; i++) push(((uint32_t)par[i] << 11) | (uint32_t)i);
+    int nn = leaves;
+    while (hs > 1) {  // the first popped node becomes the right child
+        const uint32_t kr = pop();
+        const uint32_t kl = pop();
+        if (lane == 0) {
             par[kr & 0x7ffu] = (uint16_t)nn;
             par[kl & 0x7ffu] = (uint16_t)nn;
-            push((((kr >> 11) + (kl >> 11)) << 11) | (uint32_t)nn);
-            nn++;
         }
-        // depths: every parent id is above its children's, so one pass from
-        // the root down, in place; the walk's 58-level stack limit fails the
-        // book when any node lies deeper
-        int maxd = 0;
-        if (nn > 0) {
-            par[nn - 1] = 0;
-            for (int id = nn - 2; id >= 0; id--) {
-                const int d = par[par[id]] + 1;
-                par[id] = (uint16_t)d;
-                maxd = max(maxd, d);
-            }
+        push((((kr >> 11) + (kl >> 11)) << 11) | (uint32_t)nn);
+        nn++;
+    }
+    // depths, in place: every parent id is above its children's, so 32 ids at a
+    // time from the root down; a parent in the same group is read from its lane.
+    // The walk's 58-level stack limit fails the book when any node lies deeper.
+    int maxd = 0;
+    for (int base = nn > 0 ? (nn - 1) & ~31 : -1; base >= 0; base -= 32) {
+        const int id = base + (int)lane;
+        const bool valid = id < nn;
+        const int parent = valid && id < nn - 1 ? (int)par[id] : -1;
+        int dep = !valid || parent < 0 ? 0 : parent >= base + 32 ? (int)par[parent] + 1 : -1;
+        while (__any_sync(full, dep < 0)) {
+            const int d = __shfl_sync(full, dep, parent >= base ? parent - base : 0);
+            if (dep < 0 && d >= 0) dep = d + 1;
         }
+        if (valid) {
+            par[id] = (uint16_t)dep;
+            maxd = max(maxd, dep);
+        }
+        __syncwarp();
+    }
+    maxd = __reduce_max_sync(full, maxd);
+    if (lane == 0) {
         s_ok = maxd <= 58;
         s_nsym = leaves;
     }
