@@ -112,30 +112,10 @@ int geometry(uint64_t n_total, const uint32_t dims[3], Geometry* g) {
     return FZB_OK;
 }
 
-// Dynamic shared memory of the chunk kernel: the staged windows, at least
-// the RZE working set when fused.
-size_t lq_smem_bytes(const Geometry& g, bool fused) {
-    auto gran = [](uint64_t len) { return (((len + 3) / 4 + 1) + 7) & ~(uint64_t)7; };
-    uint64_t per_plane;
-    if (g.ndim == 1) per_plane = gran(kChunkCodes + 1);
-    else if (g.nx <= kChunkCodes) per_plane = gran((uint64_t)g.nx + 1 + kChunkCodes);
-    else per_plane = 2 * gran(kChunkCodes + 1);
-    const uint64_t planes = (g.ndim == 3) ? 2 : 1;
-    size_t bytes = (size_t)(per_plane * planes * 16);
-    const size_t rze_set = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
-    if (fused && bytes < rze_set) bytes = rze_set;
-    return bytes;
-}
-
-int launch_lq(const Geometry& g, bool fused, const FwdArgs& a, size_t smem, uint32_t grid,
-              cudaStream_t s) {
-    const bool rowal = (g.ndim == 1) || (g.nx % 32 == 0);
-    return launch_lq_chunk((int)g.ndim, fused, rowal, a, smem, grid, s) == 0 ? FZB_OK : FZB_E_CUDA;
-}
-
-// Resolves abs_eb / ebx2_r on the device into eb_state (no host sync).
+// Resolves abs_eb / ebx2_r on the device into eb_state (no host sync)
+// and clears the outlier bitmap (when the field has one).
 int resolve_eb(const float* d_in, uint64_t n_total, float eb, int mode, float value_base,
-               const Work& w, float* d_eb_state, cudaStream_t s) {
+               const Work& w, float* d_eb_state, uint32_t* obits, uint32_t obits_words, cudaStream_t s) {
     if (mode != FZB_ABS && !(value_base > 0.0f)) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
@@ -146,10 +126,11 @@ int resolve_eb(const float* d_in, uint64_t n_total, float eb, int mode, float va
         if (parts > kMaxParts) parts = kMaxParts;
         TraceScope ts(s, "minmax_resolve_eb");
         minmax_kernel<<<parts, 256, 0, s>>>(d_in, n_total, w.pmin, w.pmax, w.mm_done, mode, eb,
-                                            d_eb_state);
+                                            d_eb_state, obits, obits_words);
     } else {
         TraceScope ts(s, "resolve_eb");
-        resolve_eb_kernel<<<1, 32, 0, s>>>(mode, eb, value_base, d_eb_state);
+        const uint32_t blocks = 1 + std::min(obits_words / 4096u, 592u);
+        resolve_eb_kernel<<<blocks, 256, 0, s>>>(mode, eb, value_base, d_eb_state, obits, obits_words);
     }
     CK(cudaGetLastError());
     return FZB_OK;
@@ -169,10 +150,10 @@ FwdArgs fwd_args(const Geometry& g, const Work& w, const float* d_in, uint64_t n
     a.ebx2_r = d_eb_state + 2;
     a.radius = (float)(uint16_t)radius;  // the kernel compares against TCode(radius)
     a.zigzag = zigzag;
-    a.two_piece = (g.ndim >= 2 && g.nx > (uint32_t)kChunkCodes) ? 1 : 0;
     a.codes = d_codes;
     a.n_chunks = (uint32_t)chunks_of(n_total);
     a.slots = reinterpret_cast<uint8_t*>(w.codes);
+    a.tcodes = d_codes ? d_codes : w.codes;
     a.sizes = w.sizes;
     a.ocnt = w.ocnt;
     a.obase = w.obase;
@@ -224,13 +205,19 @@ int forward_common(bool fused, const float* d_in, uint64_t n_total, const uint32
     cudaStream_t s = S(stream);
     const uint64_t nch = chunks_of(n_total);
     CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));
-    rc = resolve_eb(d_in, n_total, eb, eb_mode, value_base, w, d_eb_state, s);
-    if (rc) return rc;
-    const FwdArgs a = fwd_args(g, w, d_in, n_total, d_eb_state, radius, zigzag, d_codes, cap);
+    FwdArgs a = fwd_args(g, w, d_in, n_total, d_eb_state, radius, zigzag, d_codes, cap);
     const uint32_t nx = g.nx;
     const bool slab = fused && g.ndim == 3 && nx >= 32 && nx <= 1024 && (nx & (nx - 1)) == 0 &&
                       g.ny % ((uint32_t)kChunkCodes / nx) == 0 && g.nfield == n_total &&
                       !(flags_env() & 1);
+    const bool rows = !fused && g.ndim == 2 && nx % (uint32_t)kChunkCodes == 0 && g.nfield == n_total &&
+                      lq_rows_supported(a) && !(flags_env() & 8);
+    if (!slab && !rows && g.ndim > 1) {
+        a.obits = w.big;
+        a.obits_words = (g.nfield + 31u) / 32u + 1;
+    }
+    rc = resolve_eb(d_in, n_total, eb, eb_mode, value_base, w, d_eb_state, a.obits, a.obits_words, s);
+    if (rc) return rc;
     if (slab) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
@@ -242,8 +229,7 @@ int forward_common(bool fused, const float* d_in, uint64_t n_total, const uint32
             TraceScope ts(s, "lq3d_slab_bs_rze");
             rc = launch_lq3d_slab(a, (unsigned)(2 * sms), s) == 0 ? FZB_OK : FZB_E_CUDA;
         }
-    } else if (!fused && g.ndim == 2 && nx % (uint32_t)kChunkCodes == 0 && g.nfield == n_total &&
-               lq_rows_supported(a) && !(flags_env() & 8)) {
+    } else if (rows) {
         int dev = 0, sms = 148;
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -251,7 +237,9 @@ int forward_common(bool fused, const float* d_in, uint64_t n_total, const uint32
         rc = launch_lq_rows(a, (unsigned)sms, s) == 0 ? FZB_OK : FZB_E_CUDA;
     } else {
         TraceScope ts(s, fused ? "lq_chunk_bs_rze" : "lq_chunk");
-        rc = launch_lq(g, fused, a, lq_smem_bytes(g, fused), (uint32_t)nch, s);
+        if (!fused && g.ndim > 1 && n_total > g.nfield)
+            CK(cudaMemsetAsync(d_codes + g.nfield, 0, 2 * (n_total - g.nfield), s));
+        rc = launch_lq_chunk((int)g.ndim, fused, a, s) == 0 ? FZB_OK : FZB_E_CUDA;
     }
     if (rc) return rc;
     const AsmArgs m = asm_args(w, a, fused, d_rze, d_rze_size, d_err, d_idx, d_count);
@@ -944,8 +932,9 @@ int fzb_huff_decode(const void* d_in, uint64_t in_bytes, uint64_t n, uint32_t bk
 // ---------------------------------------------------------------------------
 // Batched LorenzoQuant -> Bitshuffle -> RZE over many fields: one reset
 // kernel, one value-base kernel for every field, the slab kernel of each
-// field the single-field call codes with one, one persistent chunk kernel
-// over the (field, chunk) units of the others and two assembly kernels,
+// field the single-field call codes with one, one tile kernel over the other
+// 2-D and 3-D fields, one persistent chunk kernel over the (field, chunk) units
+// of all but the slab fields and two assembly kernels,
 // capturable in a CUDA graph.
 // ---------------------------------------------------------------------------
 namespace {
@@ -954,7 +943,7 @@ struct BatchPlan {
     BatchArgs args;
     uint32_t mm_grid_x;
     unsigned lq_grid;
-    size_t smem;
+    uint32_t tile_blocks;
     std::vector<FwdArgs> slab;  // fields coded by a slab kernel (host copies of their arguments)
     unsigned sms = 148;
 };
@@ -975,7 +964,7 @@ struct BatchLayout {
 
 BatchLayout batch_layout(const fzb_batch_field* f, int nf) {
     BatchLayout L;
-    L.desc_bytes = align256(sizeof(BatchField) * (size_t)nf) + align256(8ull * nf + 64);
+    L.desc_bytes = align256(sizeof(BatchField) * (size_t)nf) + align256(12ull * nf + 64);
     size_t off = L.desc_bytes;
     for (int i = 0; i < nf; i++) {
         L.field_off.push_back(off);
@@ -1014,14 +1003,12 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
         *st = FZB_E_WORKSPACE;
         return nullptr;
     }
-    int dev = 0, sms = 148, max_smem = 0;
+    int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    cudaDeviceGetAttribute(&max_smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     uint8_t* base = static_cast<uint8_t*>(d_work);
     std::vector<BatchField> hf((size_t)nfields);
     std::vector<char> is_slab((size_t)nfields, 0);
-    size_t smem = 0;
     uint32_t mm_grid = 1;
     for (int i = 0; i < nfields; i++) {
         const fzb_batch_field& f = fields[i];
@@ -1052,41 +1039,39 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
         if (parts > (uint64_t)kMaxParts) parts = kMaxParts;
         b.mm_parts = b.scan ? (uint32_t)parts : 1u;
         if (b.mm_parts > mm_grid) mm_grid = b.mm_parts;
-        const bool rowal = (g.ndim == 1) || (g.nx % 32 == 0);
-        b.kind = g.ndim == 1 ? 0u : g.ndim == 2 ? (rowal ? 1u : 2u) : (rowal ? 3u : 4u);
+        b.kind = g.ndim - 1;
         b.n_chunks = (uint32_t)chunks_of(f.n_total);
         is_slab[i] = batch_slab_field(g, f.n_total) && !(flags_env() & 1) && !(tuning && tuning->flat_tiles);
-        if (!is_slab[i]) {
-            const size_t sm = lq_smem_bytes(g, true);
-            if (sm > smem) smem = sm;
+        if (!is_slab[i] && g.ndim > 1) {
+            b.a.obits = w.big;
+            b.a.obits_words = (g.nfield + 31u) / 32u + 1;
         }
-    }
-    if ((int)smem > max_smem) {
-        *st = FZB_E_INVALID;
-        return nullptr;
     }
     // field order of the unit ranges: the chunk kernel's fields first (in
     // the tuned order), the slab kernels' fields after them
-    std::vector<uint32_t> order((size_t)nfields), begin((size_t)nfields);
+    std::vector<uint32_t> order((size_t)nfields), begin((size_t)nfields), tiles((size_t)nfields);
     for (int i = 0; i < nfields; i++) order[i] = (uint32_t)i;
     if (tuning && tuning->order == 1)
         std::stable_sort(order.begin(), order.end(),
                          [&](uint32_t x, uint32_t y) { return hf[x].n_chunks > hf[y].n_chunks; });
     std::stable_partition(order.begin(), order.end(), [&](uint32_t x) { return !is_slab[x]; });
-    uint64_t units = 0, lq_units = 0;
+    uint64_t units = 0, lq_units = 0, blocks = 0;
     for (int i = 0; i < nfields; i++) {
         begin[i] = (uint32_t)units;
+        tiles[i] = (uint32_t)blocks;
+        if (hf[order[i]].a.obits) blocks += lq_tile_blocks(hf[order[i]].a);
         units += hf[order[i]].n_chunks;
         if (!is_slab[order[i]]) lq_units = units;
     }
-    if (units >= (1ull << 31)) return nullptr;
-    // descriptors: [BatchField x n][order x n][begin x n][counter]
+    if (units >= (1ull << 31) || blocks >= (1ull << 31)) return nullptr;
+    // descriptors: [BatchField x n][order x n][begin x n][tiles x n][counter]
     std::vector<uint8_t> desc(L.desc_bytes, 0);
     std::memcpy(desc.data(), hf.data(), sizeof(BatchField) * hf.size());
     const size_t o_order = align256(sizeof(BatchField) * (size_t)nfields);
     std::memcpy(desc.data() + o_order, order.data(), 4ull * nfields);
     std::memcpy(desc.data() + o_order + 4ull * nfields, begin.data(), 4ull * nfields);
-    const size_t o_counter = o_order + 8ull * nfields;
+    std::memcpy(desc.data() + o_order + 8ull * nfields, tiles.data(), 4ull * nfields);
+    const size_t o_counter = o_order + 12ull * nfields;
     if (cudaMemcpy(base, desc.data(), desc.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
         *st = FZB_E_CUDA;
         return nullptr;
@@ -1104,6 +1089,7 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
     p->args.total_units = (uint32_t)units;
     p->args.lq_units = (uint32_t)lq_units;
     p->args.counter = reinterpret_cast<uint32_t*>(base + o_counter);
+    p->args.tile_begin = reinterpret_cast<const uint32_t*>(base + o_order + 8ull * nfields);
     p->mm_grid_x = mm_grid;
     p->sms = (unsigned)sms;
     for (int i = 0; i < nfields; i++)
@@ -1112,7 +1098,7 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
     const uint64_t grid = (uint64_t)per_sm * (uint64_t)sms;
     p->lq_grid = (unsigned)(grid < lq_units ? grid : lq_units);
     if (p->lq_grid == 0) p->lq_grid = 1;
-    p->smem = smem;
+    p->tile_blocks = (uint32_t)blocks;
     *st = FZB_OK;
     return p;
 }
@@ -1128,7 +1114,7 @@ int fzb_batch_launch(void* batch, void* stream) {
                                                                       : launch_lq3d_slab(a, 2 * p->sms, s);
         if (rc != 0) return FZB_E_CUDA;
     }
-    return launch_batch_code(p->args, p->lq_grid, p->smem, s) == 0 ? FZB_OK : FZB_E_CUDA;
+    return launch_batch_code(p->args, p->lq_grid, p->tile_blocks, s) == 0 ? FZB_OK : FZB_E_CUDA;
 }
 
 void fzb_batch_destroy(void* batch) { delete static_cast<BatchPlan*>(batch); }

@@ -133,16 +133,27 @@ __device__ __forceinline__ void minmax_body(const float* __restrict__ x, uint64_
     }
 }
 
-__global__ void __launch_bounds__(256) minmax_kernel(const float* __restrict__ x, uint64_t n,
+// Clears the outlier bitmap that the tile kernel sets bits in (its own launch
+// would cost small fields more than this share of the value-base kernel).
+__device__ __forceinline__ void zero_words(uint32_t* p, uint32_t n, uint32_t tid, uint32_t stride) {
+    for (uint32_t i = tid; i < n; i += stride) p[i] = 0u;
+}
+
+// 32 registers: seven blocks an SM, which the scan's bandwidth needs (with 72,
+// three blocks, 512^3 took 190 us instead of 85).
+__global__ void __launch_bounds__(256, 8) minmax_kernel(const float* __restrict__ x, uint64_t n,
                                                      float* __restrict__ pmin, float* __restrict__ pmax,
                                                      unsigned int* __restrict__ done, int mode, float user_eb,
-                                                     float* __restrict__ st) {
+                                                     float* __restrict__ st, uint32_t* zero, uint32_t nzero) {
+    zero_words(zero, nzero, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     minmax_body(x, n, pmin, pmax, done, mode, user_eb, st, blockIdx.x, gridDim.x);
 }
 
 // Error-bound resolution without a scan (ABS, or a caller-provided base).
-__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* __restrict__ st) {
-    if (threadIdx.x == 0) resolve_eb_store(0.f, 0.f, mode, user_eb, vb_given, false, st);
+__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* __restrict__ st, uint32_t* zero,
+                                  uint32_t nzero) {
+    zero_words(zero, nzero, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
+    if (blockIdx.x == 0 && threadIdx.x == 0) resolve_eb_store(0.f, 0.f, mode, user_eb, vb_given, false, st);
 }
 
 // ---------------------------------------------------------------------------
@@ -208,181 +219,37 @@ __device__ __forceinline__ void load_window(float4* Q, const Win& w, const float
     }
 }
 
-// Windows a chunk needs: q(k) (cur) and q(k - nx) (up) for plane z and, in
-// 3-D when some element has z % 8 != 0, for plane z - 1.  Union mode covers
-// cur and up with one window per plane; rows wider than a chunk use two.
-struct Roles {
-    Win cur0, up0, cur1, up1;
-    bool two, z;  // separate up windows / plane z-1 present
-};
-
-__device__ __forceinline__ Win make_win(long long start, long long end, int& soff) {
+__device__ __forceinline__ Win make_win(long long start, long long end) {
     const long long gb = start >= 0 ? (start & ~3LL) : -(((-start) + 3) & ~3LL);
-    const int ng = (int)((end - gb + 3) >> 2);
-    Win w{gb, ng, soff};
-    soff += (ng + 7) & ~7;
-    return w;
+    return Win{gb, (int)((end - gb + 3) >> 2), 0};
 }
 
-__device__ __forceinline__ void make_roles(const FwdArgs& a, int ndim, uint32_t i0, uint32_t cnt,
-                                           bool need_z, Roles& R) {
-    int soff = 0;
-    R.two = (ndim >= 2) && a.two_piece;
-    R.z = (ndim == 3) && need_z;
-    for (int p = 0; p < (R.z ? 2 : 1); p++) {
-        const long long sh = p ? (long long)a.plane : 0;
-        const long long s0 = (long long)i0 - sh, e0 = (long long)i0 + cnt - sh;
-        Win cur, up;
-        if (ndim == 1) {
-            cur = up = make_win(s0 - 1, e0, soff);
-        } else if (!R.two) {
-            cur = up = make_win(s0 - (long long)a.nx - 1, e0, soff);
-        } else {
-            up = make_win(s0 - (long long)a.nx - 1, e0 - (long long)a.nx, soff);
-            cur = make_win(s0 - 1, e0, soff);
-        }
-        if (p == 0) { R.cur0 = cur; R.up0 = up; }
-        else { R.cur1 = cur; R.up1 = up; }
-    }
-}
-
-__device__ __forceinline__ void load_roles(float4* Q, const Roles& R, const float* in, uint32_t nfield,
-                                           float r, bool vec_ok) {
-    load_window(Q, R.cur0, in, nfield, r, vec_ok);
-    if (R.two) load_window(Q, R.up0, in, nfield, r, vec_ok);
-    if (R.z) {
-        load_window(Q, R.cur1, in, nfield, r, vec_ok);
-        if (R.two) load_window(Q, R.up1, in, nfield, r, vec_ok);
-    }
-}
-
-// Single-element q read of element k from role window w.
+// Single-element q read of element k from window w.
 __device__ __forceinline__ float qread(const float4* Q, const Win& w, long long k) {
     const int m = (int)(k - w.gbase);
     const float* Qf = reinterpret_cast<const float*>(Q);
     return Qf[4 * (w.soff + swz(m >> 2)) + (m & 3)];
 }
 
-// Lorenzo delta of element k in the reference's operation order
-// (3-D: z, x, y -- lorenzo_quant_nd.cu:234-246; 2-D: y, x -- :72-77;
-// 1-D: x -- lorenzo_quant.cu:308-321).
+// Lorenzo delta of element k from the input, in the reference's operation
+// order (3-D: z, x, y -- lorenzo_quant_nd.cu:234-246; 2-D: y, x -- :72-77;
+// 1-D: x -- lorenzo_quant.cu:308-321): the value of an outlier, whose code and
+// place the code kernels have settled.
 template <int NDIM>
-__device__ __forceinline__ float delta_xyz(const FwdArgs& a, const float4* Q, const Roles& R, uint32_t k,
-                                           uint32_t x, uint32_t y, uint32_t z) {
-    if (NDIM == 1) {
-        const float q = qread(Q, R.cur0, k);
-        return (k & 1023u) ? __fsub_rn(q, qread(Q, R.cur0, (long long)k - 1)) : q;
-    }
-    const Win& wc = R.cur0;
-    const Win& wu = R.up0;
-    const long long ku = (long long)k - a.nx;
+__device__ __forceinline__ float delta_at(const FwdArgs& a, uint32_t k, float r) {
+    auto q = [&](uint32_t i) { return q_of(__ldg(a.in + i), r); };
+    if (NDIM == 1) return (k & 1023u) ? __fsub_rn(q(k), q(k - 1)) : q(k);
     if (NDIM == 2) {
-        const uint32_t tx = x & 31u, ty = y & 31u;
-        float v0 = qread(Q, wc, k);
-        if (ty) v0 = __fsub_rn(v0, qread(Q, wu, ku));
-        if (!tx) return v0;
-        float v1 = qread(Q, wc, (long long)k - 1);
-        if (ty) v1 = __fsub_rn(v1, qread(Q, wu, ku - 1));
-        return __fsub_rn(v0, v1);
+        const uint32_t y = k / a.nx, x = k - y * a.nx;
+        const bool ty = (y & 31u) != 0;
+        auto v = [&](uint32_t i) { return ty ? __fsub_rn(q(i), q(i - a.nx)) : q(i); };
+        return (x & 31u) ? __fsub_rn(v(k), v(k - 1)) : v(k);
     }
-    const uint32_t tx = x & 7u, ty = y & 7u, tz = z & 7u;
-    const long long kz = (long long)k - a.plane, kuz = ku - a.plane;
-    auto A = [&](const Win& w, long long kk, long long kkz, const Win* wz) -> float {
-        float v = qread(Q, w, kk);
-        return tz ? __fsub_rn(v, qread(Q, *wz, kkz)) : v;
-    };
-    const Win* wcz = &R.cur1;
-    const Win* wuz = &R.up1;
-    float b0 = A(wc, k, kz, wcz);
-    if (tx) b0 = __fsub_rn(b0, A(wc, (long long)k - 1, kz - 1, wcz));
-    if (!ty) return b0;
-    float b1 = A(wu, ku, kuz, wuz);
-    if (tx) b1 = __fsub_rn(b1, A(wu, ku - 1, kuz - 1, wuz));
-    return __fsub_rn(b0, b1);
-}
-
-// Along a run of consecutive elements the x neighbour's terms are the previous
-// element's own, so the run carries them: Run::a0 = A(x, y) and a1 = A(x, y-1)
-// of the last element, with A the z-differenced value (3-D), the y-differenced
-// value (2-D, a0 only) or q itself (1-D).  delta_run gives the same float
-// operations in the same order as delta_xyz.
-struct Run {
-    float a0, a1;
-};
-template <int NDIM>
-__device__ __forceinline__ void run_terms(const FwdArgs& a, const float4* Q, const Roles& R, long long k,
-                                          uint32_t y, uint32_t z, float& a0, float& a1) {
-    if (NDIM == 1) {
-        a0 = qread(Q, R.cur0, k);
-        a1 = 0.0f;
-    } else if (NDIM == 2) {
-        a0 = qread(Q, R.cur0, k);
-        if (y & 31u) a0 = __fsub_rn(a0, qread(Q, R.up0, k - a.nx));
-        a1 = 0.0f;
-    } else {
-        const bool tz = (z & 7u) != 0;
-        a0 = qread(Q, R.cur0, k);
-        if (tz) a0 = __fsub_rn(a0, qread(Q, R.cur1, k - a.plane));
-        a1 = 0.0f;
-        if (y & 7u) {
-            a1 = qread(Q, R.up0, k - a.nx);
-            if (tz) a1 = __fsub_rn(a1, qread(Q, R.up1, k - a.nx - a.plane));
-        }
-    }
-}
-template <int NDIM>
-__device__ __forceinline__ float delta_run(const FwdArgs& a, const float4* Q, const Roles& R, uint32_t k,
-                                           uint32_t x, uint32_t y, uint32_t z, Run& run) {
-    float a0, a1;
-    run_terms<NDIM>(a, Q, R, k, y, z, a0, a1);
-    float d;
-    if (NDIM == 1) {
-        d = (k & 1023u) ? __fsub_rn(a0, run.a0) : a0;
-    } else if (NDIM == 2) {
-        d = (x & 31u) ? __fsub_rn(a0, run.a0) : a0;
-    } else {
-        const bool tx = (x & 7u) != 0;
-        const float b0 = tx ? __fsub_rn(a0, run.a0) : a0;
-        if (y & 7u) {
-            const float b1 = tx ? __fsub_rn(a1, run.a1) : a1;
-            d = __fsub_rn(b0, b1);
-        } else {
-            d = b0;
-        }
-    }
-    run.a0 = a0;
-    run.a1 = a1;
-    return d;
-}
-
-// The granule of 4 window values starting at k (k - gbase a multiple of 4).
-__device__ __forceinline__ float4 qread4(const float4* Q, const Win& w, long long k) {
-    return Q[w.soff + swz((int)((k - w.gbase) >> 2))];
-}
-
-// Element coordinates of field index k, and the step to k + 1 (x fastest),
-// so that a run of consecutive elements needs no divisions.
-struct Xyz {
-    uint32_t x, y, z;
-};
-template <int NDIM>
-__device__ __forceinline__ Xyz xyz_of(const FwdArgs& a, uint32_t k) {
-    if (NDIM == 1) return Xyz{k, 0u, 0u};
-    const uint32_t z = (NDIM == 3) ? k / a.plane : 0u;
-    const uint32_t rem = k - z * a.plane;
-    const uint32_t y = rem / a.nx;
-    return Xyz{rem - y * a.nx, y, z};
-}
-template <int NDIM>
-__device__ __forceinline__ void xyz_next(const FwdArgs& a, Xyz& c) {
-    if (NDIM == 1) return;
-    if (++c.x == a.nx) {
-        c.x = 0;
-        if (++c.y == a.ny && NDIM == 3) {
-            c.y = 0;
-            c.z++;
-        }
-    }
+    const uint32_t z = k / a.plane, rem = k - z * a.plane, y = rem / a.nx, x = rem - y * a.nx;
+    const bool tz = (z & 7u) != 0, tx = (x & 7u) != 0;
+    auto A = [&](uint32_t i) { return tz ? __fsub_rn(q(i), q(i - a.plane)) : q(i); };
+    auto B = [&](uint32_t i) { return tx ? __fsub_rn(A(i), A(i - 1)) : A(i); };
+    return (y & 7u) ? __fsub_rn(B(k), B(k - a.nx)) : B(k);
 }
 
 // Raw little-endian code words of a 32-code group from the packed form
@@ -667,17 +534,6 @@ __global__ void __launch_bounds__(256) assemble_copy_kernel(AsmArgs a) {
         assemble_copy_body(a, c, lane, 32);
 }
 
-// Row-vector path: one thread, 32 consecutive elements of one row, all
-// operands staged in shared memory.  TZ/TY say whether the z / y predecessor
-// lies inside the tile (z % 8 != 0, y % 8 != 0; 2-D: y % 32 != 0).
-struct GroupIn {
-    const float4 *Qc, *Qu, *Qcz, *Quz;
-    int rc, ru, rcz, ruz;
-    float p0;
-    uint32_t j0;
-    float radius;
-};
-
 template <bool ZZ>
 __device__ __forceinline__ uint32_t code_of(float c) {
     const int iv = __float2int_rz(c);
@@ -688,166 +544,43 @@ __device__ __forceinline__ uint32_t code_of(float c) {
     return (uint32_t)iv & 0xffffu;
 }
 
-__device__ __forceinline__ void unpack4(float4 v, float* d) {
-    d[0] = v.x; d[1] = v.y; d[2] = v.z; d[3] = v.w;
-}
-
-template <int NDIM, bool ZZ, bool TZ, bool TY>
-__device__ __forceinline__ void group_codes(const GroupIn& g, uint32_t (&x)[16], uint32_t& om) {
-    float p0 = g.p0, p1 = 0.0f;  // carried a00 / a01 (3-D), v0 (2-D), q (1-D)
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-        float qc[16], qu[16], qcz[16], quz[16];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            unpack4(g.Qc[swz(g.rc + 4 * h + k)], qc + 4 * k);
-            if (NDIM >= 2 && TY) unpack4(g.Qu[swz(g.ru + 4 * h + k)], qu + 4 * k);
-            if (NDIM == 3 && TZ) {
-                unpack4(g.Qcz[swz(g.rcz + 4 * h + k)], qcz + 4 * k);
-                if (TY) unpack4(g.Quz[swz(g.ruz + 4 * h + k)], quz + 4 * k);
-            }
-        }
-#pragma unroll
-        for (int e = 0; e < 16; e++) {
-            const int E = 16 * h + e;
-            float cc;
-            if (NDIM == 3) {
-                const float a00 = TZ ? __fsub_rn(qc[e], qcz[e]) : qc[e];
-                const float b0 = (E & 7) ? __fsub_rn(a00, p0) : a00;
-                p0 = a00;
-                if (TY) {
-                    const float a01 = TZ ? __fsub_rn(qu[e], quz[e]) : qu[e];
-                    const float b1 = (E & 7) ? __fsub_rn(a01, p1) : a01;
-                    p1 = a01;
-                    cc = __fsub_rn(b0, b1);
-                } else {
-                    cc = b0;
-                }
-            } else if (NDIM == 2) {
-                const float v0 = TY ? __fsub_rn(qc[e], qu[e]) : qc[e];
-                cc = E ? __fsub_rn(v0, p0) : v0;
-                p0 = v0;
-            } else {
-                cc = ((g.j0 + E) & 1023u) ? __fsub_rn(qc[e], p0) : qc[e];
-                p0 = qc[e];
-            }
-            const bool qz = fabsf(cc) < g.radius;
-            const uint32_t code = qz ? code_of<ZZ>(cc) : 0u;
-            om |= (qz ? 0u : 1u) << E;
-            if (h == 0) x[e] = code;
-            else x[e] = __byte_perm(x[e], code, 0x5410);
-        }
-    }
-}
-
-template <int NDIM, bool ZZ>
-__device__ __forceinline__ void group_dispatch(const GroupIn& g, bool tz, bool ty, uint32_t (&x)[16],
-                                               uint32_t& om) {
-    if (NDIM == 3) {
-        if (tz) {
-            if (ty) group_codes<NDIM, ZZ, true, true>(g, x, om);
-            else group_codes<NDIM, ZZ, true, false>(g, x, om);
-        } else {
-            if (ty) group_codes<NDIM, ZZ, false, true>(g, x, om);
-            else group_codes<NDIM, ZZ, false, false>(g, x, om);
-        }
-    } else if (NDIM == 2) {
-        if (ty) group_codes<NDIM, ZZ, false, true>(g, x, om);
-        else group_codes<NDIM, ZZ, false, false>(g, x, om);
-    } else {
-        group_codes<NDIM, ZZ, false, false>(g, x, om);
-    }
-}
-
-// Codes of one thread's whole 32-element run when rows are a multiple of 4
-// elements but not of 32 (the element path's case): every window value of the
-// run comes in 16-byte granules (k, k - nx, k - plane and k - plane - nx are
-// all multiples of 4 from the window bases), the coordinates step along the
-// run, and the x neighbour's terms are carried as in delta_run, with the same
-// float operations in the same order.
-template <int NDIM>
-__device__ __forceinline__ void run_codes_vec(const FwdArgs& a, const float4* Q, const Roles& R, uint32_t k0,
-                                              Xyz cz, bool zz, uint32_t (&x)[16], uint32_t& om) {
-    Run run{0.0f, 0.0f};
-    if ((cz.x & (NDIM == 2 ? 31u : 7u)) != 0) run_terms<NDIM>(a, Q, R, (long long)k0 - 1, cz.y, cz.z, run.a0, run.a1);
-#pragma unroll
-    for (int g = 0; g < 8; g++) {
-        const long long kg = (long long)k0 + 4 * g;
-        const float4 c4 = qread4(Q, R.cur0, kg);
-        const float4 u4 = qread4(Q, R.up0, kg - a.nx);
-        float4 cz4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f), uz4 = cz4;
-        if (NDIM == 3 && R.z) {
-            cz4 = qread4(Q, R.cur1, kg - a.plane);
-            uz4 = qread4(Q, R.up1, kg - a.plane - a.nx);
-        }
-        const float cv[4] = {c4.x, c4.y, c4.z, c4.w}, uv[4] = {u4.x, u4.y, u4.z, u4.w};
-        const float czv[4] = {cz4.x, cz4.y, cz4.z, cz4.w}, uzv[4] = {uz4.x, uz4.y, uz4.z, uz4.w};
-#pragma unroll
-        for (int e = 0; e < 4; e++) {
-            const int E = 4 * g + e;
-            float a0 = cv[e], a1 = 0.0f, d;
-            if (NDIM == 2) {
-                if (cz.y & 31u) a0 = __fsub_rn(a0, uv[e]);
-                d = (cz.x & 31u) ? __fsub_rn(a0, run.a0) : a0;
-            } else {
-                const bool tz = (cz.z & 7u) != 0, tx = (cz.x & 7u) != 0;
-                if (tz) a0 = __fsub_rn(a0, czv[e]);
-                const float b0 = tx ? __fsub_rn(a0, run.a0) : a0;
-                if (cz.y & 7u) {
-                    a1 = uv[e];
-                    if (tz) a1 = __fsub_rn(a1, uzv[e]);
-                    d = __fsub_rn(b0, tx ? __fsub_rn(a1, run.a1) : a1);
-                } else {
-                    d = b0;
-                }
-            }
-            run.a0 = a0;
-            run.a1 = a1;
-            const bool qz = fabsf(d) < a.radius;
-            const uint32_t code = qz ? encode_code(d, zz) : 0u;
-            om |= (qz ? 0u : 1u) << E;
-            x[E & 15] |= code << (16 * (E >> 4));
-            xyz_next<NDIM>(a, cz);
-        }
-    }
-}
-
 // ---------------------------------------------------------------------------
-// The chunk kernel.  FUSED=false writes codes; FUSED=true bitshuffles them
-// (16 KiB blocks, element width 2, ballot layout) and RZE-encodes the block
-// straight into the final stream.  ROWAL: rows are multiples of 32 elements,
-// so each thread's 32 codes share (y, z) and the row-vector path applies.
+// The chunk kernels: one CTA per 8192-code chunk.  1-D fields are quantized here
+// (chunk1d_codes); 2-D and 3-D ones read the codes that the tile kernel
+// (fzb_tiles.cu) left in the chunk's slot.  FUSED=false writes the codes (1-D) or
+// only the outliers; FUSED=true bitshuffles the codes (16 KiB blocks, element
+// width 2, ballot layout) and RZE-encodes the block into the slot.
 // ---------------------------------------------------------------------------
 
-// One 8192-code chunk `c` of the field `a` (every thread of the block
-// calls it; it contains block-wide barriers).  Q: dynamic shared memory,
-// s_ws: 16 words, s_obase: one word.  `preset`: windows the caller has
-// already staged (and synchronised), in place of the chunk's own.
 // Register front end for full chunks of 1-D fields (16-byte aligned input):
-// thread t's 32 elements k0 .. k0 + 31 come straight from HBM into
-// registers, are quantized with the packed round (trunc(y + copysign(
-// 0.49999997, y))) and differenced there; a 1024-element block starts at
-// every lane 0, and element k0 - 1 is lane t - 1's last.  Codes come from the
-// magic-number add; per 4-element granule a NaN-propagating max flags
-// outliers, confirmed element by element.  Same codes and outlier set as the
-// window path (group_codes).  (The same front end for 2-D rows, reading the
-// row above from L2, made the batch slower: 3.98 against 3.73 ms.)
-template <int NDIM>
-__device__ __forceinline__ bool reg_front_ok(const FwdArgs& a, uint32_t i0, uint32_t cnt) {
-    return NDIM == 1 && cnt == (uint32_t)kChunkCodes && i0 + (uint32_t)kChunkCodes <= a.nfield &&
-           (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
-}
-
+// thread t's 32 elements k0 .. k0 + 31 come straight from HBM into registers,
+// are quantized with the packed round (trunc(y + copysign(0.49999997, y))) and
+// differenced there; a 1024-element block starts at every lane 0, and element
+// k0 - 1 is lane t - 1's last.  Other chunks are staged as a window in shared
+// memory.  Codes come from the magic-number add; per 4-element granule a
+// NaN-propagating max flags outliers, confirmed element by element.  `valid`:
+// elements of this thread inside the field.
 template <bool ZZ>
-__device__ __forceinline__ void reg_codes_1d(const FwdArgs& a, uint32_t k0, float r, uint32_t (&x)[16],
-                                             uint32_t& om) {
-    const float4* src = reinterpret_cast<const float4*>(a.in + k0);
+__device__ __forceinline__ void chunk1d_codes(const FwdArgs& a, uint32_t k0, float r, bool reg, int valid, float4* Q,
+                                              const Win& w, uint32_t (&x)[16], uint32_t& om) {
     const float R = a.radius;
     Q4 q[8];
+    float left;  // the x predecessor of element 0
+    if (reg) {
+        const float4* src = reinterpret_cast<const float4*>(a.in + k0);
 #pragma unroll
-    for (int g = 0; g < 8; g++) q[g] = quant4(__ldg(src + g), r);
-    const float pl = __shfl_up_sync(0xffffffffu, q[7].b.y, 1);
-    float left = (threadIdx.x & 31u) ? pl : 0.0f;  // the x predecessor of element 0
+        for (int g = 0; g < 8; g++) q[g] = quant4(__ldg(src + g), r);
+        const float pl = __shfl_up_sync(0xffffffffu, q[7].b.y, 1);
+        left = (threadIdx.x & 31u) ? pl : 0.0f;
+    } else {
+        const int g0 = (int)(((long long)k0 - w.gbase) >> 2);  // k0 is a multiple of 32
+#pragma unroll
+        for (int g = 0; g < 8; g++) {
+            const float4 v = 4 * g < valid ? Q[w.soff + swz(g0 + g)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            q[g] = {f2(v.x, v.y), f2(v.z, v.w)};
+        }
+        left = (valid > 0 && (k0 & 1023u)) ? qread(Q, w, (long long)k0 - 1) : 0.0f;
+    }
     uint32_t rw[16];
     om = 0;
 #pragma unroll
@@ -866,166 +599,56 @@ __device__ __forceinline__ void reg_codes_1d(const FwdArgs& a, uint32_t k0, floa
         rw[2 * g] = p0;
         rw[2 * g + 1] = p1;
     }
+    if (valid < 32) {
+        om &= valid > 0 ? (1u << valid) - 1u : 0u;
+#pragma unroll
+        for (int l = 0; l < 16; l++) {
+            if (2 * l >= valid) rw[l] = 0u;
+            else if (2 * l + 1 >= valid) rw[l] &= 0xffffu;
+        }
+    }
     raw_to_packed(rw, x);
 }
 
-// 1-D delta of element k recomputed from the input, for the register front
-// end's outlier records (the window path reads its windows instead).
-__device__ __forceinline__ float reg_delta_1d(const FwdArgs& a, uint32_t k, float r) {
-    const float q = q_of(__ldg(a.in + k), r);
-    return (k & 1023u) ? __fsub_rn(q, q_of(__ldg(a.in + k - 1), r)) : q;
-}
-
-template <int NDIM, bool FUSED, bool ROWAL>
-__device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c, float4* Q, uint32_t* s_ws,
-                                              uint32_t& s_obase, const Roles* preset = nullptr) {
-    const int t = threadIdx.x;
-    const uint32_t i0 = c * (uint32_t)kChunkCodes;
-    const uint32_t cnt = min((uint32_t)kChunkCodes, a.n_total - i0);
-    const float r = *a.ebx2_r;
-    const bool zz = a.zigzag != 0;
-
-    bool need_z = false;
-    if (NDIM == 3 && i0 < a.nfield) {
-        const uint32_t last = min(i0 + cnt, a.nfield) - 1;
-        const uint32_t z0 = i0 / a.plane, z1 = last / a.plane;
-        need_z = (z0 & 7u) || (z1 != z0);
-    }
-    Roles R;
-    const bool reg = !preset && reg_front_ok<NDIM>(a, i0, cnt);  // the same for every thread of the chunk
-    if (preset) {
-        R = *preset;
-    } else if (!reg) {
-        make_roles(a, NDIM, i0, cnt, need_z, R);
-        const bool vec_ok = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
-        load_roles(Q, R, a.in, a.nfield, r, vec_ok);
-        __syncthreads();
-    }
-
-    // ---- pass 1: codes of this thread's 32 consecutive elements ----
-    const uint32_t j0 = 32u * t;
-    const uint32_t k0 = i0 + j0;
-    uint32_t x[16];
-#pragma unroll
-    for (int l = 0; l < 16; l++) x[l] = 0;
-    // row-vector path only for whole groups; partial groups use the element path
-    const bool whole = ROWAL && (j0 + 32 <= cnt) && (k0 + 32 <= a.nfield);
-    uint32_t om = 0;  // outlier bit per element
-    if (reg) {
-        if (zz) reg_codes_1d<true>(a, k0, r, x, om);
-        else reg_codes_1d<false>(a, k0, r, x, om);
-    } else if (whole) {
-        uint32_t ty = 0, tz = 0;
-        if (NDIM == 3) {
-            const uint32_t z = k0 / a.plane, y = (k0 - z * a.plane) / a.nx;
-            ty = y & 7u;
-            tz = z & 7u;
-        } else if (NDIM == 2) {
-            ty = (k0 / a.nx) & 31u;
-        }
-        GroupIn g;
-        g.Qc = Q + R.cur0.soff;
-        g.Qu = Q + R.up0.soff;
-        g.rc = (int)(((long long)k0 - R.cur0.gbase) >> 2);
-        g.ru = (int)(((long long)k0 - a.nx - R.up0.gbase) >> 2);
-        g.Qcz = g.Qc;
-        g.Quz = g.Qu;
-        g.rcz = g.ruz = 0;
-        if (NDIM == 3 && tz) {
-            g.Qcz = Q + R.cur1.soff;
-            g.Quz = Q + R.up1.soff;
-            g.rcz = (int)(((long long)k0 - a.plane - R.cur1.gbase) >> 2);
-            g.ruz = (int)(((long long)k0 - a.plane - a.nx - R.up1.gbase) >> 2);
-        }
-        g.p0 = (NDIM == 1 && (j0 & 1023u)) ? qread(Q, R.cur0, (long long)k0 - 1) : 0.0f;
-        g.j0 = j0;
-        g.radius = a.radius;
-        if (zz) group_dispatch<NDIM, true>(g, tz != 0, ty != 0, x, om);
-        else group_dispatch<NDIM, false>(g, tz != 0, ty != 0, x, om);
-    } else if (NDIM >= 2 && (a.nx & 3u) == 0 && j0 + 32 <= cnt && k0 + 32 <= a.nfield) {
-        run_codes_vec<NDIM>(a, Q, R, k0, xyz_of<NDIM>(a, k0), zz, x, om);
-    } else if (j0 < cnt && k0 < a.nfield) {
-        // element path (rows not a multiple of 4, partial groups): coordinates
-        // step along the run; the unrolled loop keeps x[] in registers
-        Xyz cz = xyz_of<NDIM>(a, k0);
-        Run run{0.0f, 0.0f};
-        {   // the x neighbour of the run's first element, when its tile uses it
-            const bool tx = NDIM == 1 ? (k0 & 1023u) != 0 : (cz.x & (NDIM == 2 ? 31u : 7u)) != 0;
-            if (tx) run_terms<NDIM>(a, Q, R, (long long)k0 - 1, cz.y, cz.z, run.a0, run.a1);
-        }
-#pragma unroll
-        for (int E = 0; E < 32; E++) {
-            const uint32_t k = k0 + E;
-            if (j0 + E < cnt && k < a.nfield) {
-                const float cc = delta_run<NDIM>(a, Q, R, k, cz.x, cz.y, cz.z, run);
-                const bool qz = fabsf(cc) < a.radius;
-                const uint32_t code = qz ? encode_code(cc, zz) : 0u;
-                om |= (qz ? 0u : 1u) << E;
-                x[E & 15] |= code << (16 * (E >> 4));
-            }
-            xyz_next<NDIM>(a, cz);
-        }
-    }
-    const uint32_t nout = __popc(om);
-
-    // ---- outliers: block scan, one staging allocation per chunk ----
-    uint32_t ototal;
-    const uint32_t ooff = block_excl_scan(nout, s_ws, &ototal);
-    if (t == 0) {
-        const uint32_t b = ototal ? atomicAdd(a.ostage_ctr, ototal) : 0u;
-        a.obase[c] = b;
-        a.ocnt[c] = ototal;
-        s_obase = b;
-    }
-    __syncthreads();
-    if (nout && reg) {  // pass 2, register front end: the deltas again from the input
-        uint32_t pos = s_obase + ooff;
-        for (int E = 0; E < 32; E++) {
-            if (!((om >> E) & 1u)) continue;
-            if (pos < a.ostage_cap) {
-                a.ostage_err[pos] = reg_delta_1d(a, k0 + E, r);
-                a.ostage_idx[pos] = k0 + E;
-            }
-            pos++;
-        }
-    } else if (nout) {  // pass 2: recompute this thread's deltas and stage its outliers
-        uint32_t pos = s_obase + ooff;
-        Xyz cz = xyz_of<NDIM>(a, k0);
-        for (int E = 0; E < 32; E++, xyz_next<NDIM>(a, cz)) {
-            const uint32_t k = k0 + E;
-            if (j0 + E < cnt && k < a.nfield) {
-                const float cc = delta_xyz<NDIM>(a, Q, R, k, cz.x, cz.y, cz.z);
-                if (!(fabsf(cc) < a.radius)) {
-                    if (pos < a.ostage_cap) {
-                        a.ostage_err[pos] = cc;
-                        a.ostage_idx[pos] = k;
-                    }
-                    pos++;
-                }
-            }
-        }
-    }
-
-    if (!FUSED) {
-        uint32_t rw[16];
-        packed_to_raw(x, rw);
-        uint16_t* dst = a.codes + k0;
-        if (j0 + 32 <= cnt && (reinterpret_cast<uintptr_t>(a.codes) & 15) == 0) {
-            uint4* d4 = reinterpret_cast<uint4*>(dst);
-#pragma unroll
-            for (int v = 0; v < 4; v++)
-                d4[v] = make_uint4(rw[4 * v], rw[4 * v + 1], rw[4 * v + 2], rw[4 * v + 3]);
-        } else {
-#pragma unroll
-            for (int E = 0; E < 32; E++)
-                if (j0 + E < cnt) dst[E] = (uint16_t)(x[E & 15] >> (16 * (E >> 4)));
+// Outliers of a chunk: one staging allocation in index order, their values
+// recomputed from the input.
+template <int NDIM>
+__device__ __forceinline__ void stage_outliers(const FwdArgs& a, uint32_t c, uint32_t k0, float r, uint32_t om,
+                                               uint32_t* s_ws, uint32_t& s_obase) {
+    if (!__syncthreads_or(om != 0u)) {
+        if (threadIdx.x == 0) {
+            a.obase[c] = 0u;
+            a.ocnt[c] = 0u;
         }
         return;
     }
+    uint32_t total;
+    uint32_t pos = block_excl_scan(__popc(om), s_ws, &total);
+    if (threadIdx.x == 0) {
+        const uint32_t b = atomicAdd(a.ostage_ctr, total);
+        a.obase[c] = b;
+        a.ocnt[c] = total;
+        s_obase = b;
+    }
+    __syncthreads();
+    pos += s_obase;
+    for (; om; om &= om - 1, pos++) {
+        if (pos >= a.ostage_cap) break;
+        const uint32_t k = k0 + (uint32_t)__ffs(om) - 1;
+        a.ostage_err[pos] = delta_at<NDIM>(a, k, r);
+        a.ostage_idx[pos] = k;
+    }
+}
 
-    // ---- Bitshuffle into S, then RZE ----
-    __syncthreads();  // windows are dead past this point
-    uint8_t* base = reinterpret_cast<uint8_t*>(Q);
+// Shared memory of a chunk: the RZE working set; 1-D chunks off the register
+// front end first stage their window there.
+constexpr size_t kChunkSmem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+static_assert(kChunkSmem >= 16 * (kChunkCodes / 4 + 8), "the 1-D window fits");
+
+// Bitshuffle of the chunk's packed codes (cnt of them), RZE, slot.
+__device__ __forceinline__ void encode_slot(const FwdArgs& a, uint32_t c, uint32_t cnt, uint32_t (&x)[16],
+                                            uint8_t* base, uint32_t* s_ws) {
+    const int t = threadIdx.x;
     RzeSmem sm;
     sm.S = reinterpret_cast<uint32_t*>(base);
     sm.O = base + kChunkBytes;
@@ -1048,21 +671,90 @@ __device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c
     write_slot(a.slots, a.sizes, c, sw, (sw >> 31) ? reinterpret_cast<const uint8_t*>(sm.S) : sm.O);
 }
 
-template <int NDIM, bool FUSED, bool ROWAL>
-__global__ void __launch_bounds__(kThreads, 3) lq_chunk_kernel(FwdArgs a) {
+// One chunk `c` of the field `a` (every thread of the block calls it; it
+// contains block-wide barriers).  Q: dynamic shared memory (kChunkSmem),
+// s_ws: 16 words, s_obase: one word.
+template <int NDIM, bool FUSED>
+__device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c, float4* Q, uint32_t* s_ws,
+                                              uint32_t& s_obase) {
+    const int t = threadIdx.x;
+    const uint32_t i0 = c * (uint32_t)kChunkCodes, j0 = 32u * t, k0 = i0 + j0;
+    const uint32_t cnt = min((uint32_t)kChunkCodes, a.n_total - i0);
+    const uint32_t fend = min(a.nfield, i0 + cnt);  // end of the field inside the chunk
+    const int valid = k0 < fend ? (int)min(32u, fend - k0) : 0;
+    const float r = *a.ebx2_r;
+    uint32_t x[16], om = 0;
+    if (NDIM == 1) {
+        const bool al = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
+        const bool reg = al && i0 + (uint32_t)kChunkCodes <= fend;  // the same for every thread
+        Win w{0, 0, 0};
+        if (!reg) {
+            w = make_win((long long)i0 - 1, (long long)i0 + cnt);
+            load_window(Q, w, a.in, a.nfield, r, al);
+            __syncthreads();
+        }
+        if (a.zigzag) chunk1d_codes<true>(a, k0, r, reg, valid, Q, w, x, om);
+        else chunk1d_codes<false>(a, k0, r, reg, valid, Q, w, x, om);
+    } else {
+        if (valid > 0) om = __ldg(a.obits + (k0 >> 5));
+        if (FUSED) {
+            const uint4* s4 = reinterpret_cast<const uint4*>(a.slots + (size_t)c * kChunkBytes) + 4 * t;
+            uint32_t rw[16];
+#pragma unroll
+            for (int v = 0; v < 4; v++) {
+                const uint4 q = 8 * v < valid ? __ldcg(s4 + v) : make_uint4(0u, 0u, 0u, 0u);
+                rw[4 * v] = q.x;
+                rw[4 * v + 1] = q.y;
+                rw[4 * v + 2] = q.z;
+                rw[4 * v + 3] = q.w;
+            }
+            if (valid < 32) {
+#pragma unroll
+                for (int l = 0; l < 16; l++) {
+                    if (2 * l >= valid) rw[l] = 0u;
+                    else if (2 * l + 1 >= valid) rw[l] &= 0xffffu;
+                }
+            }
+            raw_to_packed(rw, x);
+        }
+    }
+    stage_outliers<NDIM>(a, c, k0, r, om, s_ws, s_obase);
+    if (FUSED) {
+        __syncthreads();  // the window is dead past this point
+        encode_slot(a, c, cnt, x, reinterpret_cast<uint8_t*>(Q), s_ws);
+        return;
+    }
+    if (NDIM > 1) return;
+    uint32_t rw[16];
+    packed_to_raw(x, rw);
+    uint16_t* dst = a.codes + k0;
+    if (j0 + 32 <= cnt && (reinterpret_cast<uintptr_t>(a.codes) & 15) == 0) {
+        uint4* d4 = reinterpret_cast<uint4*>(dst);
+#pragma unroll
+        for (int v = 0; v < 4; v++) d4[v] = make_uint4(rw[4 * v], rw[4 * v + 1], rw[4 * v + 2], rw[4 * v + 3]);
+    } else {
+#pragma unroll
+        for (int E = 0; E < 32; E++)
+            if (j0 + E < cnt) dst[E] = (uint16_t)(x[E & 15] >> (16 * (E >> 4)));
+    }
+}
+
+template <int NDIM, bool FUSED>
+__global__ void __launch_bounds__(kThreads, 4) lq_chunk_kernel(FwdArgs a) {
     extern __shared__ float4 Q[];
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_obase;
-    lq_chunk_body<NDIM, FUSED, ROWAL>(a, blockIdx.x, Q, s_ws, s_obase);
+    lq_chunk_body<NDIM, FUSED>(a, blockIdx.x, Q, s_ws, s_obase);
 }
 
 // ---------------------------------------------------------------------------
 // Batched fused compression: many fields, one persistent launch.  CTAs take
 // (field, chunk) units from a global counter in the order `unit_order`
 // lists the fields; every unit runs the same chunk body as the single-field
-// kernel, so each field's bytes equal its own fzb_lq_bs_rze_compress output.
+// kernel (after one launch of the tile kernel over every 2-D and 3-D field), so
+// each field's bytes equal its own fzb_lq_bs_rze_compress output.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads, 3) lq_batch_kernel(BatchArgs b) {
+__global__ void __launch_bounds__(kThreads, 4) lq_batch_kernel(BatchArgs b) {
     extern __shared__ float4 Q[];
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_obase;
@@ -1087,11 +779,9 @@ __global__ void __launch_bounds__(kThreads, 3) lq_batch_kernel(BatchArgs b) {
         const BatchField& f = b.fields[b.unit_order[lo]];
         const uint32_t c = u - b.unit_begin[lo];
         switch (f.kind) {
-            case 0: lq_chunk_body<1, true, true>(f.a, c, Q, s_ws, s_obase); break;
-            case 1: lq_chunk_body<2, true, true>(f.a, c, Q, s_ws, s_obase); break;
-            case 2: lq_chunk_body<2, true, false>(f.a, c, Q, s_ws, s_obase); break;
-            case 3: lq_chunk_body<3, true, true>(f.a, c, Q, s_ws, s_obase); break;
-            default: lq_chunk_body<3, true, false>(f.a, c, Q, s_ws, s_obase); break;
+            case 0: lq_chunk_body<1, true>(f.a, c, Q, s_ws, s_obase); break;
+            case 1: lq_chunk_body<2, true>(f.a, c, Q, s_ws, s_obase); break;
+            default: lq_chunk_body<3, true>(f.a, c, Q, s_ws, s_obase); break;
         }
         if (threadIdx.x == 0) s_unit = next;  // read after the barrier that opens the next iteration
     }
@@ -1101,6 +791,7 @@ __global__ void __launch_bounds__(kThreads, 3) lq_batch_kernel(BatchArgs b) {
 // blockIdx.x < parts(field) take part; the last block of a field resolves it.
 __global__ void __launch_bounds__(256) batch_minmax_kernel(BatchArgs b) {
     const BatchField& f = b.fields[blockIdx.y];
+    zero_words(f.a.obits, f.a.obits_words, blockIdx.x * 256u + threadIdx.x, gridDim.x * 256u);
     if (blockIdx.x >= f.mm_parts) return;
     if (f.mm_parts == 1 && f.scan == 0) {  // ABS, or a caller-provided value base
         if (threadIdx.x == 0) resolve_eb_store(0.f, 0.f, f.mode, f.user_eb, f.vb_given, false, f.eb_state);
@@ -1142,12 +833,12 @@ int launch_batch_scan(const BatchArgs& b, uint32_t mm_grid_x, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-int launch_batch_code(const BatchArgs& b, unsigned lq_grid, size_t smem, cudaStream_t s) {
-    if (b.lq_units) {
-        cudaError_t e = cudaFuncSetAttribute(lq_batch_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        lq_batch_kernel<<<lq_grid, kThreads, smem, s>>>(b);
+int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks, cudaStream_t s) {
+    if (tile_blocks) {
+        const int rc = launch_batch_tiles(b, tile_blocks, s);
+        if (rc) return rc;
     }
+    if (b.lq_units) lq_batch_kernel<<<lq_grid, kThreads, kChunkSmem, s>>>(b);
     batch_assemble_scan_kernel<<<b.nfields, 1024, 0, s>>>(b);
     batch_assemble_copy_kernel<<<b.total_units, 256, 0, s>>>(b);
     return (int)cudaGetLastError();
@@ -1339,29 +1030,20 @@ int launch_lq3d_slab(const FwdArgs& a, unsigned grid, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-template <int NDIM, bool FUSED, bool ROWAL>
-static int launch_lq_t(const FwdArgs& a, size_t smem, unsigned grid, cudaStream_t s) {
-    auto k = lq_chunk_kernel<NDIM, FUSED, ROWAL>;
-    cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return (int)e;
-    k<<<grid, kThreads, smem, s>>>(a);
+template <int NDIM, bool FUSED>
+static int launch_lq_t(const FwdArgs& a, cudaStream_t s) {
+    // chunks that only look their outliers up need no shared memory
+    const size_t smem = FUSED || NDIM == 1 ? kChunkSmem : 0;
+    lq_chunk_kernel<NDIM, FUSED><<<a.n_chunks, kThreads, smem, s>>>(a);
     return (int)cudaGetLastError();
 }
 
-int launch_lq_chunk(int ndim, bool fused, bool rowal, const FwdArgs& a, size_t smem,
-                    unsigned grid, cudaStream_t s) {
-    if (ndim == 1) return fused ? launch_lq_t<1, true, true>(a, smem, grid, s)
-                                : launch_lq_t<1, false, true>(a, smem, grid, s);
-    if (ndim == 2) {
-        if (fused) return rowal ? launch_lq_t<2, true, true>(a, smem, grid, s)
-                                : launch_lq_t<2, true, false>(a, smem, grid, s);
-        return rowal ? launch_lq_t<2, false, true>(a, smem, grid, s)
-                     : launch_lq_t<2, false, false>(a, smem, grid, s);
-    }
-    if (fused) return rowal ? launch_lq_t<3, true, true>(a, smem, grid, s)
-                            : launch_lq_t<3, true, false>(a, smem, grid, s);
-    return rowal ? launch_lq_t<3, false, true>(a, smem, grid, s)
-                 : launch_lq_t<3, false, false>(a, smem, grid, s);
+int launch_lq_chunk(int ndim, bool fused, const FwdArgs& a, cudaStream_t s) {
+    if (ndim == 1) return fused ? launch_lq_t<1, true>(a, s) : launch_lq_t<1, false>(a, s);
+    const int rc = launch_lq_tiles(a, s);
+    if (rc) return rc;
+    if (ndim == 2) return fused ? launch_lq_t<2, true>(a, s) : launch_lq_t<2, false>(a, s);
+    return fused ? launch_lq_t<3, true>(a, s) : launch_lq_t<3, false>(a, s);
 }
 
 // ---------------------------------------------------------------------------

@@ -51,8 +51,10 @@ struct FwdArgs {
     const float* ebx2_r;   // device scalar
     float radius;
     int zigzag;
-    int two_piece;         // separate windows for q(k) and q(k - nx)
     uint16_t* codes;       // codes-only output
+    uint16_t* tcodes;      // 2-D / 3-D tile kernel's output: codes, or the chunk slots (fused)
+    uint32_t* obits;       // 2-D / 3-D: one bit per element, set for outliers (zeroed per call)
+    uint32_t obits_words;  // its words
     float* out_err;
     uint32_t* out_idx;
     uint32_t cap;
@@ -142,12 +144,17 @@ __device__ __forceinline__ bool inv_gated_off(const InvArgs& a) {
 }
 
 __global__ void minmax_kernel(const float* x, uint64_t n, float* pmin, float* pmax,
-                              unsigned int* done, int mode, float user_eb, float* st);
-__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* st);
-// Launches the chunk kernel instance for (ndim, fused, row-aligned); returns
-// a cudaError_t value.
-int launch_lq_chunk(int ndim, bool fused, bool rowal, const FwdArgs& a, size_t smem,
-                    unsigned grid, cudaStream_t s);
+                              unsigned int* done, int mode, float user_eb, float* st, uint32_t* zero,
+                              uint32_t nzero);
+__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* st, uint32_t* zero,
+                                  uint32_t nzero);
+// Quantizes a field of any extents: the tile kernel (2-D, 3-D) and the chunk
+// kernel; returns a cudaError_t value.
+int launch_lq_chunk(int ndim, bool fused, const FwdArgs& a, cudaStream_t s);
+// Codes of a 2-D / 3-D field by tiles into a.tcodes, outliers into a.obits
+// (fzb_tiles.cu); lq_tile_blocks: its CTAs.
+int launch_lq_tiles(const FwdArgs& a, cudaStream_t s);
+uint32_t lq_tile_blocks(const FwdArgs& a);
 // Slab-column fused 3-D kernel (see fzb_forward.cu); `grid` persistent CTAs.
 int launch_lq3d_slab(const FwdArgs& a, unsigned grid, cudaStream_t s);
 // Codes of a 2-D field whose rows are whole chunks (nx % 8192 == 0, no
@@ -291,7 +298,7 @@ struct BatchField {
     float vb_given;
     uint32_t mm_parts;       // blocks of the scan (1 when no scan)
     uint32_t scan;           // 1: REL/NOA scan, 0: resolve only
-    uint32_t kind;           // 0 1-D, 1 2-D rows %32, 2 2-D, 3 3-D rows %32, 4 3-D
+    uint32_t kind;           // 0 1-D, 1 2-D, 2 3-D
     uint32_t n_chunks;
 };
 
@@ -303,13 +310,15 @@ struct BatchArgs {
     uint32_t total_units;        // chunks of every field (the assembly's units)
     uint32_t lq_units;           // the chunk kernel's units: the leading slots, slab fields excluded
     uint32_t* counter;           // unit dispenser
+    const uint32_t* tile_begin;  // first tile-kernel CTA of each slot
 };
 
 // Reset and the value-base scan of every field; then the chunk kernel over
 // the first lq_units units and the assembly of every field.  Fields that take
 // a slab kernel are launched between the two.
 int launch_batch_scan(const BatchArgs& b, uint32_t mm_grid_x, cudaStream_t s);
-int launch_batch_code(const BatchArgs& b, unsigned lq_grid, size_t smem, cudaStream_t s);
+int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks, cudaStream_t s);
+int launch_batch_tiles(const BatchArgs& b, uint32_t blocks, cudaStream_t s);  // fzb_tiles.cu
 
 // Per-chunk coding with a learned selector (fzb_select.cu).
 constexpr int kSelCodes = 32768;            // codes per 64 KiB chunk
