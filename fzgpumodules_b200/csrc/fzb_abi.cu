@@ -467,7 +467,7 @@ int fzb_rze_encode(const void* d_in, uint64_t bytes, void* d_out, uint64_t* d_ou
     a.bytes = bytes;
     a.slots = reinterpret_cast<uint8_t*>(w.codes);
     a.sizes = w.sizes;
-    const int smem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+    const int smem = kRzeEncSmem;
     CK(cudaFuncSetAttribute(rze_encode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     rze_encode_kernel<<<(unsigned)nch, kThreads, smem, s>>>(a);
     CK(cudaGetLastError());

@@ -269,14 +269,13 @@ __device__ __forceinline__ void raw_to_packed(const uint32_t (&rw)[16], uint32_t
     }
 }
 
-// Writes a chunk's encoded bytes (S when stored raw, else O) to its 16 KiB
+// Writes a chunk's encoded bytes to its 16 KiB
 // slot and its size word to sizes[c].
 __device__ __forceinline__ void write_slot(uint8_t* __restrict__ slots, uint32_t* __restrict__ sizes,
-                                           uint32_t c, uint32_t sw, const uint8_t* payload) {
+                                           uint32_t c, uint32_t sw, const RzeSmem& sm) {
     const uint32_t clean = sw & 0x7fffffffu;
     uint4* d4 = reinterpret_cast<uint4*>(slots + (size_t)c * kChunkBytes);
-    const uint4* s4 = reinterpret_cast<const uint4*>(payload);
-    for (uint32_t i = threadIdx.x; i < (clean + 15) / 16; i += kThreads) d4[i] = s4[i];
+    for (uint32_t i = threadIdx.x; i < (clean + 15) / 16; i += kThreads) d4[i] = rze_payload(sm, sw, i);
     if (threadIdx.x == 0) sizes[c] = sw;
 }
 
@@ -642,33 +641,24 @@ __device__ __forceinline__ void stage_outliers(const FwdArgs& a, uint32_t c, uin
 
 // Shared memory of a chunk: the RZE working set; 1-D chunks off the register
 // front end first stage their window there.
-constexpr size_t kChunkSmem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+constexpr size_t kChunkSmem = kRzeEncSmem;
 static_assert(kChunkSmem >= 16 * (kChunkCodes / 4 + 8), "the 1-D window fits");
 
 // Bitshuffle of the chunk's packed codes (cnt of them), RZE, slot.
 __device__ __forceinline__ void encode_slot(const FwdArgs& a, uint32_t c, uint32_t cnt, uint32_t (&x)[16],
                                             uint8_t* base, uint32_t* s_ws) {
-    const int t = threadIdx.x;
-    RzeSmem sm;
-    sm.S = reinterpret_cast<uint32_t*>(base);
-    sm.O = base + kChunkBytes;
-    sm.bm1 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16);
-    sm.bm2 = base + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16 + 2048 + 256);
-    sm.ws = s_ws;
+    const RzeSmem sm = rze_smem(base, s_ws);
     if (cnt == (uint32_t)kChunkCodes) {
         transpose16x2(x);
-#pragma unroll
-        for (int b = 0; b < 16; b++) sm.S[(15 - b) * 256 + t] = x[b];
+        rze_put_planes(sm, x);
     } else {  // partial tail block: Bitshuffle copies it unchanged
         uint32_t rw[16];
         packed_to_raw(x, rw);
-#pragma unroll
-        for (int l = 0; l < 16; l++) sm.S[16 * t + l] = rw[l];
+        rze_put_words(sm, rw);
     }
     __syncthreads();
     const uint32_t sw = rze_encode_chunk(sm, (int)(2 * cnt));
-    write_slot(a.slots, a.sizes, c, sw, (sw >> 31) ? reinterpret_cast<const uint8_t*>(sm.S) : sm.O);
+    write_slot(a.slots, a.sizes, c, sw, sm);
 }
 
 // One chunk `c` of the field `a` (every thread of the block calls it; it
@@ -873,14 +863,7 @@ __global__ void __launch_bounds__(kThreads, 2) lq3d_slab_kernel(FwdArgs a, uint3
     float4* A4 = smem4;                       // A plane: 8192 floats, swizzled granules
     float4* Rw = smem4 + kChunkCodes / 4;     // raw plane prefetch: 8192 floats, swizzled
     const float* Af = reinterpret_cast<const float*>(smem4);
-    RzeSmem sm;
-    uint8_t* rz = base + 8 * kChunkCodes;
-    sm.S = reinterpret_cast<uint32_t*>(rz);
-    sm.O = rz + kChunkBytes;
-    sm.bm1 = reinterpret_cast<uint32_t*>(rz + 2 * kChunkBytes + 16);
-    sm.bm2 = rz + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = reinterpret_cast<uint32_t*>(rz + 2 * kChunkBytes + 16 + 2048 + 256);
-    sm.ws = s_ws;
+    const RzeSmem sm = rze_smem(base + 8 * kChunkCodes, s_ws);
 
     const int t = threadIdx.x;
     const uint32_t nx = a.nx, R = kChunkCodes / nx;
@@ -1003,11 +986,10 @@ __global__ void __launch_bounds__(kThreads, 2) lq3d_slab_kernel(FwdArgs a, uint3
             }
             // Bitshuffle (full chunk) and RZE
             transpose16x2(x);
-#pragma unroll
-            for (int b = 0; b < 16; b++) sm.S[(15 - b) * 256 + t] = x[b];
+            rze_put_planes(sm, x);
             __syncthreads();
             const uint32_t sw = rze_encode_chunk(sm, kChunkBytes);
-            write_slot(a.slots, a.sizes, c, sw, (sw >> 31) ? reinterpret_cast<const uint8_t*>(sm.S) : sm.O);
+            write_slot(a.slots, a.sizes, c, sw, sm);
             __syncthreads();
         }
     }
@@ -1015,7 +997,7 @@ __global__ void __launch_bounds__(kThreads, 2) lq3d_slab_kernel(FwdArgs a, uint3
 }
 
 int launch_lq3d_slab(const FwdArgs& a, unsigned grid, cudaStream_t s) {
-    const size_t smem = 8 * kChunkCodes + 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+    const size_t smem = 8 * kChunkCodes + kRzeEncSmem;
     const uint32_t slabs = a.ny / (kChunkCodes / a.nx), units = slabs * ((a.nz + 7) / 8);
     cudaError_t e;
     if (a.zigzag) {
@@ -1217,26 +1199,19 @@ __global__ void __launch_bounds__(kThreads) rze_encode_kernel(RzeEncArgs a) {
     const uint32_t c = blockIdx.x;
     const uint64_t off = (uint64_t)c * kChunkBytes;
     const int in_size = (int)min((uint64_t)kChunkBytes, a.bytes - off);
-    uint8_t* base = reinterpret_cast<uint8_t*>(Q);
-    RzeSmem sm;
-    sm.S = reinterpret_cast<uint32_t*>(base);
-    sm.O = base + kChunkBytes;
-    sm.bm1 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16);
-    sm.bm2 = base + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16 + 2048 + 256);
-    sm.ws = s_ws;
+    const RzeSmem sm = rze_smem(Q, s_ws);
     const uint8_t* src = a.in + off;
     if (in_size == kChunkBytes && (reinterpret_cast<uintptr_t>(src) & 15) == 0) {
         const uint4* s4 = reinterpret_cast<const uint4*>(src);
         uint4* d4 = reinterpret_cast<uint4*>(sm.S);
-        for (int i = t; i < kChunkBytes / 16; i += kThreads) d4[i] = __ldg(s4 + i);
+        for (int i = t; i < kChunkBytes / 16; i += kThreads) d4[rze_granule(i)] = __ldg(s4 + i);
     } else {
         uint8_t* Sb = reinterpret_cast<uint8_t*>(sm.S);
-        for (int i = t; i < kChunkBytes; i += kThreads) Sb[i] = (i < in_size) ? src[i] : 0;
+        for (int i = t; i < kChunkBytes; i += kThreads) Sb[16 * rze_granule(i >> 4) + (i & 15)] = (i < in_size) ? src[i] : 0;
     }
     __syncthreads();
     const uint32_t sw = rze_encode_chunk(sm, in_size);
-    write_slot(a.slots, a.sizes, c, sw, (sw >> 31) ? reinterpret_cast<const uint8_t*>(sm.S) : sm.O);
+    write_slot(a.slots, a.sizes, c, sw, sm);
 }
 
 }  // namespace fzb

@@ -84,7 +84,7 @@ extern "C" int fzb_rze_encode_noalloc(const void* d_in, uint64_t bytes, void* d_
     a.bytes = bytes;
     a.slots = scratch;
     a.sizes = reinterpret_cast<uint32_t*>(scratch + kSizesOff);
-    const int smem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+    const int smem = kRzeEncSmem;
     static SmemAttr attr;  // the shared-memory attribute, set once per device
     if (ensure_dyn_smem(attr, (const void*)rze_encode_kernel, smem) != cudaSuccess) return FZB_E_CUDA;
     rze_encode_kernel<<<nch, kThreads, smem, s>>>(a);

@@ -33,7 +33,7 @@ namespace fzb {
 namespace {
 
 constexpr uint32_t kPVals = 4096;  // values (u32 codes) per chunk
-constexpr int kPSmem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+constexpr int kPSmem = kRzeEncSmem;
 constexpr int kPMaxParts = 1024;
 
 struct PArgs {
@@ -90,11 +90,10 @@ __device__ __forceinline__ uint32_t pfpl_code(const PArgs& a, float x, float r, 
 // A chunk's encoded bytes (S when stored raw, else O) to its 16 KiB slot,
 // its size word to sizes[c] (the slot layout the assembly kernels read).
 __device__ __forceinline__ void store_slot(uint8_t* __restrict__ slots, uint32_t* __restrict__ sizes, uint32_t c,
-                                           uint32_t sw, const uint8_t* payload) {
+                                           uint32_t sw, const RzeSmem& sm) {
     const uint32_t clean = sw & 0x7fffffffu;
     uint4* d4 = reinterpret_cast<uint4*>(slots + (size_t)c * kChunkBytes);
-    const uint4* s4 = reinterpret_cast<const uint4*>(payload);
-    for (uint32_t i = threadIdx.x; i < (clean + 15) / 16; i += kThreads) d4[i] = s4[i];
+    for (uint32_t i = threadIdx.x; i < (clean + 15) / 16; i += kThreads) d4[i] = rze_payload(sm, sw, i);
     if (threadIdx.x == 0) sizes[c] = sw;
 }
 
@@ -171,14 +170,7 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
     }
 
     // Bitshuffle (ew 2) of the chunk's 8192 half-words, then RZE
-    uint8_t* base = reinterpret_cast<uint8_t*>(smraw);
-    RzeSmem sm;
-    sm.S = reinterpret_cast<uint32_t*>(base);
-    sm.O = base + kChunkBytes;
-    sm.bm1 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16);
-    sm.bm2 = base + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16 + 2048 + 256);
-    sm.ws = s_ws;
+    const RzeSmem sm = rze_smem(smraw, s_ws);
     if (cnt == kPVals) {
         // x[l] = half-word l | half-word (16 + l) << 16 of this thread's 32
         uint32_t x[16];
@@ -188,15 +180,13 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
             x[2 * l + 1] = __byte_perm(d[l], d[8 + l], 0x7632);
         }
         transpose16x2(x);
-#pragma unroll
-        for (int b = 0; b < 16; b++) sm.S[(15 - b) * 256 + t] = x[b];
+        rze_put_planes(sm, x);
     } else {  // partial last block: Bitshuffle leaves it unchanged
-#pragma unroll
-        for (int e = 0; e < 16; e++) sm.S[16 * t + e] = d[e];
+        rze_put_words(sm, d);
     }
     __syncthreads();
     const uint32_t sw = rze_encode_chunk(sm, (int)(4 * cnt));
-    store_slot(a.slots, a.sizes, c, sw, (sw >> 31) ? reinterpret_cast<const uint8_t*>(sm.S) : sm.O);
+    store_slot(a.slots, a.sizes, c, sw, sm);
 }
 
 __global__ void pfpl_cap_count_kernel(uint32_t* count, uint32_t cap) {

@@ -272,14 +272,7 @@ __global__ void __launch_bounds__(kThreads) sel_rze_sub_kernel(SelArgs s) {
     const uint32_t sb = j * (uint32_t)kChunkCodes;  // first code of the block within the chunk
     if (sb >= cnt) return;
     const uint32_t bc = min((uint32_t)kChunkCodes, cnt - sb);
-    uint8_t* base = reinterpret_cast<uint8_t*>(sm4);
-    RzeSmem sm;
-    sm.S = reinterpret_cast<uint32_t*>(base);
-    sm.O = base + kChunkBytes;
-    sm.bm1 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16);
-    sm.bm2 = base + 2 * kChunkBytes + 16 + 2048;
-    sm.bm3 = reinterpret_cast<uint32_t*>(base + 2 * kChunkBytes + 16 + 2048 + 256);
-    sm.ws = s_ws;
+    const RzeSmem sm = rze_smem(sm4, s_ws);
     const uint16_t* src = s.codes + (uint64_t)c * kSelCodes + sb;
     uint32_t rw[16];
     if (bc == (uint32_t)kChunkCodes && (reinterpret_cast<uintptr_t>(s.codes) & 15) == 0) {
@@ -304,19 +297,15 @@ __global__ void __launch_bounds__(kThreads) sel_rze_sub_kernel(SelArgs s) {
         uint32_t x[16];
         sel_raw_to_packed(rw, x);
         transpose16x2(x);
-#pragma unroll
-        for (int b = 0; b < 16; b++) sm.S[(15 - b) * 256 + t] = x[b];
+        rze_put_planes(sm, x);
     } else {  // the block shorter than 16 KiB is copied unchanged
-#pragma unroll
-        for (int l = 0; l < 16; l++) sm.S[16 * t + l] = rw[l];
+        rze_put_words(sm, rw);
     }
     __syncthreads();
     const uint32_t sw = rze_encode_chunk(sm, (int)(2 * bc));
     const uint32_t clean = sw & 0x7fffffffu;
-    const uint8_t* payload = (sw >> 31) ? reinterpret_cast<const uint8_t*>(sm.S) : sm.O;
     uint4* d4 = reinterpret_cast<uint4*>(s.scratch + ((size_t)c * 4 + j) * kChunkBytes);
-    const uint4* p4 = reinterpret_cast<const uint4*>(payload);
-    for (uint32_t i = t; i < (clean + 15) / 16; i += kThreads) d4[i] = p4[i];
+    for (uint32_t i = t; i < (clean + 15) / 16; i += kThreads) d4[i] = rze_payload(sm, sw, i);
     if (t == 0) s.subsizes[(size_t)c * 4 + j] = sw;
 }
 
@@ -1150,7 +1139,7 @@ int launch_sel_coders(const SelArgs& a, uint32_t nlist, unsigned coder_mask, cud
     cudaError_t e;
     if (coder_mask & 1u) {
         TraceScope ts(s, "sel_rze");
-        const int smem = 2 * kChunkBytes + 16 + 2048 + 256 + 32;
+        const int smem = kRzeEncSmem;
         e = cudaFuncSetAttribute(sel_rze_sub_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return (int)e;
         sel_rze_sub_kernel<<<dim3(nlist, 4), kThreads, smem, s>>>(a);
