@@ -335,10 +335,23 @@ __global__ void __launch_bounds__(256) sel_rze_assemble_kernel(SelArgs s) {
         for (uint32_t i = tot; i < padded; i++) dst[i] = 0;
         s.sizes[(size_t)c * kSelCoders + 0] = padded;
     }
+    // payloads by words: dst + off[j] has any byte alignment, the blocks start on
+    // 16-byte boundaries (134 MB of codes: 44 us, byte by byte 111)
     for (uint32_t j = 0; j < nsub; j++) {
         const uint8_t* src = s.scratch + ((size_t)c * 4 + j) * kChunkBytes;
-        const uint32_t len = sw[j] & 0x7fffffffu;
-        for (uint32_t i = threadIdx.x; i < len; i += blockDim.x) dst[off[j] + i] = src[i];
+        const uint32_t* s32 = reinterpret_cast<const uint32_t*>(src);
+        const uint32_t len = sw[j] & 0x7fffffffu, head = min((4u - (off[j] & 3u)) & 3u, len);
+        const uint32_t nw = (len - head) >> 2, r = head & 3u;  // whole destination words after the head
+        if (threadIdx.x < head) dst[off[j] + threadIdx.x] = src[threadIdx.x];
+        if (threadIdx.x < ((len - head) & 3u)) {
+            const uint32_t i = head + 4 * nw + threadIdx.x;
+            dst[off[j] + i] = src[i];
+        }
+        uint32_t* d32 = reinterpret_cast<uint32_t*>(dst + off[j] + head);
+        for (uint32_t i = threadIdx.x; i < nw; i += blockDim.x) {
+            const uint32_t lo = __ldg(s32 + i);
+            d32[i] = r ? __funnelshift_r(lo, __ldg(s32 + i + 1), 8 * r) : lo;
+        }
     }
 }
 
