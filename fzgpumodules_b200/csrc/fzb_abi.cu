@@ -114,7 +114,8 @@ int geometry(uint64_t n_total, const uint32_t dims[3], Geometry* g) {
 
 // Resolves abs_eb / ebx2_r on the device into eb_state (no host sync)
 // and clears the outlier bitmap (when the field has one).
-int resolve_eb(const float* d_in, uint64_t n_total, float eb, int mode, float value_base,
+// n_in of the n_total values are at d_in, the rest are zeros.
+int resolve_eb(const float* d_in, uint64_t n_in, uint64_t n_total, float eb, int mode, float value_base,
                const Work& w, float* d_eb_state, uint32_t* obits, uint32_t obits_words, cudaStream_t s) {
     if (mode != FZB_ABS && !(value_base > 0.0f)) {
         int dev = 0, sms = 148;
@@ -125,8 +126,8 @@ int resolve_eb(const float* d_in, uint64_t n_total, float eb, int mode, float va
         if (parts < 1) parts = 1;
         if (parts > kMaxParts) parts = kMaxParts;
         TraceScope ts(s, "minmax_resolve_eb");
-        minmax_kernel<<<parts, 256, 0, s>>>(d_in, n_total, w.pmin, w.pmax, w.mm_done, mode, eb,
-                                            d_eb_state, obits, obits_words);
+        minmax_kernel<<<parts, 256, 0, s>>>(d_in, n_in, w.pmin, w.pmax, w.mm_done, mode, eb,
+                                            d_eb_state, obits, obits_words, n_in < n_total);
     } else {
         TraceScope ts(s, "resolve_eb");
         const uint32_t blocks = 1 + std::min(obits_words / 4096u, 592u);
@@ -189,7 +190,7 @@ AsmArgs asm_args(const Work& w, const FwdArgs& a, bool fused, void* d_rze, uint6
     return m;
 }
 
-int forward_common(bool fused, const float* d_in, uint64_t n_total, const uint32_t dims[3],
+int forward_common(bool fused, const float* d_in, uint64_t n_in, uint64_t n_total, const uint32_t dims[3],
                    float eb, int eb_mode, float value_base, uint32_t radius, int zigzag,
                    uint16_t* d_codes, float* d_err, uint32_t* d_idx, uint64_t cap,
                    uint32_t* d_count, void* d_rze, uint64_t* d_rze_size, float* d_eb_state,
@@ -199,6 +200,7 @@ int forward_common(bool fused, const float* d_in, uint64_t n_total, const uint32
     if (rc) return rc;
     if (!d_in || !d_count || !d_eb_state || (cap && (!d_err || !d_idx))) return FZB_E_INVALID;
     if (fused ? (!d_rze || !d_rze_size) : !d_codes) return FZB_E_INVALID;
+    if (n_in > n_total || g.nfield > n_in) return FZB_E_INVALID;  // the field itself is read from d_in
     if (eb_mode < FZB_ABS || eb_mode > FZB_NOA || !(eb > 0.0f)) return FZB_E_INVALID;
     Work w = carve(d_work, n_total, cap);
     if (!d_work || work_bytes < w.need) return FZB_E_WORKSPACE;
@@ -216,7 +218,7 @@ int forward_common(bool fused, const float* d_in, uint64_t n_total, const uint32
         a.obits = w.big;
         a.obits_words = (g.nfield + 31u) / 32u + 1;
     }
-    rc = resolve_eb(d_in, n_total, eb, eb_mode, value_base, w, d_eb_state, a.obits, a.obits_words, s);
+    rc = resolve_eb(d_in, n_in, n_total, eb, eb_mode, value_base, w, d_eb_state, a.obits, a.obits_words, s);
     if (rc) return rc;
     if (slab) {
         int dev = 0, sms = 148;
@@ -356,7 +358,7 @@ int fzb_lq_forward(const float* d_in, uint64_t n_total, const uint32_t dims[3], 
                    int eb_mode, float value_base, uint32_t radius, int zigzag, uint16_t* d_codes,
                    float* d_err, uint32_t* d_idx, uint64_t cap, uint32_t* d_count,
                    float* d_eb_state, void* d_work, size_t work_bytes, void* stream) {
-    return forward_common(false, d_in, n_total, dims, eb, eb_mode, value_base, radius, zigzag,
+    return forward_common(false, d_in, n_total, n_total, dims, eb, eb_mode, value_base, radius, zigzag,
                           d_codes, d_err, d_idx, cap, d_count, nullptr, nullptr, d_eb_state,
                           d_work, work_bytes, stream);
 }
@@ -366,7 +368,17 @@ int fzb_lq_bs_rze_compress(const float* d_in, uint64_t n_total, const uint32_t d
                            float* d_err, uint32_t* d_idx, uint64_t cap, uint32_t* d_count,
                            void* d_rze, uint64_t* d_rze_size, float* d_eb_state, void* d_work,
                            size_t work_bytes, void* stream) {
-    return forward_common(true, d_in, n_total, dims, eb, eb_mode, value_base, radius, zigzag,
+    return forward_common(true, d_in, n_total, n_total, dims, eb, eb_mode, value_base, radius, zigzag,
+                          nullptr, d_err, d_idx, cap, d_count, d_rze, d_rze_size, d_eb_state,
+                          d_work, work_bytes, stream);
+}
+
+int fzb_lq_bs_rze_compress_padded(const float* d_in, uint64_t n_in, uint64_t n_total, const uint32_t dims[3],
+                                  float eb, int eb_mode, float value_base, uint32_t radius, int zigzag, float* d_err,
+                                  uint32_t* d_idx, uint64_t cap, uint32_t* d_count, void* d_rze,
+                                  uint64_t* d_rze_size, float* d_eb_state, void* d_work, size_t work_bytes,
+                                  void* stream) {
+    return forward_common(true, d_in, n_in, n_total, dims, eb, eb_mode, value_base, radius, zigzag,
                           nullptr, d_err, d_idx, cap, d_count, d_rze, d_rze_size, d_eb_state,
                           d_work, work_bytes, stream);
 }

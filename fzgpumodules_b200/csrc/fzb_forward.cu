@@ -42,11 +42,12 @@ __device__ __forceinline__ void resolve_eb_store(float lo, float hi, int mode, f
 
 // Block `blk` of `nblk` cooperating blocks: partial min/max into
 // pmin/pmax[blk]; the last block to finish reduces the partials and resolves
-// the error bound into st, then re-arms `done` for the next launch.
+// the error bound into st, then re-arms `done` for the next launch.  with_zero:
+// the range takes in 0 (the padding behind the n values).
 __device__ __forceinline__ void minmax_body(const float* __restrict__ x, uint64_t n, float* __restrict__ pmin,
                                             float* __restrict__ pmax, unsigned int* __restrict__ done, int mode,
                                             float user_eb, float* __restrict__ st, const unsigned blk,
-                                            const unsigned nblk) {
+                                            const unsigned nblk, const bool with_zero) {
     float lo = INFINITY, hi = -INFINITY;
     const bool vec = ((reinterpret_cast<uintptr_t>(x) & 15) == 0);
     const uint64_t nv = vec ? n / 4 : 0;
@@ -128,6 +129,10 @@ __device__ __forceinline__ void minmax_body(const float* __restrict__ x, uint64_
             lo = fminf(lo, slo[w]);
             hi = fmaxf(hi, shi[w]);
         }
+        if (with_zero) {
+            lo = fminf(lo, 0.0f);
+            hi = fmaxf(hi, 0.0f);
+        }
         resolve_eb_store(lo, hi, mode, user_eb, 0.0f, true, st);
         *done = 0;  // ready for the next launch
     }
@@ -144,9 +149,9 @@ __device__ __forceinline__ void zero_words(uint32_t* p, uint32_t n, uint32_t tid
 __global__ void __launch_bounds__(256, 8) minmax_kernel(const float* __restrict__ x, uint64_t n,
                                                      float* __restrict__ pmin, float* __restrict__ pmax,
                                                      unsigned int* __restrict__ done, int mode, float user_eb,
-                                                     float* __restrict__ st, uint32_t* zero, uint32_t nzero) {
+                                                     float* __restrict__ st, uint32_t* zero, uint32_t nzero, int with_zero) {
+    minmax_body(x, n, pmin, pmax, done, mode, user_eb, st, blockIdx.x, gridDim.x, with_zero != 0);
     zero_words(zero, nzero, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
-    minmax_body(x, n, pmin, pmax, done, mode, user_eb, st, blockIdx.x, gridDim.x);
 }
 
 // Error-bound resolution without a scan (ABS, or a caller-provided base).
@@ -787,7 +792,7 @@ __global__ void __launch_bounds__(256) batch_minmax_kernel(BatchArgs b) {
         if (threadIdx.x == 0) resolve_eb_store(0.f, 0.f, f.mode, f.user_eb, f.vb_given, false, f.eb_state);
         return;
     }
-    minmax_body(f.in, f.n, f.pmin, f.pmax, f.mm_done, f.mode, f.user_eb, f.eb_state, blockIdx.x, f.mm_parts);
+    minmax_body(f.in, f.n, f.pmin, f.pmax, f.mm_done, f.mode, f.user_eb, f.eb_state, blockIdx.x, f.mm_parts, false);
 }
 
 __global__ void __launch_bounds__(1024) batch_assemble_scan_kernel(BatchArgs b) {

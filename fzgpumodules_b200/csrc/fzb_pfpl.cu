@@ -39,6 +39,7 @@ constexpr int kPMaxParts = 1024;
 struct PArgs {
     const float* in;
     uint64_t n;
+    uint64_t n_in;  // values at `in`; the rest of the n are zeros
     uint32_t n_chunks;
     const float* st;  // resolved bound: [2] 1 / (2 abs_eb)
     float log2eb, log2eb_r, opp, oopp, threshold;
@@ -111,7 +112,7 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
     const float r = REL ? 0.0f : a.st[2];
 
     float v[16];
-    if (e0 + 16 <= cnt && (reinterpret_cast<uintptr_t>(a.in) & 15) == 0) {
+    if (i0 + e0 + 16 <= a.n_in && (reinterpret_cast<uintptr_t>(a.in) & 15) == 0) {
         const float4* p = reinterpret_cast<const float4*>(a.in + i0 + e0);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -120,7 +121,7 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
         }
     } else {
 #pragma unroll
-        for (int e = 0; e < 16; e++) v[e] = (e0 + e < cnt) ? a.in[i0 + e0 + e] : 0.0f;
+        for (int e = 0; e < 16; e++) v[e] = (i0 + e0 + e < a.n_in) ? a.in[i0 + e0 + e] : 0.0f;
     }
     uint32_t q[16];
     uint32_t om = 0;
@@ -352,6 +353,15 @@ int fzb_pfpl_compress(const float* d_in, uint64_t n, float eb, int eb_mode, floa
                       int zigzag, float threshold, float* d_ovals, uint32_t* d_oidx, uint64_t cap,
                       uint32_t* d_count, void* d_rze, uint64_t* d_rze_size, float* d_eb_state, void* d_work,
                       size_t work_bytes, void* stream) {
+    return fzb_pfpl_compress_padded(d_in, n, n, eb, eb_mode, value_base, radius, zigzag, threshold, d_ovals, d_oidx,
+                                    cap, d_count, d_rze, d_rze_size, d_eb_state, d_work, work_bytes, stream);
+}
+
+int fzb_pfpl_compress_padded(const float* d_in, uint64_t n_in, uint64_t n, float eb, int eb_mode, float value_base,
+                             uint32_t radius, int zigzag, float threshold, float* d_ovals, uint32_t* d_oidx,
+                             uint64_t cap, uint32_t* d_count, void* d_rze, uint64_t* d_rze_size, float* d_eb_state,
+                             void* d_work, size_t work_bytes, void* stream) {
+    if (n_in == 0 || n_in > n) return FZB_E_INVALID;
     if (!d_in || !d_rze || !d_rze_size || !d_count || !d_eb_state || n == 0 || n >= (1ull << 30)) return FZB_E_INVALID;
     if (eb_mode != FZB_ABS && eb_mode != FZB_REL && eb_mode != FZB_NOA) return FZB_E_INVALID;
     if (cap && (!d_ovals || !d_oidx)) return FZB_E_INVALID;
@@ -368,7 +378,8 @@ int fzb_pfpl_compress(const float* d_in, uint64_t n, float eb, int eb_mode, floa
             if (parts > lim) parts = lim;
             if (parts > (uint64_t)kPMaxParts) parts = kPMaxParts;
             if (parts < 1) parts = 1;
-            minmax_kernel<<<(unsigned)parts, 256, 0, s>>>(d_in, n, w.pmin, w.pmax, w.mm_done, FZB_NOA, eb, d_eb_state, nullptr, 0);
+            minmax_kernel<<<(unsigned)parts, 256, 0, s>>>(d_in, n_in, w.pmin, w.pmax, w.mm_done, FZB_NOA, eb, d_eb_state,
+                                                          nullptr, 0, n_in < n);
         } else {
             resolve_eb_kernel<<<1, 32, 0, s>>>(rel ? FZB_ABS : eb_mode, eb, value_base, d_eb_state, nullptr, 0);
         }
@@ -377,6 +388,7 @@ int fzb_pfpl_compress(const float* d_in, uint64_t n, float eb, int eb_mode, floa
     PArgs a{};
     a.in = d_in;
     a.n = n;
+    a.n_in = n_in;
     a.n_chunks = (uint32_t)((n + kPVals - 1) / kPVals);
     a.st = d_eb_state;
     rel_params_p(eb, &a.log2eb, &a.log2eb_r, &a.opp, &a.oopp);

@@ -194,7 +194,7 @@ void LorenzoQuantStage<TInput, TCode>::execute(cudaStream_t stream, MemoryPool* 
 template <typename TInput, typename TCode>
 void LorenzoQuantStage<TInput, TCode>::fusedForward(cudaStream_t stream, MemoryPool* pool, const void* d_in,
                                                     size_t in_bytes, void* d_err, void* d_idx, void* d_count,
-                                                    void* d_rze, uint64_t* d_rze_size) {
+                                                    void* d_rze, uint64_t* d_rze_size, size_t held_bytes) {
     uint32_t dims[3] = {(uint32_t)config_.dims[0], (uint32_t)config_.dims[1], (uint32_t)config_.dims[2]};
     const size_t n = in_bytes / sizeof(TInput);
     num_elements_ = n;
@@ -205,12 +205,13 @@ void LorenzoQuantStage<TInput, TCode>::fusedForward(cudaStream_t stream, MemoryP
     if (n == 0) return;
     const size_t cap = getMaxOutlierCount(n);
     void* w = forwardWorkspace(n, cap, pool, stream);
-    check(fzb_lq_bs_rze_compress(static_cast<const float*>(d_in), n, dims, config_.error_bound,
-                                 (int)config_.eb_mode, config_.precomputed_value_base,
-                                 (uint32_t)config_.quant_radius, config_.zigzag_codes ? 1 : 0,
-                                 static_cast<float*>(d_err), static_cast<uint32_t*>(d_idx), cap,
-                                 static_cast<uint32_t*>(d_count), d_rze, d_rze_size, d_eb_state_, w,
-                                 ws_.size() - kTail, stream),
+    const size_t held = (held_bytes ? held_bytes : in_bytes) / sizeof(TInput);
+    check(fzb_lq_bs_rze_compress_padded(static_cast<const float*>(d_in), held, n, dims, config_.error_bound,
+                                        (int)config_.eb_mode, config_.precomputed_value_base,
+                                        (uint32_t)config_.quant_radius, config_.zigzag_codes ? 1 : 0,
+                                        static_cast<float*>(d_err), static_cast<uint32_t*>(d_idx), cap,
+                                        static_cast<uint32_t*>(d_count), d_rze, d_rze_size, d_eb_state_, w,
+                                        ws_.size() - kTail, stream),
           "LorenzoQuant->Bitshuffle->RZE");
     d_count_ = d_count;
     pending_ = true;

@@ -272,6 +272,7 @@ private:
     void runForward(cudaStream_t stream);
     void runNode(DAGNode* n, cudaStream_t stream);
     void checkBounds(DAGNode* n);
+    bool readsUnpadded(size_t input_size) const;
     const void* prepareInput(const void* d_input, size_t input_size, cudaStream_t stream, size_t* padded);
     void collectMetadata();
     void concatOutputs(void* d_out, size_t capacity, size_t* out_size, cudaStream_t stream);
@@ -337,6 +338,7 @@ private:
     std::vector<DAGNode*> output_nodes_;
     std::vector<BufferMetadata> meta_;
     size_t input_size_hint_, input_alignment_ = 1, input_size_ = 0, original_input_size_ = 0;
+    size_t held_bytes_ = 0;  // bytes in memory of an input that is read unpadded (0: all of it)
     void* pad_buf_ = nullptr;
     size_t pad_bytes_ = 0;
     void* concat_buf_ = nullptr;

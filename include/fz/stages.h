@@ -208,7 +208,8 @@ public:
     // The fused LorenzoQuant -> Bitshuffle -> RZE path runs this stage's
     // forward kernel itself; it reports back what execute() would record.
     void fusedForward(cudaStream_t stream, MemoryPool* pool, const void* d_in, size_t in_bytes,
-                      void* d_err, void* d_idx, void* d_count, void* d_rze, uint64_t* d_rze_size);
+                      void* d_err, void* d_idx, void* d_count, void* d_rze, uint64_t* d_rze_size,
+                      size_t held_bytes = 0);
 
 private:
     void* forwardWorkspace(size_t n, size_t cap, MemoryPool* pool, cudaStream_t stream);
@@ -687,7 +688,7 @@ public:
     // path (uint32 codes) runs this stage's work itself; it records what
     // execute() would.
     void fusedForward(cudaStream_t stream, MemoryPool* pool, const void* d_in, size_t in_bytes, void* d_vals,
-                      void* d_idx, void* d_count, void* d_rze, uint64_t* d_rze_size);
+                      void* d_idx, void* d_count, void* d_rze, uint64_t* d_rze_size, size_t held_bytes = 0);
 
 private:
     bool isInplaceMode() const { return config_.inplace_outliers && config_.eb_mode != ErrorBoundMode::REL; }

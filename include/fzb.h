@@ -148,6 +148,15 @@ int fzb_lq_bs_rze_compress(const float* d_in, uint64_t n_total, const uint32_t d
                            float* d_err, uint32_t* d_idx, uint64_t cap, uint32_t* d_count,
                            void* d_rze, uint64_t* d_rze_size, float* d_eb_state,
                            void* d_work, size_t work_bytes, void* stream);
+/* The same for an input padded with zeros to n_total values of which only the
+ * first n_in (at least the field) are in memory at d_in: the same outputs as
+ * for a padded copy, without the copy.  FZB_E_INVALID when dims make the field
+ * larger than n_in. */
+int fzb_lq_bs_rze_compress_padded(const float* d_in, uint64_t n_in, uint64_t n_total, const uint32_t dims[3],
+                                  float eb, int eb_mode, float value_base, uint32_t radius, int zigzag,
+                                  float* d_err, uint32_t* d_idx, uint64_t cap, uint32_t* d_count,
+                                  void* d_rze, uint64_t* d_rze_size, float* d_eb_state,
+                                  void* d_work, size_t work_bytes, void* stream);
 
 /* Inverse of the chain (rze_stage.cu:846-994 -> bitshuffle_stage.cu:325-349
  * -> lorenzo_quant.cu:494-581).  Single pass for 3-D fields whose rows tile
@@ -321,6 +330,12 @@ int fzb_pfpl_compress(const float* d_in, uint64_t n, float eb, int eb_mode, floa
                       int zigzag, float threshold, float* d_ovals, uint32_t* d_oidx, uint64_t cap,
                       uint32_t* d_count, void* d_rze, uint64_t* d_rze_size, float* d_eb_state, void* d_work,
                       size_t work_bytes, void* stream);
+/* The same for an input padded with zeros to n values of which only the first
+ * n_in are in memory at d_in. */
+int fzb_pfpl_compress_padded(const float* d_in, uint64_t n_in, uint64_t n, float eb, int eb_mode, float value_base,
+                             uint32_t radius, int zigzag, float threshold, float* d_ovals, uint32_t* d_oidx,
+                             uint64_t cap, uint32_t* d_count, void* d_rze, uint64_t* d_rze_size, float* d_eb_state,
+                             void* d_work, size_t work_bytes, void* stream);
 /* Its inverse: RZE decode, Bitshuffle inverse, the chunks' prefix sums and
  * dequantisation in one kernel, then the outlier scatter.  abs_eb as the
  * Quantizer header stores it (ignored for REL).  Malformed streams are
