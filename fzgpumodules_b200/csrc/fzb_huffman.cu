@@ -117,7 +117,10 @@ __global__ void __launch_bounds__(512) hf_histogram_kernel(const uint16_t* __res
 // first bit, and it packs its codes MSB-first into 32-bit words that it ORs
 // into the warp's shared-memory cells (only a lane's first and last word
 // can be shared with a neighbour).  The warp then copies the cells to the
-// partition's slot and clears them for its next partition.
+// partition's slot and clears them for its next partition.  Bound by
+// instruction issue: joining four short codes before they enter the 64-bit
+// accumulator took the 67 M codes of an 8192 x 8192 field (2.4 bits each) from
+// 91 to 64 us.
 constexpr int kHfEncWarps = 8;
 
 template <int SUB>
@@ -157,11 +160,23 @@ __global__ void __launch_bounds__(32 * kHfEncWarps) hf_encode_kernel(const uint1
 #pragma unroll
             for (int k = 0; k < PER; k++) w[k] = base + k < n ? (uint32_t)in[base + k] : 0xffffffffu;
         }
-        uint32_t bits = 0;
+        // codewords right-aligned in w, their lengths four to a word
+        uint32_t bits = 0, len[PER / 4], most = 0;
 #pragma unroll
-        for (int k = 0; k < PER; k++) {
-            w[k] = w[k] < bklen ? book[w[k]] : 0u;  // symbols past the book (or the input) are not coded
-            bits += w[k] >> 27;
+        for (int q = 0; q < PER / 4; q++) {
+            uint32_t sum = 0;
+            len[q] = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                const uint32_t u = w[4 * q + k];
+                const uint32_t e = u < bklen ? book[u] : 0u;  // symbols past the book (or the input) are not coded
+                const uint32_t l = e >> 27;
+                w[4 * q + k] = e & 0x7ffffffu;
+                len[q] |= l << (8 * k);
+                sum += l;
+            }
+            bits += sum;
+            most = max(most, sum);
         }
         uint32_t inc = bits;
 #pragma unroll
@@ -173,17 +188,29 @@ __global__ void __launch_bounds__(32 * kHfEncWarps) hf_encode_kernel(const uint1
         const uint32_t off = inc - bits;
         uint32_t cw = off >> 5, nb = off & 31u;  // acc holds the cell's first nb bits, MSB-aligned
         uint64_t acc = 0;
-#pragma unroll
-        for (int k = 0; k < PER; k++) {
-            const uint32_t len = w[k] >> 27;
-            if (len) acc |= (uint64_t)(w[k] & 0x7ffffffu) << (64 - nb - len);
-            nb += len;
+        auto put = [&](uint32_t code, uint32_t l) {
+            if (l) acc |= (uint64_t)code << (64 - nb - l);
+            nb += l;
             if (nb >= 32) {
                 atomicOr(&cells[cw], (uint32_t)(acc >> 32));
                 cw++;
                 acc <<= 32;
                 nb -= 32;
             }
+        };
+        if (!__any_sync(~0u, most > 32u)) {
+            // every four codes of the warp fit a word: they are joined first, so
+            // the 64-bit accumulator takes one step for four codes
+#pragma unroll
+            for (int q = 0; q < PER / 4; q++) {
+                const uint32_t l0 = len[q] & 0xffu, l1 = (len[q] >> 8) & 0xffu, l2 = (len[q] >> 16) & 0xffu,
+                               l3 = len[q] >> 24, l23 = l2 + l3;
+                const uint32_t lo = (w[4 * q + 2] << l3) | w[4 * q + 3], hi = (w[4 * q] << l1) | w[4 * q + 1];
+                put(l23 < 32u ? (hi << l23) | lo : lo, l0 + l1 + l23);
+            }
+        } else {
+#pragma unroll
+            for (int k = 0; k < PER; k++) put(w[k], (len[k >> 2] >> (8 * (k & 3))) & 0xffu);
         }
         if (nb) atomicOr(&cells[cw], (uint32_t)(acc >> 32));  // zero bits of other lanes OR in harmlessly
         __syncwarp();
