@@ -1059,21 +1059,23 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
             b.a.obits_words = (g.nfield + 31u) / 32u + 1;
         }
     }
-    // field order of the unit ranges: the chunk kernel's fields first (in
-    // the tuned order), the slab kernels' fields after them
+    // field order of the unit ranges: the chunk kernels' fields first (1-D, then
+    // the others, in the tuned order), the slab kernels' fields after them
     std::vector<uint32_t> order((size_t)nfields), begin((size_t)nfields), tiles((size_t)nfields);
     for (int i = 0; i < nfields; i++) order[i] = (uint32_t)i;
     if (tuning && tuning->order == 1)
         std::stable_sort(order.begin(), order.end(),
                          [&](uint32_t x, uint32_t y) { return hf[x].n_chunks > hf[y].n_chunks; });
     std::stable_partition(order.begin(), order.end(), [&](uint32_t x) { return !is_slab[x]; });
-    uint64_t units = 0, lq_units = 0, blocks = 0;
+    std::stable_partition(order.begin(), order.end(), [&](uint32_t x) { return hf[x].kind == 0; });
+    uint64_t units = 0, lq_units = 0, one_units = 0, blocks = 0;
     for (int i = 0; i < nfields; i++) {
         begin[i] = (uint32_t)units;
         tiles[i] = (uint32_t)blocks;
         if (hf[order[i]].a.obits) blocks += lq_tile_blocks(hf[order[i]].a);
         units += hf[order[i]].n_chunks;
         if (!is_slab[order[i]]) lq_units = units;
+        if (hf[order[i]].kind == 0) one_units = units;
     }
     if (units >= (1ull << 31) || blocks >= (1ull << 31)) return nullptr;
     // descriptors: [BatchField x n][order x n][begin x n][tiles x n][counter]
@@ -1100,16 +1102,17 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
     p->args.unit_begin = reinterpret_cast<const uint32_t*>(base + o_order + 4ull * nfields);
     p->args.total_units = (uint32_t)units;
     p->args.lq_units = (uint32_t)lq_units;
+    p->args.one_units = (uint32_t)one_units;
     p->args.counter = reinterpret_cast<uint32_t*>(base + o_counter);
     p->args.tile_begin = reinterpret_cast<const uint32_t*>(base + o_order + 8ull * nfields);
     p->mm_grid_x = mm_grid;
     p->sms = (unsigned)sms;
     for (int i = 0; i < nfields; i++)
         if (is_slab[order[i]]) p->slab.push_back(hf[order[i]].a);
-    const int per_sm = (tuning && tuning->ctas_per_sm > 0) ? tuning->ctas_per_sm : 2;
-    const uint64_t grid = (uint64_t)per_sm * (uint64_t)sms;
-    p->lq_grid = (unsigned)(grid < lq_units ? grid : lq_units);
-    if (p->lq_grid == 0) p->lq_grid = 1;
+    // pairs of CTAs an SM; the default is what the chunk kernels' registers leave
+    // room for
+    const int pairs = (tuning && tuning->ctas_per_sm > 0) ? tuning->ctas_per_sm : 2;
+    p->lq_grid = (unsigned)std::min<uint64_t>(2ull * (uint64_t)pairs * (uint64_t)sms, 0x7fffffffull);
     p->tile_blocks = (uint32_t)blocks;
     *st = FZB_OK;
     return p;

@@ -734,8 +734,14 @@ __device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c
     }
 }
 
+// CTAs an SM: the chunk coder waits at its barriers, so five resident chunks of the
+// codes the tile kernel left beat four (500 x 500 x 100: 54.2 us against 56.3; 65.8
+// with six, which spill), and the 1-D front end, with eight granules in flight,
+// needs the registers of four.
+constexpr int chunk_ctas(int ndim) { return ndim == 1 ? 4 : 5; }
+
 template <int NDIM, bool FUSED>
-__global__ void __launch_bounds__(kThreads, 4) lq_chunk_kernel(FwdArgs a) {
+__global__ void __launch_bounds__(kThreads, chunk_ctas(NDIM)) lq_chunk_kernel(FwdArgs a) {
     extern __shared__ float4 Q[];
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_obase;
@@ -743,27 +749,36 @@ __global__ void __launch_bounds__(kThreads, 4) lq_chunk_kernel(FwdArgs a) {
 }
 
 // ---------------------------------------------------------------------------
-// Batched fused compression: many fields, one persistent launch.  CTAs take
-// (field, chunk) units from a global counter in the order `unit_order`
-// lists the fields; every unit runs the same chunk body as the single-field
-// kernel (after one launch of the tile kernel over every 2-D and 3-D field), so
-// each field's bytes equal its own fzb_lq_bs_rze_compress output.
+// Batched fused compression: many fields, one persistent launch for the 1-D ones
+// and one for the others.  CTAs take (field, chunk) units from a global counter
+// in the order `unit_order` lists the fields; every unit runs the same chunk body
+// as the single-field kernel (after one launch of the tile kernel over every 2-D
+// and 3-D field), so each field's bytes equal its own fzb_lq_bs_rze_compress
+// output.
 // ---------------------------------------------------------------------------
+// ONE_D: the units of the 1-D fields, the first b.one_units; else the 2-D and 3-D
+// fields' units after them.  One kernel for all of them was as large as its three
+// bodies and took 519 us for twenty fields of 0.96 GB with two CTAs an SM; these
+// take 194 + 150 with the four an SM that their registers leave room for (154
+// for the second with five).
+template <bool ONE_D>
 __global__ void __launch_bounds__(kThreads, 4) lq_batch_kernel(BatchArgs b) {
     extern __shared__ float4 Q[];
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_obase;
     __shared__ uint32_t s_unit;
+    uint32_t* counter = b.counter + (ONE_D ? 0 : 1);
+    const uint32_t base = ONE_D ? 0u : b.one_units, end = ONE_D ? b.one_units : b.lq_units;
     // thread 0 takes the next unit's ticket as this one starts, so the
     // dispenser's round trip overlaps the chunk instead of preceding it
     uint32_t next = 0;
-    if (threadIdx.x == 0) s_unit = atomicAdd(b.counter, 1u);
+    if (threadIdx.x == 0) s_unit = base + atomicAdd(counter, 1u);
     for (;;) {
         __syncthreads();
         const uint32_t u = s_unit;
         __syncthreads();  // s_unit is rewritten at the end of this iteration
-        if (u >= b.lq_units) break;
-        if (threadIdx.x == 0) next = atomicAdd(b.counter, 1u);
+        if (u >= end) break;
+        if (threadIdx.x == 0) next = base + atomicAdd(counter, 1u);
         // field = last slot whose unit_begin <= u (fields in unit_order)
         uint32_t lo = 0, hi = b.nfields;
         while (hi - lo > 1) {
@@ -773,11 +788,9 @@ __global__ void __launch_bounds__(kThreads, 4) lq_batch_kernel(BatchArgs b) {
         }
         const BatchField& f = b.fields[b.unit_order[lo]];
         const uint32_t c = u - b.unit_begin[lo];
-        switch (f.kind) {
-            case 0: lq_chunk_body<1, true>(f.a, c, Q, s_ws, s_obase); break;
-            case 1: lq_chunk_body<2, true>(f.a, c, Q, s_ws, s_obase); break;
-            default: lq_chunk_body<3, true>(f.a, c, Q, s_ws, s_obase); break;
-        }
+        if (ONE_D) lq_chunk_body<1, true>(f.a, c, Q, s_ws, s_obase);
+        else if (f.kind == 1) lq_chunk_body<2, true>(f.a, c, Q, s_ws, s_obase);
+        else lq_chunk_body<3, true>(f.a, c, Q, s_ws, s_obase);
         if (threadIdx.x == 0) s_unit = next;  // read after the barrier that opens the next iteration
     }
 }
@@ -818,7 +831,7 @@ __global__ void batch_reset_kernel(BatchArgs b) {
     if (threadIdx.x == 0) {
         *f.a.ostage_ctr = 0;
         *f.a.err = 0;
-        if (blockIdx.x == 0) *b.counter = 0;
+        if (blockIdx.x == 0) b.counter[0] = b.counter[1] = 0;
     }
 }
 
@@ -833,7 +846,9 @@ int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks
         const int rc = launch_batch_tiles(b, tile_blocks, s);
         if (rc) return rc;
     }
-    if (b.lq_units) lq_batch_kernel<<<lq_grid, kThreads, kChunkSmem, s>>>(b);
+    const unsigned one = b.one_units, rest = b.lq_units - b.one_units;
+    if (one) lq_batch_kernel<true><<<min(lq_grid, one), kThreads, kChunkSmem, s>>>(b);
+    if (rest) lq_batch_kernel<false><<<min(lq_grid, rest), kThreads, kChunkSmem, s>>>(b);
     batch_assemble_scan_kernel<<<b.nfields, 1024, 0, s>>>(b);
     batch_assemble_copy_kernel<<<b.total_units, 256, 0, s>>>(b);
     return (int)cudaGetLastError();

@@ -309,7 +309,8 @@ struct BatchArgs {
     const uint32_t* unit_begin;  // first unit (chunk) of each slot
     uint32_t total_units;        // chunks of every field (the assembly's units)
     uint32_t lq_units;           // the chunk kernel's units: the leading slots, slab fields excluded
-    uint32_t* counter;           // unit dispenser
+    uint32_t one_units;          // of them the 1-D fields' units, which come first
+    uint32_t* counter;           // unit dispensers: 1-D, 2-D and 3-D
     const uint32_t* tile_begin;  // first tile-kernel CTA of each slot
 };
 

@@ -125,7 +125,7 @@ __device__ __forceinline__ void feat_code(FeatAcc& f, uint32_t u, uint32_t pv, b
     }
 }
 
-__global__ void __launch_bounds__(256) sel_features_kernel(const uint16_t* __restrict__ codes, uint64_t n,
+__global__ void __launch_bounds__(256, 5) sel_features_kernel(const uint16_t* __restrict__ codes, uint64_t n,
                                                            float* __restrict__ feats) {
     __shared__ uint32_t h1024[1024];
     __shared__ uint32_t hlo_x[256], hhi_x[256];  // low bytes of codes >= 256, high bytes of codes >= 1024
@@ -261,7 +261,7 @@ __global__ void __launch_bounds__(256) sel_features_kernel(const uint16_t* __res
 // 16 KiB block into scratch; the assembly kernel writes the chunk's RZE
 // stream ([u32 orig][u32 nsub][u32 size x nsub][payloads], padded to 4).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) sel_rze_sub_kernel(SelArgs s) {
+__global__ void __launch_bounds__(kThreads, 6) sel_rze_sub_kernel(SelArgs s) {
     extern __shared__ uint4 sm4[];
     __shared__ uint32_t s_ws[16];
     const int ci = sel_chunk(s, 0);

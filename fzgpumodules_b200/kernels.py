@@ -515,7 +515,7 @@ class _BatchField(C.Structure):
 
 
 class BatchTuning(C.Structure):
-    """fzb_batch_tuning: CTAs per SM, dispatch order, flat tiles for
+    """fzb_batch_tuning: pairs of CTAs per SM, dispatch order, flat tiles for
     slab-shaped fields, value-base scan blocks per SM (0 = default)."""
     _fields_ = [("ctas_per_sm", C.c_int), ("order", C.c_int), ("flat_tiles", C.c_int), ("scan_parts", C.c_int)]
 

@@ -397,18 +397,18 @@ int fzb_status_from_bits(uint32_t bits, int* rerun_exact);
 
 /* ------------------------------------------------------------------------
  * Batched compression of many fields (no reference counterpart: it runs the
- * chain of fzb_lq_bs_rze_compress for every field in five launches --
- * reset, one value-base scan over all fields, one persistent chunk kernel
- * over every (field, chunk) unit, two assembly kernels -- plus one slab
- * kernel launch per field the single-field call codes with a slab kernel
- * (3-D, nx a power of two in [32, 1024], whole-row chunks), so a batch is one
- * CUDA graph node group).  Each field's outputs are
+ * chain of fzb_lq_bs_rze_compress for every field in at most seven launches --
+ * reset, one value-base scan over all fields, the codes of every 2-D and 3-D
+ * field, one persistent chunk kernel over the 1-D fields' chunks and one over
+ * the others', two assembly kernels -- plus one slab kernel launch per field
+ * the single-field call codes with a slab kernel (3-D, nx a power of two in
+ * [32, 1024], whole-row chunks), so a batch is one CUDA graph node group).  Each field's outputs are
  * byte-identical to its own fzb_lq_bs_rze_compress call.
  *
  * fzb_batch_create validates the fields, writes the descriptors into
  * d_work (synchronous copy) and returns a handle; fzb_batch_launch only
  * enqueues (capturable; the buffers named at create time are reused on
- * every launch).  Tuning: CTAs per SM of the persistent kernel, and the
+ * every launch).  Tuning: CTAs per SM of the persistent kernels, and the
  * order fields are dispensed in (0 as given, 1 largest first); neither
  * changes any output byte.  fzb_batch_autotune times the candidates on the
  * given fields and returns the fastest.
@@ -432,7 +432,7 @@ typedef struct fzb_batch_field {
 } fzb_batch_field;
 
 /* Launch shape of a batch (zero fields take the defaults):
- * ctas_per_sm  CTAs per SM of the persistent chunk kernel (default 2);
+ * ctas_per_sm  pairs of CTAs per SM of the persistent chunk kernels (default 2);
  * order        1: the chunk kernel dispenses the largest fields first;
  * flat_tiles   1: slab-shaped 3-D fields go through the chunk kernel's flat
  *              8192-element chunks instead of the slab kernel's R-row x
