@@ -1,0 +1,42 @@
+"""RLE at the edges of its tiles (4096 elements encoded, 1024 runs decoded)
+against the oracle, exact bytes: sizes around a tile, a run that ends at, before
+and after its edge, runs over whole tiles, one run and no runs shorter than two."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import oracle as O
+
+pytestmark = pytest.mark.gpu
+
+TDT = {np.uint8: torch.uint8, np.uint16: torch.uint16, np.uint32: torch.int32}
+
+
+def _runs(lengths, dtype):
+    v = (np.arange(len(lengths)) % 7 + 1).astype(dtype)
+    return np.repeat(v, lengths)
+
+
+def _cases(dtype):
+    rng = np.random.default_rng(5)
+    for n in (1, 2, 4095, 4096, 4097, 8191, 3 * 4096 + 1):
+        yield _runs([n], dtype)                                   # one run
+        yield (np.arange(n) % 5).astype(dtype)                    # no run of two
+        yield np.repeat(rng.integers(0, 9, n).astype(dtype), 2)[:n]
+    for d in (-1, 0, 1):
+        yield _runs([4096 + d, 4096, 1, 4096 * 5 + d, 63, 64, 65, 2], dtype)
+        yield _runs([1] * (1024 + d), dtype)                      # decoder tiles
+        yield _runs([1] * (2047 + d) + [5000], dtype)
+        yield _runs([3] * 1023 + [70000 + d] + [1, 2] * 700, dtype)
+
+
+@pytest.mark.parametrize("dtype", [np.uint8, np.uint16, np.uint32])
+def test_rle_tile_edges(cuda, dtype):
+    from fzgpumodules_b200 import kernels as K
+    for a in _cases(dtype):
+        t = torch.from_numpy(a.view(np.int32) if dtype == np.uint32 else a).to(cuda)
+        ref = O.rle_encode(a)
+        enc, _ = K.rle_encode(t)
+        assert np.array_equal(enc.cpu().numpy(), ref)
+        dec = K.rle_decode(enc, a.size, TDT[dtype])
+        assert np.array_equal(dec.cpu().numpy().view(dtype), a)
