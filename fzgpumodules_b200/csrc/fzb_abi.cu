@@ -298,8 +298,7 @@ int exact_inverse(const InvArgs& a, const Geometry& g, cudaStream_t s) {
     if (a.obits) {
         TraceScope ts(s, "mark_outliers");
         const uint64_t want = std::min<uint64_t>((a.cap + 255ull) / 256u, std::min(lim, 4096u));
-        mark_outliers_kernel<<<(unsigned)want, 256, 0, s>>>(a);
-        CK(cudaGetLastError());
+        CK(launch_dependent(mark_outliers_kernel, (unsigned)want, 256, 0, s, a));
     }
     TraceScope ts(s, "lq_inverse");
     return launch_lq_inverse(a, (int)g.ndim, lim, s) == 0 ? FZB_OK : FZB_E_CUDA;
@@ -611,9 +610,8 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
     {
         TraceScope ts(s, "rze_decode_bitunshuffle");
         const uint64_t lim = a.gate ? 4ull * (uint64_t)sm_count() : nch;
-        rze_decode_codes_kernel<<<(unsigned)std::min<uint64_t>(nch, lim), kThreads, 0, s>>>(a);
+        CK(launch_dependent(rze_decode_codes_kernel, (unsigned)std::min<uint64_t>(nch, lim), kThreads, 0, s, a));
     }
-    CK(cudaGetLastError());
     rc = exact_inverse(a, g, s);
     if (rc || (flags & (FZB_NO_SYNC | FZB_DEVICE_FALLBACK))) return rc;
     uint32_t bits = 0;

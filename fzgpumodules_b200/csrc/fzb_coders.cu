@@ -148,6 +148,7 @@ template <typename T>
 __global__ void __launch_bounds__(256) rle_count_kernel(const T* __restrict__ in, uint32_t n, int vec,
                                                         uint32_t* __restrict__ tcnt, uint32_t* __restrict__ tfirst) {
     __shared__ uint32_t w[8], f[8];
+    follow();
     T v[16];
     const uint32_t b = blockIdx.x * kScanTile + threadIdx.x * 16;
     const uint32_t m = run_starts16(in, n, b, vec != 0, v);
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(256) rle_emit_kernel(const T* __restrict__ in,
     __shared__ uint32_t ws[16];
     __shared__ uint32_t s_start[kScanTile + 1];
     __shared__ T s_val[kScanTile];
+    follow();
     const uint32_t R = *total, t = threadIdx.x;
     const uint32_t vbytes = R * (uint32_t)sizeof(T), valigned = (vbytes + 3u) & ~3u;
     T* values = reinterpret_cast<T*>(out + 4);
@@ -270,6 +272,7 @@ __device__ __forceinline__ const uint32_t* rle_lens(const uint8_t* in, uint32_t 
 // Sum of each tile of runs, a warp a tile.
 __global__ void __launch_bounds__(256) rle_sums_kernel(const uint8_t* __restrict__ in, uint32_t n, uint32_t elem,
                                                        uint32_t* __restrict__ tsum, uint32_t ntiles) {
+    follow();
     const uint32_t R = rle_runs(in, n), lane = threadIdx.x & 31u;
     const uint32_t* lens = rle_lens(in, elem);
     for (uint32_t tile = blockIdx.x * 8 + (threadIdx.x >> 5); tile < ntiles; tile += gridDim.x * 8) {
@@ -291,6 +294,7 @@ __global__ void __launch_bounds__(256) rle_expand_kernel(const uint8_t* __restri
     constexpr uint32_t kLong = 64;  // runs from this length on are filled by the whole block
     __shared__ __align__(16) T s_out[kScanTile];
     __shared__ uint32_t ws[16], s_long[kScanTile / kLong + 2], s_nlong;
+    follow();
     const uint32_t R = rle_runs(in, n), t = threadIdx.x;
     const uint32_t* lens = rle_lens(in, sizeof(T));
     const T* values = reinterpret_cast<const T*>(in + 4);
@@ -352,9 +356,11 @@ int launch_rle_encode_t(const T* in, uint32_t n, uint8_t* out, unsigned long lon
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
     const int vec = (reinterpret_cast<uintptr_t>(in) & 15u) == 0;
     rle_count_kernel<T><<<ntiles, 256, 0, s>>>(in, n, vec, tcnt, tfirst);
-    scan_tile_offsets<<<1, 1024, 0, s>>>(tcnt, ntiles, runs_total);
-    rle_emit_kernel<T><<<ntiles, 256, 0, s>>>(in, n, vec, tcnt, tfirst, runs_total, out, out_size);
-    return (int)cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_dependent(scan_tile_offsets, 1, 1024, 0, s, tcnt, ntiles, runs_total);
+    if (e == cudaSuccess)
+        e = launch_dependent(rle_emit_kernel<T>, ntiles, 256, 0, s, in, n, vec, tcnt, tfirst, runs_total, out, out_size);
+    return (int)e;
 }
 
 int launch_rle_encode(const void* in, uint32_t n, int elem, uint8_t* out, unsigned long long* out_size,
@@ -368,12 +374,16 @@ int launch_rle_decode(const uint8_t* in, uint32_t n, int elem, void* out, uint32
                       uint32_t* err, cudaStream_t s) {
     const uint32_t nrt = (n + kRunTile - 1) / kRunTile;  // tiles of runs, at most n runs
     rle_sums_kernel<<<min((nrt + 7) / 8, 1184u), 256, 0, s>>>(in, n, (uint32_t)elem, tsum, nrt);
-    scan_tile_offsets<<<1, 1024, 0, s>>>(tsum, nrt, total);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_dependent(scan_tile_offsets, 1, 1024, 0, s, tsum, nrt, total);
+    if (e != cudaSuccess) return (int)e;
     const uint32_t ntiles = (n + kScanTile - 1) / kScanTile;
-    if (elem == 1) rle_expand_kernel<uint8_t><<<ntiles, 256, 0, s>>>(in, tsum, total, n, (uint8_t*)out, err);
-    else if (elem == 2) rle_expand_kernel<uint16_t><<<ntiles, 256, 0, s>>>(in, tsum, total, n, (uint16_t*)out, err);
-    else rle_expand_kernel<uint32_t><<<ntiles, 256, 0, s>>>(in, tsum, total, n, (uint32_t*)out, err);
-    return (int)cudaGetLastError();
+    auto expand = [&](auto* kernel, auto* o) {
+        return (int)launch_dependent(kernel, ntiles, 256, 0, s, in, tsum, total, n, o, err);
+    };
+    if (elem == 1) return expand(rle_expand_kernel<uint8_t>, (uint8_t*)out);
+    if (elem == 2) return expand(rle_expand_kernel<uint16_t>, (uint16_t*)out);
+    return expand(rle_expand_kernel<uint32_t>, (uint32_t*)out);
 }
 
 // ---------------------------------------------------------------------------

@@ -9,6 +9,7 @@
 #include <cstdint>
 
 #include "../../include/fzb.h"
+#include "fzb_common.cuh"
 
 namespace {
 
@@ -185,6 +186,7 @@ struct ConcatDevParams {
 };
 
 __global__ void concat_dev_kernel(ConcatDevParams p, uint8_t* __restrict__ out) {
+    fzb::follow();
     __shared__ uint64_t s_len[kMaxSeg], s_off[kMaxSeg];
     static_assert(kMaxSeg <= 32, "one warp lays the segments out");
     if (threadIdx.x < 32) {  // lane k: segment k's length, then an exclusive scan of the padded lengths
@@ -261,6 +263,7 @@ struct GatherParams {
 // One warp per item; a lane reads a word, stores it and, for a status word,
 // clears the source.
 __global__ void gather_words_kernel(GatherParams p, uint32_t* dst) {
+    fzb::follow();
     const int lane = threadIdx.x & 31;
     for (int k = threadIdx.x >> 5; k < p.n; k += blockDim.x >> 5) {
         for (uint32_t i = lane; i < p.words[k]; i += 32) {
@@ -307,9 +310,8 @@ extern "C" int fzb_concat_dev(const void* const* d_srcs, const uint64_t* caps, c
     uint64_t blocks = (maxcap / 16 + 255) / 256;
     if (blocks < 1) blocks = 1;
     if (blocks > 8ull * (uint64_t)sms) blocks = 8ull * (uint64_t)sms;
-    concat_dev_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        p, static_cast<uint8_t*>(d_out));
-    return cudaGetLastError() == cudaSuccess ? FZB_OK : FZB_E_CUDA;
+    return fzb::launch_dependent(concat_dev_kernel, (unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream), p,
+                                 static_cast<uint8_t*>(d_out)) == cudaSuccess ? FZB_OK : FZB_E_CUDA;
 }
 
 extern "C" int fzb_gather_words(const void* const* d_srcs, const uint32_t* bytes, const uint8_t* clear, int n,
@@ -329,6 +331,6 @@ extern "C" int fzb_gather_words(const void* const* d_srcs, const uint32_t* bytes
         off += (bytes[i] + 7) & ~7u;
         if (clear[i]) p.clear_mask |= 1u << i;
     }
-    gather_words_kernel<<<1, 256, 0, static_cast<cudaStream_t>(stream)>>>(p, static_cast<uint32_t*>(dst));
-    return cudaGetLastError() == cudaSuccess ? FZB_OK : FZB_E_CUDA;
+    return fzb::launch_dependent(gather_words_kernel, 1, 256, 0, static_cast<cudaStream_t>(stream), p,
+                                 static_cast<uint32_t*>(dst)) == cudaSuccess ? FZB_OK : FZB_E_CUDA;
 }

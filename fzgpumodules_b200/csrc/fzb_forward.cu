@@ -157,6 +157,7 @@ __global__ void __launch_bounds__(256, 8) minmax_kernel(const float* __restrict_
 // Error-bound resolution without a scan (ABS, or a caller-provided base).
 __global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* __restrict__ st, uint32_t* zero,
                                   uint32_t nzero) {
+    follow();
     zero_words(zero, nzero, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     if (blockIdx.x == 0 && threadIdx.x == 0) resolve_eb_store(0.f, 0.f, mode, user_eb, vb_given, false, st);
 }
@@ -531,7 +532,7 @@ __device__ __forceinline__ void assemble_copy_body(const AsmArgs& a, const uint3
 
 // One warp per chunk, grid-stride over the chunks.
 __global__ void __launch_bounds__(256) assemble_copy_kernel(AsmArgs a) {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    follow();
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t nw = gridDim.x * (blockDim.x >> 5);
     for (uint32_t c = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); c < a.n_chunks; c += nw)
@@ -742,6 +743,7 @@ constexpr int chunk_ctas(int ndim) { return ndim == 1 ? 4 : 5; }
 
 template <int NDIM, bool FUSED>
 __global__ void __launch_bounds__(kThreads, chunk_ctas(NDIM)) lq_chunk_kernel(FwdArgs a) {
+    follow();
     extern __shared__ float4 Q[];
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_obase;
@@ -1036,8 +1038,7 @@ template <int NDIM, bool FUSED>
 static int launch_lq_t(const FwdArgs& a, cudaStream_t s) {
     // chunks that only look their outliers up need no shared memory
     const size_t smem = FUSED || NDIM == 1 ? kChunkSmem : 0;
-    lq_chunk_kernel<NDIM, FUSED><<<a.n_chunks, kThreads, smem, s>>>(a);
-    return (int)cudaGetLastError();
+    return (int)launch_dependent(lq_chunk_kernel<NDIM, FUSED>, a.n_chunks, kThreads, smem, s, a);
 }
 
 int launch_lq_chunk(int ndim, bool fused, const FwdArgs& a, cudaStream_t s) {

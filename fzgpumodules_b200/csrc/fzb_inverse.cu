@@ -205,6 +205,7 @@ __global__ void __launch_bounds__(kThreads, 6) rze_decode_kernel(InvArgs a) {
 // waits at its barriers (3600 x 1800: 14.0 us, 15.5 with four).
 __global__ void __launch_bounds__(kThreads, 6) rze_decode_codes_kernel(InvArgs a) {
     __shared__ RzeDecSmem sm;
+    follow();
     if (inv_gated_off(a)) return;
     rze_decode_init(sm);
     if (a.obits)

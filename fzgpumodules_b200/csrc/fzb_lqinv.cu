@@ -316,6 +316,7 @@ __device__ __noinline__ void exact_brick_3d(const InvArgs& a, uint32_t x0, uint3
 // 1-D: one warp a tile, 8 steps of 128 elements.
 template <bool ZZ>
 __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid_constant__ InvArgs a, int mode) {
+    follow();
     if (inv_gated_off(a)) return;
     const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu;
     const float ebx2 = inv_ebx2(a);
@@ -427,6 +428,7 @@ template <bool ZZ, bool AL>
 __global__ void __launch_bounds__(32 * kWarps)
     lq_inverse_2d_kernel(const __grid_constant__ InvArgs a, int mode) {
     __shared__ __align__(16) float strips[kWarps][32 * 36];
+    follow();
     if (inv_gated_off(a)) return;
     const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu, r = lane >> 2, c = lane & 3u;
     float* strip = strips[threadIdx.x >> 5];
@@ -522,6 +524,7 @@ template <bool ZZ, bool AL>
 __global__ void __launch_bounds__(32 * kWarps)
     lq_inverse_3d_kernel(const __grid_constant__ InvArgs a, int mode) {
     __shared__ __align__(16) float bricks[kWarps][8 * 260];
+    follow();
     if (inv_gated_off(a)) return;
     const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu, z = lane >> 2, c = lane & 3u;
     float* brick = bricks[threadIdx.x >> 5];
@@ -630,6 +633,7 @@ __global__ void __launch_bounds__(32 * kWarps)
 // zeroed words: the sum of the magnitudes (infinite for a non-integer) and the
 // rows (1-D: steps of 128) that hold outliers.
 __global__ void mark_outliers_kernel(InvArgs a) {
+    follow();
     if (inv_gated_off(a)) return;
     const uint32_t n = min(*a.out_count, a.cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -677,9 +681,8 @@ int launch_lq_inverse(const InvArgs& a, int ndim, unsigned max_grid, cudaStream_
     if (ndim == 1) {
         const unsigned g = grid(((uint64_t)a.nfield + 1023u) / 1024u, 1);
         const int m1 = (pc & 7u) == 0 ? 0 : (pc & 3u) == 0 ? 1 : 2;
-        if (a.zigzag) lq_inverse_1d_kernel<true><<<g, 32 * kWarps, 0, s>>>(a, m1);
-        else lq_inverse_1d_kernel<false><<<g, 32 * kWarps, 0, s>>>(a, m1);
-        return (int)cudaGetLastError();
+        return (int)launch_dependent(a.zigzag ? lq_inverse_1d_kernel<true> : lq_inverse_1d_kernel<false>, g, 32 * kWarps, 0,
+                                     s, a, m1);
     }
     // the widest loads and stores that the rows' alignment allows
     const int mode = (pc & 15u) == 0 && a.nx % 8u == 0 ? 0 : (pc & 7u) == 0 && a.nx % 4u == 0 ? 1 : (pc & 3u) == 0 ? 2 : 3;
@@ -688,14 +691,13 @@ int launch_lq_inverse(const InvArgs& a, int ndim, unsigned max_grid, cudaStream_
         const unsigned g = grid((uint64_t)((a.nx + 31u) / 32u) * ((a.ny + 31u) / 32u), 1);
         auto k = a.zigzag ? (al ? lq_inverse_2d_kernel<true, true> : lq_inverse_2d_kernel<true, false>)
                           : (al ? lq_inverse_2d_kernel<false, true> : lq_inverse_2d_kernel<false, false>);
-        k<<<g, 32 * kWarps, 0, s>>>(a, mode);
+        return (int)launch_dependent(k, g, 32 * kWarps, 0, s, a, mode);
     } else {
         const unsigned g = grid((uint64_t)((a.nx + 7u) / 8u) * ((a.ny + 7u) / 8u) * ((a.nz + 7u) / 8u), 4);
         auto k = a.zigzag ? (al ? lq_inverse_3d_kernel<true, true> : lq_inverse_3d_kernel<true, false>)
                           : (al ? lq_inverse_3d_kernel<false, true> : lq_inverse_3d_kernel<false, false>);
-        k<<<g, 32 * kWarps, 0, s>>>(a, mode);
+        return (int)launch_dependent(k, g, 32 * kWarps, 0, s, a, mode);
     }
-    return (int)cudaGetLastError();
 }
 
 }  // namespace fzb

@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_last[kThreads / 32];
     __shared__ uint32_t s_obase;
+    follow();
     const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t c = blockIdx.x;
     const uint64_t i0 = (uint64_t)c * kPVals;
@@ -191,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
 }
 
 __global__ void pfpl_cap_count_kernel(uint32_t* count, uint32_t cap) {
+    follow();
     if (*count > cap) *count = cap;
 }
 
@@ -226,6 +228,7 @@ template <bool REL>
 __global__ void __launch_bounds__(kThreads, 6) pfpl_decode_kernel(PDec a) {
     __shared__ RzeDecSmem sm;
     __shared__ uint32_t s_ws[16];
+    follow();
     rze_decode_init(sm);
     const int t = threadIdx.x;
     const uint32_t c = blockIdx.x;
@@ -276,6 +279,7 @@ __global__ void __launch_bounds__(256) pfpl_scatter_kernel(const float* __restri
                                                            const uint32_t* __restrict__ idx,
                                                            const uint32_t* __restrict__ count, uint64_t cap,
                                                            uint64_t n, float* __restrict__ out) {
+    follow();
     const uint64_t m = *count < cap ? *count : cap;
     for (uint64_t k = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; k < m; k += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t j = idx[k];
@@ -406,9 +410,9 @@ int fzb_pfpl_compress_padded(const float* d_in, uint64_t n_in, uint64_t n, float
     a.ostage_cap = (uint32_t)cap;
     {
         TraceScope ts(s, "pfpl_chunk");
-        if (rel) pfpl_chunk_kernel<true><<<a.n_chunks, kThreads, kPSmem, s>>>(a);
-        else pfpl_chunk_kernel<false><<<a.n_chunks, kThreads, kPSmem, s>>>(a);
-        if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
+        if (launch_dependent(rel ? pfpl_chunk_kernel<true> : pfpl_chunk_kernel<false>, a.n_chunks, kThreads, kPSmem, s,
+                             a) != cudaSuccess)
+            return FZB_E_CUDA;
     }
     AsmArgs m{};
     m.slots = w.slots;
@@ -435,11 +439,9 @@ int fzb_pfpl_compress_padded(const float* d_in, uint64_t n_in, uint64_t n, float
     {
         TraceScope ts(s, "assemble_copy");
         unsigned g = a.n_chunks < 4u * (unsigned)device_sms() * 8u ? a.n_chunks : 4u * (unsigned)device_sms() * 8u;
-        assemble_copy_kernel<<<g, 256, 0, s>>>(m);
-        if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
+        if (launch_dependent(assemble_copy_kernel, g, 256, 0, s, m) != cudaSuccess) return FZB_E_CUDA;
     }
-    pfpl_cap_count_kernel<<<1, 1, 0, s>>>(d_count, (uint32_t)cap);
-    return cudaGetLastError() == cudaSuccess ? FZB_OK : FZB_E_CUDA;
+    return launch_dependent(pfpl_cap_count_kernel, 1, 1, 0, s, d_count, (uint32_t)cap) == cudaSuccess ? FZB_OK : FZB_E_CUDA;
 }
 
 size_t fzb_pfpl_decompress_workspace_bytes(uint64_t n) {
@@ -480,15 +482,16 @@ int fzb_pfpl_decompress(const void* d_rze, uint64_t rze_bytes, const float* d_ov
     a.err = err;
     {
         TraceScope ts(s, "pfpl_decode");
-        if (eb_mode == FZB_REL) pfpl_decode_kernel<true><<<nch, kThreads, 0, s>>>(a);
-        else pfpl_decode_kernel<false><<<nch, kThreads, 0, s>>>(a);
-        if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
+        if (launch_dependent(eb_mode == FZB_REL ? pfpl_decode_kernel<true> : pfpl_decode_kernel<false>, nch, kThreads, 0, s,
+                             a) != cudaSuccess)
+            return FZB_E_CUDA;
     }
     if (cap) {
         uint64_t sg = (cap + 255) / 256;
         if (sg > 4096) sg = 4096;
-        pfpl_scatter_kernel<<<(unsigned)sg, 256, 0, s>>>(d_ovals, d_oidx, d_count, cap, n, d_out);
-        if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
+        if (launch_dependent(pfpl_scatter_kernel, (unsigned)sg, 256, 0, s, d_ovals, d_oidx, d_count, cap, n, d_out) !=
+            cudaSuccess)
+            return FZB_E_CUDA;
     }
     return FZB_OK;
 }

@@ -59,6 +59,7 @@ __global__ void __launch_bounds__(kRowThreads, kRowCtasPerSm) lq2d_rows_kernel(F
                                                                              uint32_t units) {
     __shared__ uint32_t s_ws[16];
     __shared__ uint32_t s_obase;
+    follow();
     const uint32_t t = threadIdx.x, lane = t & 31u;
     const float r = __ldcg(a.ebx2_r);
     const float R = a.radius;
@@ -170,9 +171,8 @@ int launch_lq_rows(const FwdArgs& a, unsigned sms, cudaStream_t s) {
     if (rpr >= 32) rpr = (rpr + 31) & ~31u;
     const uint32_t runs = (ny + rpr - 1) / rpr, units = m * runs;
     const unsigned grid = units < want ? units : want;
-    if (a.zigzag) lq2d_rows_kernel<true><<<grid, kRowThreads, 0, s>>>(a, m, rpr, units);
-    else lq2d_rows_kernel<false><<<grid, kRowThreads, 0, s>>>(a, m, rpr, units);
-    return (int)cudaGetLastError();
+    return (int)launch_dependent(a.zigzag ? lq2d_rows_kernel<true> : lq2d_rows_kernel<false>, grid, kRowThreads, 0, s, a,
+                                 m, rpr, units);
 }
 
 }  // namespace fzb

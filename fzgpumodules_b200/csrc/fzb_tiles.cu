@@ -292,6 +292,7 @@ __device__ __forceinline__ void tile_block(const FwdArgs& a, uint32_t block, Til
 }
 
 __global__ void __launch_bounds__(32 * kTileWarps, 8) lq_tiles_kernel(const __grid_constant__ FwdArgs a) {
+    follow();
     __shared__ TileSmem sm[kTileWarps];
     if (a.zigzag) tile_block<true>(a, blockIdx.x, sm[threadIdx.x >> 5]);
     else tile_block<false>(a, blockIdx.x, sm[threadIdx.x >> 5]);
@@ -323,7 +324,7 @@ uint32_t lq_tile_blocks(const FwdArgs& a) {
 }
 
 int launch_lq_tiles(const FwdArgs& a, cudaStream_t s) {
-    lq_tiles_kernel<<<lq_tile_blocks(a), 32 * kTileWarps, 0, s>>>(a);
+    (void)launch_dependent(lq_tiles_kernel, lq_tile_blocks(a), 32 * kTileWarps, 0, s, a);
     return (int)cudaGetLastError();
 }
 
