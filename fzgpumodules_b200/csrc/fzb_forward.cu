@@ -162,80 +162,7 @@ __global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float
     if (blockIdx.x == 0 && threadIdx.x == 0) resolve_eb_store(0.f, 0.f, mode, user_eb, vb_given, false, st);
 }
 
-// ---------------------------------------------------------------------------
-// Lorenzo windows.  Each role (current / up neighbour row, plane z / z-1)
-// stages q = round(x * ebx2_r) for a contiguous index range into shared
-// memory as 16-byte granules; granule r of a window lives at
-// soff + (r ^ ((r >> 3) & 7)) so that the per-thread 32-element reads of a
-// warp hit distinct banks.
-// ---------------------------------------------------------------------------
-
-struct Win {
-    long long gbase;  // first element (multiple of 4, may be negative)
-    int ngran;        // granules
-    int soff;         // granule offset in shared memory (multiple of 8)
-};
-
-__device__ __forceinline__ int swz(int r) { return r ^ ((r >> 3) & 7); }
-
 __device__ __forceinline__ float q_of(float v, float r) { return round_half_away(__fmul_rn(v, r)); }
-
-__device__ __forceinline__ void load_window(float4* Q, const Win& w, const float* __restrict__ in,
-                                            uint32_t nfield, float r, bool vec_ok) {
-    constexpr int kPer = 9;  // granules in flight per thread
-    for (int base = 0; base < w.ngran; base += kPer * kThreads) {
-        float4 buf[kPer];
-#pragma unroll
-        for (int i = 0; i < kPer; i++) {
-            const int gi = base + threadIdx.x + i * kThreads;
-            buf[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (gi < w.ngran) {
-                const long long g = w.gbase + 4LL * gi;
-                if (vec_ok && g >= 0 && g + 4 <= (long long)nfield) {
-                    buf[i] = __ldg(reinterpret_cast<const float4*>(in + g));
-                } else {
-                    float e[4];
-#pragma unroll
-                    for (int k = 0; k < 4; k++)
-                        e[k] = (g + k >= 0 && g + k < (long long)nfield) ? __ldg(in + g + k) : 0.0f;
-                    buf[i] = make_float4(e[0], e[1], e[2], e[3]);
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < kPer; i++) {
-            const int gi = base + threadIdx.x + i * kThreads;
-            if (gi < w.ngran) {
-                const long long g = w.gbase + 4LL * gi;
-                float4 v = buf[i];
-                if (g >= 0 && g + 4 <= (long long)nfield) {
-                    v.x = q_of(v.x, r);
-                    v.y = q_of(v.y, r);
-                    v.z = q_of(v.z, r);
-                    v.w = q_of(v.w, r);
-                } else {  // field edge: positions outside stage as 0 (never read by a valid element)
-                    v.x = (g + 0 >= 0 && g + 0 < (long long)nfield) ? q_of(v.x, r) : 0.0f;
-                    v.y = (g + 1 >= 0 && g + 1 < (long long)nfield) ? q_of(v.y, r) : 0.0f;
-                    v.z = (g + 2 >= 0 && g + 2 < (long long)nfield) ? q_of(v.z, r) : 0.0f;
-                    v.w = (g + 3 >= 0 && g + 3 < (long long)nfield) ? q_of(v.w, r) : 0.0f;
-                }
-                Q[w.soff + swz(gi)] = v;
-            }
-        }
-    }
-}
-
-__device__ __forceinline__ Win make_win(long long start, long long end) {
-    const long long gb = start >= 0 ? (start & ~3LL) : -(((-start) + 3) & ~3LL);
-    return Win{gb, (int)((end - gb + 3) >> 2), 0};
-}
-
-// Single-element q read of element k from window w.
-__device__ __forceinline__ float qread(const float4* Q, const Win& w, long long k) {
-    const int m = (int)(k - w.gbase);
-    const float* Qf = reinterpret_cast<const float*>(Q);
-    return Qf[4 * (w.soff + swz(m >> 2)) + (m & 3)];
-}
 
 // Lorenzo delta of element k from the input, in the reference's operation
 // order (3-D: z, x, y -- lorenzo_quant_nd.cu:234-246; 2-D: y, x -- :72-77;
@@ -557,52 +484,66 @@ __device__ __forceinline__ uint32_t code_of(float c) {
 // width 2, ballot layout) and RZE-encodes the block into the slot.
 // ---------------------------------------------------------------------------
 
-// Register front end for full chunks of 1-D fields (16-byte aligned input):
-// thread t's 32 elements k0 .. k0 + 31 come straight from HBM into registers,
-// are quantized with the packed round (trunc(y + copysign(0.49999997, y))) and
-// differenced there; a 1024-element block starts at every lane 0, and element
-// k0 - 1 is lane t - 1's last.  Other chunks are staged as a window in shared
-// memory.  Codes come from the magic-number add; per 4-element granule a
-// NaN-propagating max flags outliers, confirmed element by element.  `valid`:
-// elements of this thread inside the field.
+// Codes of a chunk of a 1-D field: warp w takes its 1024 elements, which are one
+// prediction tile, as 16-byte granules l, l + 32, ... of lane l, all eight loads
+// ahead of their use; quantizes them with the packed round (trunc(y +
+// copysign(0.49999997, y))) and differences them, a granule's predecessor coming
+// from the lane before; the codes change places through shared memory, so that
+// thread t ends with those of elements 32t .. 32t + 31 in x and their outliers in
+// om.  base: the encoder's shared memory (free before and after).  `fend`: end of
+// the field inside the chunk; `valid`: elements of this thread before it.
+//
+// Bound by HBM and the chunk coder behind it.  With each thread loading its own 128
+// bytes (every load of a warp on 32 lines) and four CTAs an SM 20 million elements
+// took 37.6 us instead of 33.2, the 1-D fields of a batch of 0.96 GB 194 instead of
+// 158.
 template <bool ZZ>
-__device__ __forceinline__ void chunk1d_codes(const FwdArgs& a, uint32_t k0, float r, bool reg, int valid, float4* Q,
-                                              const Win& w, uint32_t (&x)[16], uint32_t& om) {
+__device__ __forceinline__ void chunk1d_codes(const FwdArgs& a, uint32_t i0, uint32_t fend, float r, int valid,
+                                              void* base, uint32_t (&x)[16], uint32_t& om) {
     const float R = a.radius;
-    Q4 q[8];
-    float left;  // the x predecessor of element 0
-    if (reg) {
-        const float4* src = reinterpret_cast<const float4*>(a.in + k0);
+    const uint32_t t = threadIdx.x, lane = t & 31u, warp = t >> 5, full = 0xffffffffu;
+    uint32_t* S = static_cast<uint32_t*>(base);                 // 16-byte granules at rze_granule
+    uint32_t* s_om = S + kChunkBytes / 4;                       // a word a thread
+    const uint32_t e0 = i0 + 1024u * warp + 4u * lane;
+    const bool al = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
+    float4 v[8];
 #pragma unroll
-        for (int g = 0; g < 8; g++) q[g] = quant4(__ldg(src + g), r);
-        const float pl = __shfl_up_sync(0xffffffffu, q[7].b.y, 1);
-        left = (threadIdx.x & 31u) ? pl : 0.0f;
-    } else {
-        const int g0 = (int)(((long long)k0 - w.gbase) >> 2);  // k0 is a multiple of 32
-#pragma unroll
-        for (int g = 0; g < 8; g++) {
-            const float4 v = 4 * g < valid ? Q[w.soff + swz(g0 + g)] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            q[g] = {f2(v.x, v.y), f2(v.z, v.w)};
+    for (int i = 0; i < 8; i++) {
+        const uint32_t e = e0 + 128u * i;
+        if (al && e + 4u <= fend) {
+            v[i] = __ldg(reinterpret_cast<const float4*>(a.in + e));
+        } else {
+            v[i].x = e < fend ? __ldg(a.in + e) : 0.0f;
+            v[i].y = e + 1u < fend ? __ldg(a.in + e + 1) : 0.0f;
+            v[i].z = e + 2u < fend ? __ldg(a.in + e + 2) : 0.0f;
+            v[i].w = e + 3u < fend ? __ldg(a.in + e + 3) : 0.0f;
         }
-        left = (valid > 0 && (k0 & 1023u)) ? qread(Q, w, (long long)k0 - 1) : 0.0f;
     }
-    uint32_t rw[16];
-    om = 0;
+    s_om[t] = 0u;
+    __syncwarp();
+    float before = 0.0f;  // lane 0: the last value of the granules before; 0 at the tile's start
 #pragma unroll
-    for (int g = 0; g < 8; g++) {
-        const Q4 c = {sub2(q[g].a, f2(left, q[g].a.x)), sub2(q[g].b, f2(q[g].a.y, q[g].b.x))};
-        left = q[g].b.y;
-        const float mx = max_nan(max_nan(fabsf(c.a.x), fabsf(c.a.y)), max_nan(fabsf(c.b.x), fabsf(c.b.y)));
-        uint32_t p0 = code_pair<ZZ>(c.a), p1 = code_pair<ZZ>(c.b);
-        if (!(mx < R)) {  // outliers: their codes are 0
-            const uint32_t b = (fabsf(c.a.x) < R ? 0u : 1u) | (fabsf(c.a.y) < R ? 0u : 2u) |
-                               (fabsf(c.b.x) < R ? 0u : 4u) | (fabsf(c.b.y) < R ? 0u : 8u);
-            om |= b << (4 * g);
-            p0 &= ((b & 1u) ? 0xffff0000u : 0xffffffffu) & ((b & 2u) ? 0x0000ffffu : 0xffffffffu);
-            p1 &= ((b & 4u) ? 0xffff0000u : 0xffffffffu) & ((b & 8u) ? 0x0000ffffu : 0xffffffffu);
-        }
-        rw[2 * g] = p0;
-        rw[2 * g + 1] = p1;
+    for (int i = 0; i < 8; i++) {
+        const Q4 q = quant4(v[i], r);
+        const float n = __shfl_sync(full, q.b.y, (lane + 31u) & 31u);
+        const float left = lane ? n : before;
+        before = n;
+        uint32_t m;
+        const uint2 p = codes4<ZZ>({sub2(q.a, f2(left, q.a.x)), sub2(q.b, f2(q.a.y, q.b.x))}, R, m);
+        const uint32_t g = 256u * warp + lane + 32u * i;  // 8-byte granule of codes
+        *reinterpret_cast<uint2*>(S + 4u * rze_granule(g >> 1) + 2u * (g & 1u)) = p;
+        if (m) atomicOr(s_om + (g >> 3), m << (4u * (g & 7u)));
+    }
+    __syncwarp();
+    om = s_om[t];
+    uint32_t rw[16];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        const uint4 q = reinterpret_cast<const uint4*>(S)[rze_granule(4u * t + i)];
+        rw[4 * i] = q.x;
+        rw[4 * i + 1] = q.y;
+        rw[4 * i + 2] = q.z;
+        rw[4 * i + 3] = q.w;
     }
     if (valid < 32) {
         om &= valid > 0 ? (1u << valid) - 1u : 0u;
@@ -645,10 +586,10 @@ __device__ __forceinline__ void stage_outliers(const FwdArgs& a, uint32_t c, uin
     }
 }
 
-// Shared memory of a chunk: the RZE working set; 1-D chunks off the register
-// front end first stage their window there.
+// Shared memory of a chunk: the RZE working set; the codes of a 1-D chunk change
+// places there first.
 constexpr size_t kChunkSmem = kRzeEncSmem;
-static_assert(kChunkSmem >= 16 * (kChunkCodes / 4 + 8), "the 1-D window fits");
+static_assert(kChunkSmem >= kChunkBytes + 4 * kThreads, "the codes and the outlier words fit");
 
 // Bitshuffle of the chunk's packed codes (cnt of them), RZE, slot.
 __device__ __forceinline__ void encode_slot(const FwdArgs& a, uint32_t c, uint32_t cnt, uint32_t (&x)[16],
@@ -681,16 +622,8 @@ __device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c
     const float r = *a.ebx2_r;
     uint32_t x[16], om = 0;
     if (NDIM == 1) {
-        const bool al = (reinterpret_cast<uintptr_t>(a.in) & 15) == 0;
-        const bool reg = al && i0 + (uint32_t)kChunkCodes <= fend;  // the same for every thread
-        Win w{0, 0, 0};
-        if (!reg) {
-            w = make_win((long long)i0 - 1, (long long)i0 + cnt);
-            load_window(Q, w, a.in, a.nfield, r, al);
-            __syncthreads();
-        }
-        if (a.zigzag) chunk1d_codes<true>(a, k0, r, reg, valid, Q, w, x, om);
-        else chunk1d_codes<false>(a, k0, r, reg, valid, Q, w, x, om);
+        if (a.zigzag) chunk1d_codes<true>(a, i0, fend, r, valid, Q, x, om);
+        else chunk1d_codes<false>(a, i0, fend, r, valid, Q, x, om);
     } else {
         if (valid > 0) om = __ldg(a.obits + (k0 >> 5));
         if (FUSED) {
@@ -715,8 +648,7 @@ __device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c
         }
     }
     stage_outliers<NDIM>(a, c, k0, r, om, s_ws, s_obase);
-    if (FUSED) {
-        __syncthreads();  // the window is dead past this point
+    if (FUSED) {  // the barrier of stage_outliers: the codes are out of shared memory
         encode_slot(a, c, cnt, x, reinterpret_cast<uint8_t*>(Q), s_ws);
         return;
     }
@@ -735,14 +667,12 @@ __device__ __forceinline__ void lq_chunk_body(const FwdArgs& a, const uint32_t c
     }
 }
 
-// CTAs an SM: the chunk coder waits at its barriers, so five resident chunks of the
-// codes the tile kernel left beat four (500 x 500 x 100: 54.2 us against 56.3; 65.8
-// with six, which spill), and the 1-D front end, with eight granules in flight,
-// needs the registers of four.
-constexpr int chunk_ctas(int ndim) { return ndim == 1 ? 4 : 5; }
+// The chunk coder waits at its barriers, so five resident chunks beat four (500 x
+// 500 x 100: 54.2 us against 56.3; 65.8 with six, which spill).
+constexpr int kChunkCtas = 5;
 
 template <int NDIM, bool FUSED>
-__global__ void __launch_bounds__(kThreads, chunk_ctas(NDIM)) lq_chunk_kernel(FwdArgs a) {
+__global__ void __launch_bounds__(kThreads, kChunkCtas) lq_chunk_kernel(FwdArgs a) {
     follow();
     extern __shared__ float4 Q[];
     __shared__ uint32_t s_ws[16];
@@ -761,8 +691,7 @@ __global__ void __launch_bounds__(kThreads, chunk_ctas(NDIM)) lq_chunk_kernel(Fw
 // ONE_D: the units of the 1-D fields, the first b.one_units; else the 2-D and 3-D
 // fields' units after them.  One kernel for all of them was as large as its three
 // bodies and took 519 us for twenty fields of 0.96 GB with two CTAs an SM; these
-// take 194 + 150 with the four an SM that their registers leave room for (154
-// for the second with five).
+// take 158 + 147 with four an SM (159 + 150 with five, which spill).
 template <bool ONE_D>
 __global__ void __launch_bounds__(kThreads, 4) lq_batch_kernel(BatchArgs b) {
     extern __shared__ float4 Q[];

@@ -128,6 +128,26 @@ __device__ __forceinline__ uint32_t code_pair(float2 c) {
     return p;
 }
 
+// Bits of the four deltas that are not quantizable.
+__device__ __forceinline__ uint32_t outliers4(Q4 c, float R) {
+    return (fabsf(c.a.x) < R ? 0u : 1u) | (fabsf(c.a.y) < R ? 0u : 2u) | (fabsf(c.b.x) < R ? 0u : 4u) |
+           (fabsf(c.b.y) < R ? 0u : 8u);
+}
+
+// Codes of four deltas (0 for outliers, whose bits go to m).
+template <bool ZZ>
+__device__ __forceinline__ uint2 codes4(Q4 c, float R, uint32_t& m) {
+    uint2 p = make_uint2(code_pair<ZZ>(c.a), code_pair<ZZ>(c.b));
+    const float mx = max_nan(max_nan(fabsf(c.a.x), fabsf(c.a.y)), max_nan(fabsf(c.b.x), fabsf(c.b.y)));
+    m = 0;
+    if (!(mx < R)) {
+        m = outliers4(c, R);
+        p.x &= ((m & 1u) ? 0xffff0000u : 0xffffffffu) & ((m & 2u) ? 0x0000ffffu : 0xffffffffu);
+        p.y &= ((m & 4u) ? 0xffff0000u : 0xffffffffu) & ((m & 8u) ? 0x0000ffffu : 0xffffffffu);
+    }
+    return p;
+}
+
 // Byte offset in a 128-byte-swizzled buffer of 16-byte granule g of row `row`
 // (the TMA SWIZZLE_128B layout: granule index XOR row % 8).  Thread t of a
 // slab kernel owns row t (32 floats).

@@ -28,26 +28,6 @@ namespace {
 
 constexpr int kTileWarps = 4;  // warps a CTA
 
-// Bits of the four deltas that are not quantizable.
-__device__ __forceinline__ uint32_t outliers4(Q4 c, float R) {
-    return (fabsf(c.a.x) < R ? 0u : 1u) | (fabsf(c.a.y) < R ? 0u : 2u) | (fabsf(c.b.x) < R ? 0u : 4u) |
-           (fabsf(c.b.y) < R ? 0u : 8u);
-}
-
-// Codes of four deltas (0 for outliers, whose bits go to m).
-template <bool ZZ>
-__device__ __forceinline__ uint2 codes4(Q4 c, float R, uint32_t& m) {
-    uint2 p = make_uint2(code_pair<ZZ>(c.a), code_pair<ZZ>(c.b));
-    const float mx = max_nan(max_nan(fabsf(c.a.x), fabsf(c.a.y)), max_nan(fabsf(c.b.x), fabsf(c.b.y)));
-    m = 0;
-    if (!(mx < R)) {
-        m = outliers4(c, R);
-        p.x &= ((m & 1u) ? 0xffff0000u : 0xffffffffu) & ((m & 2u) ? 0x0000ffffu : 0xffffffffu);
-        p.y &= ((m & 4u) ? 0xffff0000u : 0xffffffffu) & ((m & 8u) ? 0x0000ffffu : 0xffffffffu);
-    }
-    return p;
-}
-
 // Marks the outliers m (bit i: element g + i) of a field's bitmap.
 __device__ __forceinline__ void mark_bits(uint32_t* bits, uint32_t g, uint32_t m) {
     const uint32_t s = g & 31u;

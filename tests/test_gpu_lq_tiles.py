@@ -1,4 +1,4 @@
-"""Codes by tiles (2-D, 3-D fields of any extents) against the oracle: extents
+"""Codes by tiles (fields of any rank and extents) against the oracle: extents
 around the tile, load and chunk sizes, input at 16- and 4-byte alignment, few
 and many outliers, NaN and infinities; the codes call and the fused chain, and
 an input counted as padded without a padded copy."""
@@ -13,6 +13,7 @@ from oracle import oracle as O
 pytestmark = pytest.mark.gpu
 
 DIMS = [(31, 33, 1), (32, 64, 1), (36, 5, 1), (333, 130, 1), (8, 2000, 1), (9000, 3, 1),
+        (3, 1, 1), (1023, 1, 1), (8192, 1, 1), (8193, 1, 1), (40961, 1, 1),
         (7, 9, 3), (8, 8, 8), (33, 17, 9), (64, 10, 21), (130, 5, 40), (100, 100, 9), (1, 5, 300)]
 
 
