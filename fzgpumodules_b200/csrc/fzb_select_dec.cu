@@ -205,7 +205,7 @@ int launch_sel_decode(const SelDec& a, cudaStream_t s) {
     sel_decode_kernel<<<4 * a.nch, kThreads, 0, s>>>(a);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return (int)e;
-    return launch_sel_hf_decode(a, device_sms(), s);
+    return launch_sel_hf_decode(a, s);
 }
 
 }  // namespace fzb
