@@ -495,8 +495,9 @@ __global__ void __launch_bounds__(256) sel_hf_hist_kernel(SelArgs s) {
 // nodes, and one pass from the root down turns the parents into depths (the
 // code lengths of the reference's tree walk).  The merges are a serial chain, so
 // its length is the time: five levels of a sift are decided at once, a lane a
-// node (300 books of up to 1024 symbols: 700 us with one lane sifting level by
-// level, 455 so).  The leaf gather and the
+// node, and the place reached is the largest index on the path (300 books of up to
+// 1024 symbols: 700 us with one lane sifting level by level, 455 with the place from
+// votes and leading-bit counts, 425 so).  The leaf gather and the
 // canonical codebook are warp-parallel.  Dynamic shared memory (8 KB, so
 // about 25 chunks run per SM): the heap (later the per-symbol lengths), then
 // the parent/depth array.
@@ -548,12 +549,15 @@ __global__ void __launch_bounds__(32) sel_hf_book_kernel(SelArgs s) {
     // stops at a parent whose frequency is <= the new node's; removal sinks
     // the moved node, taking the right child only when strictly smaller and
     // swapping only when strictly larger.
+    // k < (m & ~0x7ff) compares the frequencies of two keys alone.
+    constexpr uint32_t kFreq = ~0x7ffu;
     int hs = 0;
+    if (lane == 0) hk[0] = 0u;  // above the root: never sinks
+    __syncwarp();
     auto push = [&](uint32_t key) {
         const int i = ++hs;
-        const int up = i >> (lane < 30u ? lane + 1 : 30u);  // lane j: ancestor j + 1
-        const uint32_t kp = up ? hk[up] : 0u;
-        const uint32_t above = __ballot_sync(full, up != 0 && (kp >> 11) > (key >> 11));
+        const uint32_t kp = hk[i >> (lane < 30u ? lane + 1 : 30u)];  // lane j: ancestor j + 1
+        const uint32_t above = __ballot_sync(full, key < (kp & kFreq));
         const uint32_t cnt = (uint32_t)__ffs(~above) - 1;  // ancestors that move down one level
         if (lane < cnt) hk[i >> lane] = kp;
         if (lane == 0) hk[i >> cnt] = key;
@@ -569,30 +573,35 @@ __global__ void __launch_bounds__(32) sel_hf_book_kernel(SelArgs s) {
         aexp |= (l & 1u) << (l >> 1);
     }
     auto pop = [&]() -> uint32_t {
-        const uint32_t top = hk[1], moved = hk[hs], mf = moved >> 11;
+        const uint32_t top = hk[1], moved = hk[hs], mf = moved & kFreq;
         hs--;
-        int i = 1;
+        uint32_t i = 1;
         while (true) {
-            const int P = (i << dl) + (int)(lane - (1u << dl));
-            const bool in = lane != 0 && 2 * P <= hs;
-            const uint2 kk = in ? *reinterpret_cast<const uint2*>(hk + 2 * P) : make_uint2(0u, 0u);
-            const bool right = in && 2 * P + 1 <= hs && (kk.y >> 11) < (kk.x >> 11);
-            const uint32_t kc = right ? kk.y : kk.x;
-            const bool sink = in && mf > (kc >> 11);
+            const uint32_t P = (i << dl) + (lane - (1u << dl));
+            const uint2 kk = lane != 0 && 2 * P <= (uint32_t)hs ? *reinterpret_cast<const uint2*>(hk + 2 * P)
+                                                                 : make_uint2(~0u, ~0u);
+            const uint32_t ky = 2 * P + 1 <= (uint32_t)hs ? kk.y : ~0u;
+            const bool right = ky < (kk.x & kFreq);
+            const bool sink = min(kk.x, ky) < mf;  // the chosen child has the smaller frequency
             const uint32_t choice = __ballot_sync(full, right), sinks = __ballot_sync(full, sink);
             const bool move = sink && (choice & amask) == aexp && (sinks & amask) == amask;
-            const uint32_t moves = __ballot_sync(full, move);  // the path's lanes, the last the deepest
-            if (move) hk[P] = kc;
-            if (!moves) break;
-            const uint32_t D = 31u - __clz(moves), dd = 31u - __clz(D);
-            i = 2 * ((i << dd) + (int)(D - (1u << dd))) + (int)((choice >> D) & 1u);
-            if (dd < 4u) break;
+            if (move) hk[P] = right ? ky : kk.x;
+            // the deepest place on the path has the largest index
+            const uint32_t to = __reduce_max_sync(full, move ? 2 * P + (right ? 1u : 0u) : 0u);
+            if (to == 0) break;
+            const bool on = to >= i << 5;  // five levels down: the path may go on
+            i = to;
+            if (!on) break;
         }
         if (lane == 0) hk[i] = moved;
         __syncwarp();
         return top;
     };
-    for (int i = 0; i < leaves; i++) push(((uint32_t)par[i] << 11) | (uint32_t)i);
+    for (uint32_t i = 0, f = leaves ? par[0] : 0u; i < (uint32_t)leaves; i++) {
+        const uint32_t key = (f << 11) | i;
+        f = par[i + 1];  // (leaves <= kSelBk, half of par)
+        push(key);
+    }
     int nn = leaves;
     while (hs > 1) {  // the first popped node becomes the right child
         const uint32_t kr = pop();
