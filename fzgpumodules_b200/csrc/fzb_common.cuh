@@ -17,10 +17,10 @@ namespace fzb {
 // griddepcontrol.wait before reading its results, see follow()); a plain launch
 // when the attribute is refused.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_dependent(void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+inline cudaError_t launch_dependent(void (*kernel)(KArgs...), dim3 grid, unsigned block, size_t smem,
                                     cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;

@@ -868,6 +868,7 @@ __global__ void __launch_bounds__(kHfDecThreads, 2)
 // 2048 chunks: 78 us; 131 with two CTAs an SM taking every 296th chunk, some of
 // which met four).
 __global__ void __launch_bounds__(kHfDecThreads, 2) sel_hf_decode_kernel(SelDec a) {
+    follow();
     if (*a.state == 0u) return;
     const uint32_t c = blockIdx.x;
     if (sel_tag(a, c) != 3u) return;
@@ -938,12 +939,10 @@ int launch_hf_encode(const uint16_t* in, uint64_t n, const uint32_t* bk4, uint32
                                  ctrl, reinterpret_cast<uint32_t*>(out + 24));
 }
 
-int launch_sel_hf_decode(const SelDec& a, cudaStream_t s) {
+cudaError_t launch_sel_hf_decode(const SelDec& a, cudaStream_t s) {
     static SmemAttr attr;
     const cudaError_t e = ensure_dyn_smem(attr, (const void*)sel_hf_decode_kernel, (int)kHfDecSmem);
-    if (e != cudaSuccess) return (int)e;
-    sel_hf_decode_kernel<<<a.nch, kHfDecThreads, kHfDecSmem, s>>>(a);
-    return (int)cudaGetLastError();
+    return e == cudaSuccess ? launch_dependent(sel_hf_decode_kernel, a.nch, kHfDecThreads, kHfDecSmem, s, a) : e;
 }
 
 int launch_hf_decode(const uint8_t* blob, uint64_t blob_bytes, uint64_t n, uint32_t bklen,

@@ -372,7 +372,7 @@ __device__ __forceinline__ void sel_fail(const SelDec& a, uint32_t c, uint32_t c
     atomicMax(a.fault, ~(4u * c + cause));
 }
 int launch_sel_decode(const SelDec& a, cudaStream_t s);
-int launch_sel_hf_decode(const SelDec& a, cudaStream_t s);
+cudaError_t launch_sel_hf_decode(const SelDec& a, cudaStream_t s);
 
 int launch_sel_features(const uint16_t* codes, uint64_t n, float* feats, cudaStream_t s);
 int launch_sel_coders(const SelArgs& a, uint32_t nchunks, unsigned coder_mask, cudaStream_t s);

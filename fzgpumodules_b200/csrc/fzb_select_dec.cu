@@ -178,10 +178,14 @@ __device__ __forceinline__ void decode_bitpack(const SelDec& a, uint32_t c, uint
 }
 
 // Four CTAs a chunk: everything but the Huffman chunks.  Six CTAs an SM (134 MB of
-// codes: 100 us, 106 with four).
+// codes: 100 us, 106 with four).  Launched as a dependent of the Huffman decoder,
+// beside whose last CTAs it runs: the offsets that both read were complete when the
+// first of them began.  Only the last block awaits that kernel, so that what follows
+// comes after both.
 __global__ void __launch_bounds__(kThreads, 6) sel_decode_kernel(SelDec a) {
     __shared__ RzeDecSmem sm;
     __shared__ uint32_t s_ws[16];
+    if (blockIdx.x == gridDim.x - 1) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (*a.state == 0u) return;
     const uint32_t c = blockIdx.x >> 2, tag = sel_tag(a, c), sz = sel_size(a, c);
     const uint64_t off = 4ull * a.offs[c];
@@ -202,10 +206,10 @@ __global__ void __launch_bounds__(kThreads, 6) sel_decode_kernel(SelDec a) {
 
 int launch_sel_decode(const SelDec& a, cudaStream_t s) {
     sel_offsets_kernel<<<1, 1024, 0, s>>>(a);
-    sel_decode_kernel<<<4 * a.nch, kThreads, 0, s>>>(a);
-    const cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return (int)e;
-    return launch_sel_hf_decode(a, s);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_sel_hf_decode(a, s);
+    if (e == cudaSuccess) e = launch_dependent(sel_decode_kernel, 4 * a.nch, kThreads, 0, s, a);
+    return (int)e;
 }
 
 }  // namespace fzb
