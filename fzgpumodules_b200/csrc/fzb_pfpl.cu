@@ -148,16 +148,16 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
 
     // outliers: block scan, one staging allocation per chunk
     const uint32_t nout = __popc(om);
-    uint32_t ototal;
-    const uint32_t ooff = block_excl_scan(nout, s_ws, &ototal);
-    if (t == 0) {
-        const uint32_t b = ototal ? atomicAdd(a.ostage_ctr, ototal) : 0u;
-        a.obase[c] = b;
-        a.ocnt[c] = ototal;
-        s_obase = b;
-    }
-    __syncthreads();
-    if (nout) {
+    if (__syncthreads_or(nout != 0)) {
+        uint32_t ototal;
+        const uint32_t ooff = block_excl_scan(nout, s_ws, &ototal);
+        if (t == 0) {
+            const uint32_t b = atomicAdd(a.ostage_ctr, ototal);
+            a.obase[c] = b;
+            a.ocnt[c] = ototal;
+            s_obase = b;
+        }
+        __syncthreads();
         uint32_t pos = s_obase + ooff;
 #pragma unroll
         for (int e = 0; e < 16; e++) {
@@ -169,6 +169,9 @@ __global__ void __launch_bounds__(kThreads, 5) pfpl_chunk_kernel(PArgs a) {
                 pos++;
             }
         }
+    } else if (t == 0) {
+        a.obase[c] = 0u;
+        a.ocnt[c] = 0u;
     }
 
     // Bitshuffle (ew 2) of the chunk's 8192 half-words, then RZE
