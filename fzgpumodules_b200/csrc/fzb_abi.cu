@@ -16,7 +16,7 @@ using namespace fzb;
 namespace {
 
 constexpr int kVersion = 100;
-constexpr size_t kCtrlBytes = 256;   // err, ticket, scalars
+constexpr size_t kCtrlBytes = 4 * kCtrlWords;  // err, ticket, scalars
 constexpr int kMaxParts = 1024;      // min/max partials
 
 struct Work {
@@ -112,8 +112,8 @@ int geometry(uint64_t n_total, const uint32_t dims[3], Geometry* g) {
     return FZB_OK;
 }
 
-// Resolves abs_eb / ebx2_r on the device into eb_state (no host sync)
-// and clears the outlier bitmap (when the field has one).
+// Clears the control words, resolves abs_eb / ebx2_r on the device into eb_state (no
+// host sync) and clears the outlier bitmap (when the field has one).
 // n_in of the n_total values are at d_in, the rest are zeros.
 int resolve_eb(const float* d_in, uint64_t n_in, uint64_t n_total, float eb, int mode, float value_base,
                const Work& w, float* d_eb_state, uint32_t* obits, uint32_t obits_words, cudaStream_t s) {
@@ -125,13 +125,14 @@ int resolve_eb(const float* d_in, uint64_t n_in, uint64_t n_total, float eb, int
         int parts = (int)(want < (uint64_t)(7 * sms) ? want : (uint64_t)(7 * sms));
         if (parts < 1) parts = 1;
         if (parts > kMaxParts) parts = kMaxParts;
+        CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));  // the scan's ticket among them
         TraceScope ts(s, "minmax_resolve_eb");
         minmax_kernel<<<parts, 256, 0, s>>>(d_in, n_in, w.pmin, w.pmax, w.mm_done, mode, eb,
                                             d_eb_state, obits, obits_words, n_in < n_total);
     } else {
         TraceScope ts(s, "resolve_eb");
         const uint32_t blocks = 1 + std::min(obits_words / 4096u, 592u);
-        resolve_eb_kernel<<<blocks, 256, 0, s>>>(mode, eb, value_base, d_eb_state, obits, obits_words);
+        resolve_eb_kernel<<<blocks, 256, 0, s>>>(mode, eb, value_base, d_eb_state, w.err, obits, obits_words);
     }
     CK(cudaGetLastError());
     return FZB_OK;
@@ -206,7 +207,6 @@ int forward_common(bool fused, const float* d_in, uint64_t n_in, uint64_t n_tota
     if (!d_work || work_bytes < w.need) return FZB_E_WORKSPACE;
     cudaStream_t s = S(stream);
     const uint64_t nch = chunks_of(n_total);
-    CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));
     FwdArgs a = fwd_args(g, w, d_in, n_total, d_eb_state, radius, zigzag, d_codes, cap);
     const uint32_t nx = g.nx;
     const bool slab = fused && g.ndim == 3 && nx >= 32 && nx <= 1024 && (nx & (nx - 1)) == 0 &&
@@ -506,7 +506,6 @@ int fzb_rze_decode(const void* d_in, uint64_t in_bytes, uint64_t orig_bytes, voi
     Work w = carve(d_work, n_equiv, 0);
     if (!d_work || work_bytes < w.need) return FZB_E_WORKSPACE;
     cudaStream_t s = S(stream);
-    CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));
     if (launch_rze_prepass(static_cast<const uint8_t*>(d_in), in_bytes, (uint32_t)nch, (uint32_t)orig_bytes,
                            w.in_off, w.err, s) != 0)
         return FZB_E_CUDA;
@@ -539,7 +538,6 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
     Work w = carve(d_work, n_total, 0);
     if (!d_work || work_bytes < w.need) return FZB_E_WORKSPACE;
     cudaStream_t s = S(stream);
-    CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));
     {
         TraceScope ts(s, "rze_prepass");
         if (launch_rze_prepass(static_cast<const uint8_t*>(d_rze), rze_bytes, (uint32_t)nch,

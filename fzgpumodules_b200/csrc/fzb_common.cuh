@@ -49,6 +49,7 @@ __device__ __forceinline__ void follow() {
 }
 
 constexpr int kThreads = 256;            // threads per chunk CTA
+constexpr uint32_t kCtrlWords = 64;      // control words at the head of a workspace, zero when a call begins
 constexpr int kChunkBytes = 16384;       // Bitshuffle block == RZE chunk
 constexpr int kChunkCodes = kChunkBytes / 2;  // u16 codes per chunk
 constexpr int kRzeAvail = kChunkBytes - 2;    // rze_stage.cu:369

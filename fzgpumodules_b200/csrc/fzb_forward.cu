@@ -154,10 +154,12 @@ __global__ void __launch_bounds__(256, 8) minmax_kernel(const float* __restrict_
     zero_words(zero, nzero, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
 }
 
-// Error-bound resolution without a scan (ABS, or a caller-provided base).
-__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* __restrict__ st, uint32_t* zero,
-                                  uint32_t nzero) {
+// Error-bound resolution without a scan (ABS, or a caller-provided base); the call's
+// first kernel, so it also clears the control words (null: the caller has).
+__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* __restrict__ st, uint32_t* ctrl,
+                                  uint32_t* zero, uint32_t nzero) {
     follow();
+    if (blockIdx.x == 0 && ctrl) zero_words(ctrl, kCtrlWords, threadIdx.x, blockDim.x);
     zero_words(zero, nzero, blockIdx.x * blockDim.x + threadIdx.x, gridDim.x * blockDim.x);
     if (blockIdx.x == 0 && threadIdx.x == 0) resolve_eb_store(0.f, 0.f, mode, user_eb, vb_given, false, st);
 }

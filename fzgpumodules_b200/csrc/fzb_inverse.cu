@@ -94,6 +94,10 @@ __global__ void __launch_bounds__(1024) rze_prepass_tiles_kernel(const uint8_t* 
                                                                  unsigned long long* __restrict__ in_off,
                                                                  uint32_t* err) {
     __shared__ uint32_t ws[66];
+    if (gridDim.x == 1) {  // the launcher left the control words to the only CTA
+        if (threadIdx.x < kCtrlWords) err[threadIdx.x] = 0u;
+        __syncthreads();
+    }
     const uint32_t* h = reinterpret_cast<const uint32_t*>(rze);
     const uint32_t n = n_expect, t = threadIdx.x, base = blockIdx.x * 1024u;
     const bool last = base + 1024u >= n;
@@ -122,16 +126,22 @@ __global__ void __launch_bounds__(1024) rze_prepass_tiles_kernel(const uint8_t* 
     asm volatile("griddepcontrol.launch_dependents;");  // outlier_ranges_kernel may start
 }
 
+// Clears the kCtrlWords control words at err and lays the chunks out.
 int launch_rze_prepass(const uint8_t* rze, uint64_t rze_bytes, uint32_t n_expect, uint32_t orig_expect,
                        unsigned long long* in_off, uint32_t* err, cudaStream_t s) {
     if (n_expect <= kTiledScanMax && !(flags_env() & 16)) {
-        rze_prepass_tiles_kernel<<<(n_expect + 1023u) / 1024u + (n_expect == 0), 1024, 0, s>>>(
-            rze, rze_bytes, n_expect, orig_expect, in_off, err);
+        const uint32_t grid = (n_expect + 1023u) / 1024u + (n_expect == 0);
+        if (grid > 1) {  // one CTA clears them itself
+            const cudaError_t e = cudaMemsetAsync(err, 0, 4 * kCtrlWords, s);
+            if (e != cudaSuccess) return (int)e;
+        }
+        rze_prepass_tiles_kernel<<<grid, 1024, 0, s>>>(rze, rze_bytes, n_expect, orig_expect, in_off, err);
         return (int)cudaGetLastError();
     }
     const int smem = (int)((kAsmTile + kAsmTile / 32) * sizeof(uint32_t));
     static SmemAttr attr;
-    const cudaError_t e = ensure_dyn_smem(attr, (const void*)rze_prepass_kernel, smem);
+    cudaError_t e = ensure_dyn_smem(attr, (const void*)rze_prepass_kernel, smem);
+    if (e == cudaSuccess) e = cudaMemsetAsync(err, 0, 4 * kCtrlWords, s);
     if (e != cudaSuccess) return (int)e;
     rze_prepass_kernel<<<1, 1024, smem, s>>>(rze, rze_bytes, n_expect, orig_expect, in_off, err);
     return (int)cudaGetLastError();
@@ -154,13 +164,14 @@ __global__ void outlier_ranges_kernel(const uint32_t* __restrict__ idx, const ui
         }
         ostart[c] = lo;
     }
-    for (uint32_t i = tid; i + 1 < nout; i += stride)
-        if (idx[i] >= idx[i + 1]) atomicOr(err, kErrUnsorted);
+    bool unsorted = false;
+    for (uint32_t i = tid; i + 1 < nout; i += stride) unsorted |= idx[i] >= idx[i + 1];
     // launched as a programmatic dependent of the RZE prepass, whose offsets it
     // does not read: the fused inverse may start launching now, and this grid
     // ends only after the prepass has, so the inverse's wait covers both
     asm volatile("griddepcontrol.launch_dependents;");
     asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (unsorted) atomicOr(err, kErrUnsorted);  // err was cleared by the prepass at the latest
 }
 
 // Decodes chunk c of a.rze into x (see rze_decode_words); returns its original size.

@@ -146,7 +146,7 @@ __device__ __forceinline__ bool inv_gated_off(const InvArgs& a) {
 __global__ void minmax_kernel(const float* x, uint64_t n, float* pmin, float* pmax,
                               unsigned int* done, int mode, float user_eb, float* st, uint32_t* zero,
                               uint32_t nzero, int with_zero);
-__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* st, uint32_t* zero,
+__global__ void resolve_eb_kernel(int mode, float user_eb, float vb_given, float* st, uint32_t* ctrl, uint32_t* zero,
                                   uint32_t nzero);
 // Quantizes a field of any extents: the tile kernel (2-D, 3-D) and the chunk
 // kernel; returns a cudaError_t value.

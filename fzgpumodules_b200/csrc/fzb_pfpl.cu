@@ -387,7 +387,6 @@ int fzb_pfpl_compress_padded(const float* d_in, uint64_t n_in, uint64_t n, float
     if (!d_work || work_bytes < w.need) return FZB_E_WORKSPACE;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const bool rel = eb_mode == FZB_REL;
-    if (cudaMemsetAsync(d_work, 0, 256, s) != cudaSuccess) return FZB_E_CUDA;
     {
         TraceScope ts(s, "pfpl_resolve_eb");
         if (eb_mode == FZB_NOA && !(value_base > 0.0f)) {
@@ -395,10 +394,12 @@ int fzb_pfpl_compress_padded(const float* d_in, uint64_t n_in, uint64_t n, float
             if (parts > lim) parts = lim;
             if (parts > (uint64_t)kPMaxParts) parts = kPMaxParts;
             if (parts < 1) parts = 1;
+            if (cudaMemsetAsync(d_work, 0, 4 * kCtrlWords, s) != cudaSuccess) return FZB_E_CUDA;
             minmax_kernel<<<(unsigned)parts, 256, 0, s>>>(d_in, n_in, w.pmin, w.pmax, w.mm_done, FZB_NOA, eb, d_eb_state,
                                                           nullptr, 0, n_in < n);
         } else {
-            resolve_eb_kernel<<<1, 32, 0, s>>>(rel ? FZB_ABS : eb_mode, eb, value_base, d_eb_state, nullptr, 0);
+            resolve_eb_kernel<<<1, 32, 0, s>>>(rel ? FZB_ABS : eb_mode, eb, value_base, d_eb_state,
+                                              static_cast<uint32_t*>(d_work), nullptr, 0);
         }
         if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
     }
@@ -472,7 +473,6 @@ int fzb_pfpl_decompress(const void* d_rze, uint64_t rze_bytes, const float* d_ov
     uint32_t* err = static_cast<uint32_t*>(d_work);
     unsigned long long* in_off = reinterpret_cast<unsigned long long*>(static_cast<uint8_t*>(d_work) + 256);
     const uint32_t nch = (uint32_t)((n + kPVals - 1) / kPVals);
-    if (cudaMemsetAsync(d_work, 0, 256, s) != cudaSuccess) return FZB_E_CUDA;
     {
         TraceScope ts(s, "rze_prepass");
         if (launch_rze_prepass(static_cast<const uint8_t*>(d_rze), rze_bytes, nch, (uint32_t)(4 * n), in_off, err,

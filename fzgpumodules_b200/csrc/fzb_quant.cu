@@ -467,7 +467,7 @@ int fzb_quantizer_forward(const float* d_in, uint64_t n, int code_bytes, float e
             if (parts < 1) parts = 1;
             minmax_kernel<<<(unsigned)parts, 256, 0, s>>>(d_in, n, w.pmin, w.pmax, w.mm_done, FZB_NOA, eb, d_eb_state, nullptr, 0, 0);
         } else {
-            resolve_eb_kernel<<<1, 32, 0, s>>>(rel ? FZB_ABS : eb_mode, eb, value_base, d_eb_state, nullptr, 0);
+            resolve_eb_kernel<<<1, 32, 0, s>>>(rel ? FZB_ABS : eb_mode, eb, value_base, d_eb_state, nullptr, nullptr, 0);
         }
         if (cudaGetLastError() != cudaSuccess) return FZB_E_CUDA;
     }
