@@ -209,6 +209,7 @@ __global__ void __launch_bounds__(256) rle_emit_kernel(const T* __restrict__ in,
         uint32_t next = n;
         if (r1 < R) {
             uint32_t lo = blockIdx.x + 1, hi = gridDim.x - 1;  // tile lo .. hi holds run r1
+            if (lo < hi && toff[lo + 1] > r1) hi = lo;         // mostly the next one (3600 x 1800: 15 us, 17 without)
             while (lo < hi) {
                 const uint32_t mid = (lo + hi) >> 1;
                 if (toff[mid + 1] > r1) hi = mid;
@@ -228,12 +229,10 @@ __global__ void __launch_bounds__(256) rle_emit_kernel(const T* __restrict__ in,
 // ---------------------------------------------------------------------------
 // RLE decode.  The run lengths are summed per 1024 runs and the sums scanned;
 // then each 4096-element output tile finds its first tile of runs, scans the
-// lengths of the tiles of runs that overlap it and fills its part of shared
-// memory: short runs by their own thread, longer ones by the whole block.
+// lengths of the tiles of runs that overlap it and places their values.
 //
-// Bound by HBM (lengths read twice, 4 B a run; values and output once).  It
-// replaced a scan that wrote every run's offset and a binary search for every
-// element: the same stream took 5 + 37 + 50 us, now 5 + 32.
+// It replaced a scan that wrote every run's offset and a binary search for every
+// element: the same stream took 5 + 37 + 50 us, now 5 + 26.
 // ---------------------------------------------------------------------------
 constexpr uint32_t kRunTile = 1024;
 
