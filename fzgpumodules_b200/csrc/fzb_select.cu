@@ -479,11 +479,23 @@ __global__ void __launch_bounds__(256) sel_hf_hist_kernel(SelArgs s) {
     for (uint32_t i = t; i < kSelBk; i += 256) h[i] = 0;
     if (t == 0) bad = 0;
     __syncthreads();
-    for (uint32_t i = t; i < cnt; i += 256) {
-        const uint32_t u = src[i];
+    auto count = [&](uint32_t u) {
         if (u < (uint32_t)kSelBk) atomicAdd(&h[u], 1u);
         else bad = 1;
+    };
+    // 16-byte loads (300 chunks: 36 us code by code, 17 so, in two launches)
+    const uint32_t nv = (reinterpret_cast<uintptr_t>(src) & 15) == 0 ? cnt / 8 : 0u;
+#pragma unroll 4
+    for (uint32_t i = t; i < nv; i += 256) {
+        const uint4 q = __ldg(reinterpret_cast<const uint4*>(src) + i);
+        const uint32_t v[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+        for (int k = 0; k < 4; k++) {
+            count(v[k] & 0xffffu);
+            count(v[k] >> 16);
+        }
     }
+    for (uint32_t i = 8 * nv + t; i < cnt; i += 256) count(src[i]);
     __syncthreads();
     uint32_t* f = s.hf_freq + (size_t)c * kSelBk;
     for (uint32_t i = t; i < kSelBk; i += 256) f[i] = h[i];
