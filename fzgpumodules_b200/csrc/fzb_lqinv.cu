@@ -183,6 +183,13 @@ __device__ __forceinline__ float code_bound(uint32_t any) {
     return any ? (float)(1u << (31 - __clz(any))) : 0.0f;
 }
 
+// Whether magnitudes that add up to at most `bound` (a power of two) and the
+// outliers' `osum` stay within 2^24.  A running sum that ever reached 2^24 cannot
+// read below it, so `osum` is exact where it counts; false for infinite ones.
+__device__ __forceinline__ bool sums_exact(float bound, float osum) {
+    return osum < kIntSum && bound <= kIntSum - osum;
+}
+
 // Sum of four deltas' magnitudes.
 template <bool ZZ>
 __device__ __forceinline__ float magnitudes(uint2 w) {
@@ -338,7 +345,7 @@ __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid
 #pragma unroll
         for (int k = 0; k < 8; k++) ors |= abs_bits<ZZ>(w[k].x) | abs_bits<ZZ>(w[k].y);
         ors = __reduce_or_sync(full, ors);
-        if (!(1024.0f * code_bound(ors) + osum <= kIntSum)) {
+        if (!sums_exact(1024.0f * code_bound(ors), osum)) {
             float s = osum;  // the deltas' own magnitudes instead of their bound
 #pragma unroll
             for (int k = 0; k < 8; k++) s += magnitudes<ZZ>(w[k]);
@@ -449,7 +456,7 @@ __global__ void __launch_bounds__(32 * kWarps)
 #pragma unroll
             for (int i = 0; i < 4; i++) ors |= abs_bits<ZZ>(w[k][i]);
         ors = __reduce_or_sync(full, ors);
-        if (!(1024.0f * code_bound(ors) + osum <= kIntSum)) {
+        if (!sums_exact(1024.0f * code_bound(ors), osum)) {
             float s = 0.0f;  // the deltas' own magnitudes instead of their bound
 #pragma unroll
             for (int k = 0; k < 4; k++)
@@ -555,7 +562,7 @@ __global__ void __launch_bounds__(32 * kWarps)
 #pragma unroll
                 for (int j = 0; j < 4; j++) ors |= abs_bits<ZZ>(w[i][j]);
             ors = __reduce_or_sync(full, ors);
-            if (__any_sync(full, osum != 0.0f && !(512.0f * code_bound(ors) + osum <= kIntSum))) {
+            if (__any_sync(full, osum != 0.0f && !sums_exact(512.0f * code_bound(ors), osum))) {
                 float s = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; i++)

@@ -55,3 +55,20 @@ def test_inverse_edges(cuda, dims, kind):
         codes[idx] = 0
     for zigzag, shift in ((True, 0), (False, 0), (True, 1), (True, 2)):
         _run(cuda, dims, codes, err, idx, zigzag, shift)
+
+
+@pytest.mark.parametrize("dims", [(1024, 1, 1), (5000, 1, 1), (32, 32, 1), (100, 70, 1), (8, 8, 8), (33, 17, 9)])
+def test_outliers_that_reach_2_24(cuda, dims):
+    """Sums at 2^24, where adding 1 is lost: which elements lose it depends on the order."""
+    n = int(np.prod(dims))
+    codes = np.zeros(n, np.uint16)
+    for at, values in (((0, 5), (16744448, 32769)), ((0, 13), (16744448, 32769)), ((0, 4, 8), (1 << 24, 1, 1)),
+                       ((0, 8, 16), (1 << 24, 1, 1)), ((0, 1, 2), (1 << 24, 1, 1)), ((0, 1, 2), (1, 1, 1 << 24)),
+                       ((0, 1, 2), (-(1 << 24), -1, -1)), ((0, 3, 5), ((1 << 24) - 1, 1, 1))):
+        for order in (list(range(len(at))), list(range(len(at)))[::-1]):
+            idx = np.array([at[i] for i in order], np.uint32)
+            err = np.array([values[i] for i in order], np.float32)
+            _run(cuda, dims, codes, err, idx, True, 0)
+    # all codes at the largest magnitude their bound allows, and one more from an outlier
+    full = np.full(n, 32767, np.uint16)  # zigzag -16384: 1024 of them reach 2^24
+    _run(cuda, dims, full, np.array([-1], np.float32), np.array([3], np.uint32), True, 0)
