@@ -304,8 +304,7 @@ uint32_t lq_tile_blocks(const FwdArgs& a) {
 }
 
 int launch_lq_tiles(const FwdArgs& a, cudaStream_t s) {
-    (void)launch_dependent(lq_tiles_kernel, lq_tile_blocks(a), 32 * kTileWarps, 0, s, a);
-    return (int)cudaGetLastError();
+    return (int)launch_dependent(lq_tiles_kernel, lq_tile_blocks(a), 32 * kTileWarps, 0, s, a);
 }
 
 int launch_batch_tiles(const BatchArgs& b, uint32_t blocks, cudaStream_t s) {
