@@ -396,6 +396,7 @@ int lq_inverse_common(const uint16_t* d_codes, const float* d_err, const uint32_
     CK(cudaMemsetAsync(w.err, 0, kCtrlBytes, s));
     InvArgs a = inv_args(w, g, n_total);
     a.codes = const_cast<uint16_t*>(d_codes);
+    a.n_codes = (uint32_t)n_total;
     a.out_err = d_err;
     a.out_idx = d_idx;
     a.out_count = d_count;
@@ -604,6 +605,7 @@ int lq_bs_rze_decompress_common(const void* d_rze, uint64_t rze_bytes, const flo
         }
     }
     a.codes = w.codes;
+    a.n_codes = ((uint32_t)n_total + 1u) & ~1u;  // the workspace goes on past an odd number
     if (cap) outlier_records(a, w, g);
     {
         TraceScope ts(s, "rze_decode_bitunshuffle");

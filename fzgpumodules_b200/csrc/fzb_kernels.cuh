@@ -121,6 +121,7 @@ struct InvArgs {
     int zigzag;
     int shuffled;                 // full chunks are bitshuffled (ew = 2)
     float* out;
+    uint32_t n_codes;             // Lorenzo inverse: codes that may be read
     uint32_t* obits;              // Lorenzo inverse: one bit per element with an outlier (null: none)
     uint32_t* otiles;             // with obits: three words a tile (fzb_lqinv.cu), right after the bitmap
     uint64_t ozero;               // words of both, zeroed before the outliers are marked

@@ -31,6 +31,7 @@
 // (now 52 and 5 for the records).  Summing whole tiles in one lane's registers
 // (no shared memory) left too few warps: 21 us for 3600 x 1800, 70 for
 // 500 x 500 x 100.
+#include "fzb_codeload.cuh"
 #include "fzb_rzedec.cuh"
 
 namespace fzb {
@@ -40,32 +41,19 @@ constexpr float kIntSum = 16777216.0f;      // 2^24
 constexpr float kSumSlack = 16700000.0f;    // a rounded sum of 1024 magnitudes below this is below 2^24
 constexpr int kWarps = 4;                   // warps a CTA
 
-// Four codes from element g on (`valid` of them, the rest zero) as two packed
-// pairs; mode 0: codes + g is 8-byte aligned and valid is 0 or 4; 1: codes is
-// 4-byte aligned; 2: single codes.
-__device__ __forceinline__ uint2 load4(const uint16_t* __restrict__ codes, uint32_t g, int valid, int mode) {
-    if (valid <= 0) return make_uint2(0u, 0u);
-    if (mode == 0) return __ldcs(reinterpret_cast<const uint2*>(codes + g));
-    uint2 w = make_uint2(0u, 0u);
-    if (mode == 1) {
-        const uint32_t odd = g & 1u;
-        const uint32_t* p = reinterpret_cast<const uint32_t*>(codes + (g - odd));
-        const uint32_t v0 = __ldg(p), v1 = 2 < valid + (int)odd ? __ldg(p + 1) : 0u,
-                       v2 = 4 < valid + (int)odd ? __ldg(p + 2) : 0u;
-        w.x = odd ? __funnelshift_r(v0, v1, 16) : v0;
-        w.y = odd ? __funnelshift_r(v1, v2, 16) : v1;
-    } else {
-        w.x = __ldg(codes + g);
-        if (valid > 1) w.x |= (uint32_t)__ldg(codes + g + 1) << 16;
-        if (valid > 2) w.y = __ldg(codes + g + 2);
-        if (valid > 3) w.y |= (uint32_t)__ldg(codes + g + 3) << 16;
+// The field's codes as load4 / load8 read them.
+struct GlobalCodes {
+    const uint16_t* p;
+    __device__ __forceinline__ GlobalCodes from(uint32_t g) const { return {p + g}; }
+    __device__ __forceinline__ uint32_t u16(int i) const { return __ldg(p + i); }
+    __device__ __forceinline__ uint32_t u32(int i) const { return __ldg(reinterpret_cast<const uint32_t*>(p + i)); }
+    __device__ __forceinline__ uint2 u64(int i) const { return __ldg(reinterpret_cast<const uint2*>(p + i)); }
+    __device__ __forceinline__ uint2 u64_once(int i) const { return __ldcs(reinterpret_cast<const uint2*>(p + i)); }
+    __device__ __forceinline__ uint4 u128_once(int i) const { return __ldcs(reinterpret_cast<const uint4*>(p + i)); }
+    __device__ __forceinline__ uint32_t shift(uint32_t lo, uint32_t hi, uint32_t bits) const {
+        return __funnelshift_r(lo, hi, bits);
     }
-    if (valid < 4) {
-        if (valid < 2) w.x &= 0xffffu;
-        w.y = valid == 3 ? (w.y & 0xffffu) : 0u;
-    }
-    return w;
-}
+};
 
 // The deltas of two packed code pairs (u - 32768 through 1.5 * 2^23 + u).
 template <bool ZZ>
@@ -104,50 +92,6 @@ __device__ __forceinline__ float4 row_prefix(float4 v) {
     }
     const float ex = __fsub_rn(inc, v.w);  // exact: integers
     return add4(v, make_float4(ex, ex, ex, ex));
-}
-
-// Eight codes from element g on (`valid` of them, the rest zero) as four packed
-// pairs.  mode 0: codes + g is 16-byte aligned, 1: 8-byte aligned (and valid a
-// multiple of 4), 2: codes is 4-byte aligned, 3: single codes.
-__device__ __forceinline__ void load8(const uint16_t* __restrict__ codes, uint32_t g, int valid, int mode,
-                                      uint32_t (&w)[4]) {
-#pragma unroll
-    for (int i = 0; i < 4; i++) w[i] = 0u;
-    if (valid <= 0) return;
-    if (mode == 0 && valid == 8) {
-        const uint4 q = __ldcs(reinterpret_cast<const uint4*>(codes + g));
-        w[0] = q.x, w[1] = q.y, w[2] = q.z, w[3] = q.w;
-        return;
-    }
-    if (mode <= 1) {
-        const uint2 q = __ldg(reinterpret_cast<const uint2*>(codes + g));
-        w[0] = q.x, w[1] = q.y;
-        if (valid > 4) {
-            const uint2 h = __ldg(reinterpret_cast<const uint2*>(codes + g + 4));
-            w[2] = h.x, w[3] = h.y;
-        }
-        return;
-    }
-    if (mode == 2) {
-        const uint32_t odd = g & 1u, sh = 16u * odd;
-        const uint32_t* p = reinterpret_cast<const uint32_t*>(codes + (g - odd));
-        uint32_t v[5];
-#pragma unroll
-        for (int i = 0; i < 5; i++) v[i] = 2 * i < valid + (int)odd ? __ldg(p + i) : 0u;
-#pragma unroll
-        for (int i = 0; i < 4; i++) w[i] = __funnelshift_r(v[i], v[i + 1], sh);
-    } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++)
-            if (i < valid) w[i >> 1] |= (uint32_t)__ldg(codes + g + i) << (16 * (i & 1));
-    }
-    if (valid < 8) {
-#pragma unroll
-        for (int i = 0; i < 4; i++) {
-            if (2 * i >= valid) w[i] = 0u;
-            else if (2 * i + 1 >= valid) w[i] &= 0xffffu;
-        }
-    }
 }
 
 // A pair of codes as two words whose highest set bit grows with the delta's
@@ -340,7 +284,7 @@ __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid
 #pragma unroll
         for (int k = 0; k < 8; k++) {
             const int v = valid(k);
-            w[k] = load4(a.codes, g0 + 128u * k, v, (mode == 0 && v != 4) ? 1 : mode);
+            w[k] = load4(GlobalCodes{a.codes}, g0 + 128u * k, v, v != 4 ? 2 : mode);
         }
 #pragma unroll
         for (int k = 0; k < 8; k++) ors |= abs_bits<ZZ>(w[k].x) | abs_bits<ZZ>(w[k].y);
@@ -448,9 +392,10 @@ __global__ void __launch_bounds__(32 * kWarps)
         const uint32_t ny = min(32u, a.ny - y0), g0 = (y0 + r) * a.nx + x;
         const float osum = has ? __uint_as_float(__ldg(a.otiles + 3u * tile)) : 0.0f;
         const uint32_t rows = has ? __ldg(a.otiles + 3u * tile + 1) : 0u;
+        const int tmode = AL ? mode : end_mode(mode, tile + 1u == ntiles, a.n_codes);  // AL: even rows
         uint32_t w[4][4], ors = 0;
 #pragma unroll
-        for (int k = 0; k < 4; k++) load8(a.codes, g0 + 8 * k * a.nx, r + 8 * k < ny ? nv : 0, mode, w[k]);
+        for (int k = 0; k < 4; k++) load8(GlobalCodes{a.codes}, g0 + 8 * k * a.nx, r + 8 * k < ny ? nv : 0, tmode, w[k]);
 #pragma unroll
         for (int k = 0; k < 4; k++)
 #pragma unroll
@@ -552,9 +497,10 @@ __global__ void __launch_bounds__(32 * kWarps)
             osum = __uint_as_float(__ldg(a.otiles + 3u * tile));
             rows = (__ldg(a.otiles + 3u * tile + 1 + (z >> 2)) >> (8u * (z & 3u))) & 0xffu;
         }
+        const int tmode = AL ? mode : end_mode(mode, wt + 4u >= ntiles, a.n_codes);
         uint32_t w[8][4];
 #pragma unroll
-        for (int i = 0; i < 8; i++) load8(a.codes, g0 + i * a.nx, i < ny ? nvz : 0, mode, w[i]);
+        for (int i = 0; i < 8; i++) load8(GlobalCodes{a.codes}, g0 + i * a.nx, i < ny ? nvz : 0, tmode, w[i]);
         if (__any_sync(full, osum != 0.0f)) {  // NaN counts
             uint32_t ors = 0;
 #pragma unroll
