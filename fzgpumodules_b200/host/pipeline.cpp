@@ -560,8 +560,10 @@ size_t Pipeline::getMaxCompressedSize(size_t input_bytes) const {
 // whose extents are all given and inside the input (an inferred x takes in the
 // padding).  The padded copy they do without read and wrote the whole input: 40
 // of the 350 us of a 500 x 500 x 100 compression.
-bool Pipeline::readsUnpadded(size_t input_size) const {
+// An input off a float's boundary, which the kernels cannot load, is copied too.
+bool Pipeline::readsUnpadded(const void* d_input, size_t input_size) const {
     if (!fused_ || input_size % sizeof(float) != 0) return false;
+    if (reinterpret_cast<uintptr_t>(d_input) % sizeof(float) != 0) return false;
     if (fused_pfpl_) return true;
     const auto d = static_cast<LorenzoQuantStage<float, uint16_t>*>(input_node_->stage)->getDims();
     const size_t y = d[1] ? d[1] : 1, z = d[2] ? d[2] : 1, n = input_size / sizeof(float);
@@ -573,7 +575,7 @@ const void* Pipeline::prepareInput(const void* d_input, size_t input_size, cudaS
     held_bytes_ = 0;
     if (input_alignment_ > 1 && input_size % input_alignment_ != 0) {
         const size_t p = (input_size + input_alignment_ - 1) / input_alignment_ * input_alignment_;
-        if (readsUnpadded(input_size)) {
+        if (readsUnpadded(d_input, input_size)) {
             original_input_size_ = held_bytes_ = input_size;
             *padded = p;
             return d_input;

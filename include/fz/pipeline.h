@@ -272,7 +272,7 @@ private:
     void runForward(cudaStream_t stream);
     void runNode(DAGNode* n, cudaStream_t stream);
     void checkBounds(DAGNode* n);
-    bool readsUnpadded(size_t input_size) const;
+    bool readsUnpadded(const void* d_input, size_t input_size) const;
     const void* prepareInput(const void* d_input, size_t input_size, cudaStream_t stream, size_t* padded);
     void collectMetadata();
     void concatOutputs(void* d_out, size_t capacity, size_t* out_size, cudaStream_t stream);
