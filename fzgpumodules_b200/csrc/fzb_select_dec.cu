@@ -27,17 +27,17 @@ __global__ void __launch_bounds__(1024) sel_offsets_kernel(SelDec a) {
     for (uint32_t c0 = 0; c0 < a.nch; c0 += 1024u) {
         const uint32_t c = c0 + t;
         const uint32_t sz = c < a.nch ? sel_size(a, c) : 0u;
-        // a chunk never holds more than 64 KiB; a larger size ends past the input below
-        const uint32_t words = (uint32_t)min(((uint64_t)sz + 3) / 4, (uint64_t)(1u << 20));
-        uint32_t e0, e1, total, t1;
-        block_scan2_1024(words, 0u, e0, e1, total, t1, ws);
+        // words by low and high halves, so that the sums of 1024 of any size fit
+        const uint32_t words = (uint32_t)(((uint64_t)sz + 3) / 4);
+        uint32_t e0, e1, t0, t1;
+        block_scan2_1024(words & 0xffffu, words >> 16, e0, e1, t0, t1, ws);
         if (c < a.nch) {
-            const uint64_t o = base + e0;
-            a.offs[c] = (uint32_t)min(o, in_words);
-            if (4 * o + sz > a.in_bytes) sel_fail(a, c, kSelMalformed);
-            else if (sel_tag(a, c) > 3u) sel_fail(a, c, kSelMalformed);
+            const uint64_t o = base + e0 + ((uint64_t)e1 << 16);
+            a.offs[c] = (uint32_t)min(min(o, in_words), (uint64_t)0xffffffffu);
+            // (a payload that starts past 2^32 words is refused with those past the input)
+            if (4 * o + sz > a.in_bytes || o > 0xffffffffu || sel_tag(a, c) > 3u) sel_fail(a, c, kSelMalformed);
         }
-        base = min(base + total, in_words);
+        base = min(base + t0 + ((uint64_t)t1 << 16), in_words);
     }
     if (t == 0) *a.state = 1u;
 }

@@ -62,3 +62,21 @@ def test_faults_are_refused(cuda, kind):
         bad(put(16 + pad + 1, 5))       # bits a code (a Bitpack payload has no header)
     else:
         bad(put(first, 77))             # the first payload's own header
+
+
+@pytest.mark.parametrize("kind", range(4))
+def test_chunk_with_a_gap_behind_its_payload(cuda, kind):
+    """A chunk's size in the container may be any that fits the container (here
+    over 4 MiB): the next payload starts behind it."""
+    n = 3 * 32768
+    c = _codes(kind, n)
+    blob, _ = Sel().encode(torch.from_numpy(c).to(cuda), Sel().fixed(kind))
+    b = blob.cpu().numpy()
+    at = 16 + 2 * 4  # three sizes behind the tags and params
+    sizes = b[at: at + 12].view(np.uint32).copy()
+    cut = at + 12 + (int(sizes[0]) + 3) // 4 * 4
+    gap = np.zeros(5 << 20, np.uint8)
+    wide = np.concatenate([b[:cut], gap, b[cut:]])
+    wide[at: at + 4] = np.array([cut - at - 12 + gap.size], np.uint32).view(np.uint8)
+    got = Sel().decode(torch.from_numpy(wide).to(cuda), n).cpu().numpy()
+    assert np.array_equal(got, c)
