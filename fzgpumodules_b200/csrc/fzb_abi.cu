@@ -217,6 +217,7 @@ int forward_common(bool fused, const float* d_in, uint64_t n_in, uint64_t n_tota
     if (!slab && !rows && g.ndim > 1) {
         a.obits = w.big;
         a.obits_words = (g.nfield + 31u) / 32u + 1;
+        a.cells = lq_cells(g.ndim, g.nx, g.ny, g.nz);
     }
     rc = resolve_eb(d_in, n_in, n_total, eb, eb_mode, value_base, w, d_eb_state, a.obits, a.obits_words, s);
     if (rc) return rc;
@@ -1055,6 +1056,7 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
         if (!is_slab[i] && g.ndim > 1) {
             b.a.obits = w.big;
             b.a.obits_words = (g.nfield + 31u) / 32u + 1;
+            b.a.cells = lq_cells(g.ndim, g.nx, g.ny, g.nz);
         }
     }
     // field order of the unit ranges: the chunk kernels' fields first (1-D, then

@@ -55,6 +55,7 @@ struct FwdArgs {
     uint16_t* tcodes;      // 2-D / 3-D tile kernel's output: codes, or the chunk slots (fused)
     uint32_t* obits;       // 2-D / 3-D: one bit per element, set for outliers (zeroed per call)
     uint32_t obits_words;  // its words
+    uint32_t cells;        // 2-D / 3-D: the tile kernel walks elements (lq_cells)
     float* out_err;
     uint32_t* out_idx;
     uint32_t cap;
@@ -156,6 +157,9 @@ int launch_lq_chunk(int ndim, bool fused, const FwdArgs& a, cudaStream_t s);
 // (fzb_tiles.cu); lq_tile_blocks: its CTAs.
 int launch_lq_tiles(const FwdArgs& a, cudaStream_t s);
 uint32_t lq_tile_blocks(const FwdArgs& a);
+// Whether a 2-D / 3-D field fills so little of its tiles that the tile kernel walks
+// its elements instead.
+bool lq_cells(uint32_t ndim, uint32_t nx, uint32_t ny, uint32_t nz);
 // Slab-column fused 3-D kernel (see fzb_forward.cu); `grid` persistent CTAs.
 int launch_lq3d_slab(const FwdArgs& a, unsigned grid, cudaStream_t s);
 // Codes of a 2-D field whose rows are whole chunks (nx % 8192 == 0, no

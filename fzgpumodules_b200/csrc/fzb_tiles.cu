@@ -245,6 +245,142 @@ __device__ __forceinline__ void tiles_3d(const FwdArgs& a, uint32_t wt, uint32_t
     if (!AL) __syncwarp();
 }
 
+// A field whose tiles are mostly empty (lq_cells: a few columns, rows or planes in
+// tiles of 32 or 8), where tile_2d and tiles_3d leave their lanes idle: a warp takes
+// kCellRun consecutive elements, W a lane and step, and forms each delta from the
+// element and its neighbours above and in the plane before, loaded as they are
+// (mostly from L1); the x difference is against the lane before.  A neighbour of
+// another tile counts as 0 (q - 0 is exact).  W = 4 where rows are a multiple of
+// four elements and 16-byte aligned, else 1.
+//
+// Bound by instruction issue.  16.8 M elements with the chunks' encoding behind (us,
+// tiles -> cells): 2-D 1 wide 629 -> 72, 4 wide 119 -> 57, 7 wide 125 -> 72, 8 wide
+// 78 -> 57, two rows 195 -> 60; 3-D 1 x 1 1368 -> 98, 2 x 500 136 -> 93, 1000 x 1
+// 127 -> 69.  The line lies where both meet: in 2-D at 9/16 of the tiles filled (16
+// wide 59.7 and 57.0, 33 wide 75 and 72, but 40 wide, 10/16, 57.3 and 57.5), in 3-D,
+// where the cells read up to four elements for one, at 3/8 (1000 x 3 69.8 and 69.8,
+// 3 x 300 105 and 93, but 4 x 256, 4/8, 61 and 67).
+constexpr uint32_t kCellRun = 1024;
+
+// k / d and k % d for k < 2^31, m = 0xffffffff / d: the estimate is at most one
+// too small.
+__device__ __forceinline__ uint32_t split(uint32_t k, uint32_t d, uint32_t m, uint32_t& rem) {
+    uint32_t q = __umulhi(k, m);
+    rem = k - q * d;
+    if (rem >= d) {
+        rem -= d;
+        q++;
+    }
+    return q;
+}
+
+// W elements from k on and their neighbours (0 outside the tile or the field);
+// tx: the first one has an x predecessor in its tile.
+template <int W>
+struct Cells {
+    float v[W], up[W], back[W], upback[W];
+    bool tx;
+};
+
+template <int W>
+__device__ __forceinline__ void load_cells(const float* p, bool in, float (&v)[W]) {
+    if (W == 4) {
+        const float4 q = in ? __ldg(reinterpret_cast<const float4*>(p)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        v[0] = q.x, v[1 % W] = q.y, v[2 % W] = q.z, v[3 % W] = q.w;
+    } else {
+        v[0] = in ? __ldg(p) : 0.0f;
+    }
+}
+
+// The differences along z (3-D) or y (2-D).
+template <int W>
+__device__ __forceinline__ void quant_sub(const float (&v)[W], const float (&w)[W], float r, float (&d)[W]) {
+    if (W == 4) {
+        const Q4 a = quant4(make_float4(v[0], v[1 % W], v[2 % W], v[3 % W]), r);
+        const Q4 b = quant4(make_float4(w[0], w[1 % W], w[2 % W], w[3 % W]), r);
+        const float2 x = sub2(a.a, b.a), y = sub2(a.b, b.b);
+        d[0] = x.x, d[1 % W] = x.y, d[2 % W] = y.x, d[3 % W] = y.y;
+    } else {
+        auto q = [&](float u) { return truncf(__fadd_rn(__fmul_rn(u, r), __uint_as_float(half_bits(u)))); };
+        d[0] = __fsub_rn(q(v[0]), q(w[0]));
+    }
+}
+
+template <int NDIM, bool ZZ, int W>
+__device__ __forceinline__ void cells(const FwdArgs& a, uint32_t warp, float r) {
+    constexpr uint32_t kIn = NDIM == 3 ? 7u : 31u;  // a place in the tile: its low bits
+    constexpr int U = W == 4 ? 2 : 4;               // steps with their loads in flight together
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu, n = a.nfield, k0 = warp * kCellRun;
+    if (k0 >= n) return;
+    const uint32_t my = ~0u / a.nx, mz = NDIM == 3 ? ~0u / a.plane : 0u;
+    auto load = [&](uint32_t k, Cells<W>& c) {
+        uint32_t rem = k, x;
+        const bool in = k < n, tz = NDIM == 3 && in && (split(k, a.plane, mz, rem) & kIn) != 0;
+        const bool ty = (split(rem, a.nx, my, x) & kIn) != 0 && in;
+        c.tx = (x & kIn) != 0;
+        const float* p = a.in + k;
+        load_cells<W>(p, in, c.v);
+        load_cells<W>(p - a.nx, ty, c.up);
+        if (NDIM == 3) {
+            load_cells<W>(p - a.plane, tz, c.back);
+            load_cells<W>(p - a.plane - a.nx, ty && tz, c.upback);
+        }
+    };
+    auto first = [&](const Cells<W>& c, float (&d)[W], float (&du)[W]) {
+        quant_sub<W>(c.v, NDIM == 3 ? c.back : c.up, r, d);
+        if (NDIM == 3) quant_sub<W>(c.up, c.upback, r, du);
+    };
+    float cd = 0.0f, cu = 0.0f;  // of the element before the run
+    if (k0) {
+        Cells<W> c;
+        float d[W], du[W];
+        load(k0 - W, c);
+        first(c, d, du);
+        cd = d[W - 1];
+        if (NDIM == 3) cu = du[W - 1];
+    }
+    for (uint32_t b = k0; b < min(n, k0 + kCellRun); b += 32u * W * U) {
+        Cells<W> c[U];
+#pragma unroll
+        for (int i = 0; i < U; i++) load(b + W * (32u * i + lane), c[i]);
+#pragma unroll
+        for (int i = 0; i < U; i++) {
+            float d[W], du[W];
+            first(c[i], d, du);
+            const float nd = __shfl_up_sync(full, d[W - 1], 1), ld = lane ? nd : cd;
+            cd = __shfl_sync(full, d[W - 1], 31);
+            float lu = 0.0f;
+            if (NDIM == 3) {
+                const float nu = __shfl_up_sync(full, du[W - 1], 1);
+                lu = lane ? nu : cu;
+                cu = __shfl_sync(full, du[W - 1], 31);
+            }
+            // 2-D: y, x (lorenzo_quant_nd.cu:72-77); 3-D: z, x, y (:234-246)
+            const uint32_t k = b + W * (32u * i + lane);
+            if (W == 4) {
+                Q4 e = xdiff(Q4{f2(d[0], d[1 % W]), f2(d[2 % W], d[3 % W])}, c[i].tx ? ld : 0.0f);
+                if (NDIM == 3) {
+                    const Q4 u = xdiff(Q4{f2(du[0], du[1 % W]), f2(du[2 % W], du[3 % W])}, c[i].tx ? lu : 0.0f);
+                    e = Q4{sub2(e.a, u.a), sub2(e.b, u.b)};
+                }
+                uint32_t m;
+                const uint2 p = codes4<ZZ>(e, a.radius, m);
+                if (k < n) {
+                    *reinterpret_cast<uint2*>(a.tcodes + k) = p;
+                    if (m) mark_bits(a.obits, k, m);
+                }
+            } else {
+                float e = __fsub_rn(d[0], c[i].tx ? ld : 0.0f);
+                if (NDIM == 3) e = __fsub_rn(e, __fsub_rn(du[0], c[i].tx ? lu : 0.0f));
+                const bool in = fabsf(e) < a.radius;
+                const uint32_t m = __ballot_sync(full, !in && k < n);
+                if (k < n) a.tcodes[k] = (uint16_t)code_pair<ZZ>(f2(in ? e : 0.0f, 0.0f));
+                if (m && lane == 0) a.obits[(b >> 5) + i] = m;
+            }
+        }
+    }
+}
+
 // How a field's rows are read and written: bit 0 aligned input rows, bits 1-2
 // the store mode (0: 16 bytes, 1: 8 bytes, else single codes).
 __device__ __host__ __forceinline__ int tile_modes(const FwdArgs& a) {
@@ -259,6 +395,11 @@ __device__ __forceinline__ void tile_block(const FwdArgs& a, uint32_t block, Til
     const uint32_t warp = block * kTileWarps + (threadIdx.x >> 5);
     const float r = *a.ebx2_r;
     const int modes = tile_modes(a), smode = modes >> 1;
+    if (a.cells) {
+        if (modes & 1) a.nz > 1 ? cells<3, ZZ, 4>(a, warp, r) : cells<2, ZZ, 4>(a, warp, r);
+        else a.nz > 1 ? cells<3, ZZ, 1>(a, warp, r) : cells<2, ZZ, 1>(a, warp, r);
+        return;
+    }
     if (a.nz > 1) {
         const uint32_t n = ((a.nx + 7u) / 8u) * ((a.ny + 7u) / 8u) * ((a.nz + 7u) / 8u), wt = 4u * warp;
         if (wt >= n) return;
@@ -297,8 +438,15 @@ __global__ void __launch_bounds__(32 * kTileWarps, 8) batch_tiles_kernel(BatchAr
 
 }  // namespace
 
+bool lq_cells(uint32_t ndim, uint32_t nx, uint32_t ny, uint32_t nz) {
+    auto up = [](uint32_t v, uint32_t to) { return (uint64_t)((v + to - 1) / to * to); };
+    const uint64_t n = (uint64_t)nx * ny * nz;
+    return ndim == 2 ? 16 * n <= 9 * up(nx, 32) * up(ny, 32) : 8 * n <= 3 * up(nx, 8) * up(ny, 8) * up(nz, 8);
+}
+
 uint32_t lq_tile_blocks(const FwdArgs& a) {
-    const uint64_t warps = a.nz > 1 ? ((uint64_t)((a.nx + 7u) / 8u) * ((a.ny + 7u) / 8u) * ((a.nz + 7u) / 8u) + 3) / 4
+    const uint64_t warps = a.cells ? (a.nfield + kCellRun - 1u) / kCellRun
+                         : a.nz > 1 ? ((uint64_t)((a.nx + 7u) / 8u) * ((a.ny + 7u) / 8u) * ((a.nz + 7u) / 8u) + 3) / 4
                                     : (uint64_t)((a.nx + 31u) / 32u) * ((a.ny + 31u) / 32u);
     return (uint32_t)((warps + kTileWarps - 1) / kTileWarps);
 }

@@ -57,6 +57,39 @@ def test_codes_and_chain(cuda, dims, radius, special):
                 assert np.array_equal(out["codes"].cpu().numpy(), codes)
 
 
+# fields that fill little of their tiles, on both sides of the line, rows a multiple
+# of four elements and not, runs of 1024 elements ending inside the field
+NARROW = [(1, 2, 1), (1, 5000, 1), (2, 3001, 1), (3, 1025, 1), (4, 2049, 1), (5, 999, 1), (7, 700, 1), (8, 601, 1),
+          (16, 200, 1), (18, 130, 1), (19, 64, 1), (4100, 2, 1), (4099, 3, 1), (2000, 18, 1), (333, 19, 1),
+          (1, 1, 5000), (1, 300, 9), (2, 2, 999), (3, 300, 7), (4, 4, 100), (4, 6, 90), (100, 2, 31), (1001, 1, 17),
+          (1000, 3, 9), (33, 3, 40), (64, 64, 2), (65, 31, 3)]
+
+
+@pytest.mark.parametrize("special", [False, True])
+@pytest.mark.parametrize("radius", [32768, 40])
+@pytest.mark.parametrize("dims", NARROW)
+def test_narrow_fields(cuda, dims, radius, special):
+    test_codes_and_chain(cuda, dims, radius, special)
+
+
+def test_narrow_fields_in_a_batch(cuda):
+    from fzgpumodules_b200 import kernels as K
+    fields = [dict(x=torch.from_numpy(_field(d, 7 + i, False)).to(cuda), dims=d, eb=1e-2, mode=K.ABS,
+                   radius=40 if i % 2 else 32768, zigzag=True)
+              for i, d in enumerate(NARROW + [(100, 90, 1), (5000, 1, 1), (100, 41, 9)])]
+    b = K.Batch(fields)
+    b.launch()
+    torch.cuda.synchronize()
+    for f, o in zip(fields, b.outputs):
+        r = K.lq_bs_rze_compress(f["x"], f["dims"], f["eb"], f["mode"], f["radius"], True, 0.2)
+        size, cnt = int(r["rze_size"].item()), int(r["count"].item())
+        assert int(o["rze_size"].item()) == size and torch.equal(o["rze"][:size], r["rze"][:size])
+        assert int(o["count"].item()) == cnt
+        kept = min(cnt, r["cap"])
+        assert torch.equal(o["idx"][:kept], r["idx"][:kept]) and torch.equal(o["err"][:kept], r["err"][:kept])
+    b.close()
+
+
 @pytest.mark.parametrize("mode", [0, 1, 2])
 @pytest.mark.parametrize("dims", [(5000, 1, 1), (100, 41, 1), (33, 17, 9), (90, 91, 1)])
 def test_padding_is_counted_without_a_copy(cuda, dims, mode):
