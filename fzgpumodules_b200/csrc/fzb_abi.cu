@@ -1057,6 +1057,9 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
             b.a.obits = w.big;
             b.a.obits_words = (g.nfield + 31u) / 32u + 1;
             b.a.cells = lq_cells(g.ndim, g.nx, g.ny, g.nz);
+            // blocks past the scan's only clear the bitmap (4000 x 4000 with an absolute
+            // bound, which needs no scan: 109 us with one block for its 2 MB)
+            mm_grid = std::max(mm_grid, 1 + std::min(b.a.obits_words / 4096u, 592u));
         }
     }
     // field order of the unit ranges: the chunk kernels' fields first (1-D, then

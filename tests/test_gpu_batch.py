@@ -113,3 +113,25 @@ def test_batch_graph_replay(cuda):
         _same(o, r)
     del g
     b.close()
+
+
+def test_absolute_bound_costs_no_more_than_a_scan(cuda):
+    """A field with an absolute bound has its outlier bitmap cleared by as many
+    blocks as one whose value base is scanned for."""
+    from fzgpumodules_b200 import fields as F
+    x = F.grf((4000, 4000), seed=3, device=cuda).reshape(-1).contiguous()
+
+    def least(mode):
+        b = K().Batch([dict(x=x, dims=(4000, 4000, 1), eb=1e-3, mode=mode, radius=32768, zigzag=True)])
+        times = []
+        for _ in range(12):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(10):
+                b.launch()
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        b.close()
+        return min(times)
+    assert least(K().ABS) < least(K().REL)
