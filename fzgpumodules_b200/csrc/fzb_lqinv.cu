@@ -290,12 +290,12 @@ __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid
         for (int k = 0; k < 8; k++) ors |= abs_bits<ZZ>(w[k].x) | abs_bits<ZZ>(w[k].y);
         ors = __reduce_or_sync(full, ors);
         if (!sums_exact(1024.0f * code_bound(ors), osum)) {
-            float s = osum;  // the deltas' own magnitudes instead of their bound
+            float s = 0.0f;  // the deltas' own magnitudes instead of their bound
 #pragma unroll
             for (int k = 0; k < 8; k++) s += magnitudes<ZZ>(w[k]);
 #pragma unroll
             for (int d = 16; d >= 1; d >>= 1) s += __shfl_xor_sync(full, s, d);
-            if (!(s < kSumSlack)) {
+            if (!(s + osum < kSumSlack)) {
                 exact_tile_1d(a, base, has, ebx2);
                 continue;
             }

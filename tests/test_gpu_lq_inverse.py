@@ -72,3 +72,31 @@ def test_outliers_that_reach_2_24(cuda, dims):
     # all codes at the largest magnitude their bound allows, and one more from an outlier
     full = np.full(n, 32767, np.uint16)  # zigzag -16384: 1024 of them reach 2^24
     _run(cuda, dims, full, np.array([-1], np.float32), np.array([3], np.uint32), True, 0)
+
+
+def test_outlier_sum_of_a_flat_tile_is_counted_once(cuda):
+    """1-D tiles with a code of the largest bound and one outlier: a sum of 600,000
+    is far below 2^24 and takes no longer than one of 400,000."""
+    from fzgpumodules_b200 import kernels as K
+    n = 1 << 24
+    codes = torch.zeros(n, dtype=torch.int16, device=cuda)
+    codes[5::1024] = 32767
+    idx = torch.arange(9, n, 1024, dtype=torch.int32, device=cuda)
+    cnt = torch.tensor([idx.numel()], dtype=torch.int32, device=cuda)
+
+    def least(value):
+        err = torch.full((idx.numel(),), float(value), device=cuda)
+        times = []
+        for _ in range(10):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(5):
+                y = K.lq_inverse(codes.view(torch.uint16), err, idx, cnt, idx.numel(), (n, 1, 1), 1.0, True)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        assert y[4] == 0 and y[1023] == 2 * (value - 16384)
+        return min(times)
+    t = least(400000), least(600000)
+    print("us a call", [1e3 * v / 5 for v in t])
+    assert t[1] < 1.2 * t[0]
