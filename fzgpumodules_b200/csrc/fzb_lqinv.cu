@@ -20,7 +20,12 @@
 // tile without outliers is known by one load, and rows without them take no
 // extra work.  The condition then follows from that sum and a bound on the
 // codes (in 3-D without outliers 512 deltas of at most 2^15 always meet it); a
-// tile where it fails takes the reference's add tree.
+// tile where it fails takes the reference's add tree, in a function of its own
+// (inlined it cost registers): in 3-D from the deltas in shared memory, in 1-D and
+// 2-D from the codes, loaded again by rows.  Read code by code from memory, with the
+// bitmap for each, the trees took 283 us where 500 x 500 x 100 has 0.65 % outliers
+// of up to 4e7 (now 79; 109 when every tile took them by CTAs), and 93
+// for 4096 x 4096 codes of all 16 bits (now 42; 65).
 //
 // Bound by HBM in 2-D (2 B of code read, 4 B written an element: 8192 x 8192 in
 // 87 us, 4.6 TB/s) and by load latency at the warps that 80 registers and the
@@ -141,23 +146,19 @@ __device__ __forceinline__ float magnitudes(uint2 w) {
     return (fabsf(d.x) + fabsf(d.y)) + (fabsf(d.z) + fabsf(d.w));
 }
 
-__device__ __forceinline__ float delta_at(const InvArgs& a, bool zz, bool has, uint32_t g) {
-    const float c = decode_code(a.codes[g], zz);
-    if (!has || !((a.obits[g >> 5] >> (g & 31u)) & 1u)) return __fadd_rn(0.0f, c);
-    return __fadd_rn(a.out[g], c);
-}
-
-// The reference's add trees, one tile (in 3-D up to four tiles of a row) a warp.
-__device__ __noinline__ void exact_tile_1d(const InvArgs& a, uint32_t base, bool has, float ebx2) {
+// The reference's add trees, a warp one tile (in 3-D four).  rows: the steps of 128
+// elements that hold outliers; mode: load4's.
+template <bool ZZ>
+__device__ __noinline__ void exact_tile_1d(const InvArgs& a, uint32_t base, uint32_t rows, int mode, float ebx2) {
     const uint32_t lane = threadIdx.x & 31u;
-    const bool zz = a.zigzag != 0;
     float tot[8];
 #pragma unroll
     for (int vw = 0; vw < 8; vw++) {  // the reference's eight warps of four elements a thread
         const uint32_t g0 = base + 128u * vw + 4u * lane;
-        float v[4];
-#pragma unroll
-        for (int i = 0; i < 4; i++) v[i] = g0 + i < a.nfield ? delta_at(a, zz, has, g0 + i) : 0.0f;
+        const int valid = g0 < a.nfield ? (int)min(4u, a.nfield - g0) : 0;
+        float4 d = deltas4<ZZ>(load4(GlobalCodes{a.codes}, g0, valid, valid != 4 ? 2 : mode));
+        if ((rows >> vw) & 1u) d = with_outliers(d, a, g0, valid);
+        float v[4] = {d.x, d.y, d.z, d.w};
 #pragma unroll
         for (int i = 1; i < 4; i++) v[i] = __fadd_rn(v[i], v[i - 1]);
         float ts = v[3];
@@ -189,78 +190,6 @@ __device__ __noinline__ void exact_tile_1d(const InvArgs& a, uint32_t base, bool
 #pragma unroll
         for (int i = 0; i < 4; i++)
             if (g0 + i < a.nfield) a.out[g0 + i] = __fmul_rn(v[i], ebx2);
-    }
-}
-
-__device__ __noinline__ void exact_tile_2d(const InvArgs& a, uint32_t x0, uint32_t y0, bool has, float ebx2) {
-    const uint32_t lane = threadIdx.x & 31u, gx = x0 + lane;
-    const bool zz = a.zigzag != 0;
-    float tot[4];
-#pragma unroll
-    for (int wy = 0; wy < 4; wy++) {  // the reference's four groups of 8 rows
-        float v[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t gy = y0 + 8u * wy + i;
-            v[i] = (gx < a.nx && gy < a.ny) ? delta_at(a, zz, has, gy * a.nx + gx) : 0.0f;
-        }
-#pragma unroll
-        for (int i = 1; i < 8; i++) v[i] = __fadd_rn(v[i], v[i - 1]);
-        tot[wy] = v[7];
-        if (wy > 0) {
-            float add = tot[0];
-            if (wy > 1) add = __fadd_rn(add, tot[1]);
-            if (wy > 2) add = __fadd_rn(add, tot[2]);
-#pragma unroll
-            for (int i = 0; i < 8; i++) v[i] = __fadd_rn(v[i], add);
-        }
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const float n = __shfl_up_sync(0xffffffffu, v[i], d);
-                if ((int)lane >= d) v[i] = __fadd_rn(v[i], n);
-            }
-            const uint32_t gy = y0 + 8u * wy + i;
-            if (gx < a.nx && gy < a.ny) a.out[gy * a.nx + gx] = __fmul_rn(v[i], ebx2);
-        }
-    }
-}
-
-__device__ __noinline__ void exact_brick_3d(const InvArgs& a, uint32_t x0, uint32_t y0, uint32_t z0, uint32_t tiles,
-                                            bool has, float ebx2) {
-    const uint32_t lane = threadIdx.x & 31u, gx = lane < 8u * tiles ? x0 + lane : a.nx;
-    const bool zz = a.zigzag != 0;
-    float run[8];
-#pragma unroll
-    for (int z = 0; z < 8; z++) run[z] = 0.0f;
-#pragma unroll
-    for (int y = 0; y < 8; y++) {
-        const uint32_t gy = y0 + y;
-        float w[8];
-#pragma unroll
-        for (int z = 0; z < 8; z++) {
-            const uint32_t gz = z0 + z;
-            const float v = (gx < a.nx && gy < a.ny && gz < a.nz)
-                                ? delta_at(a, zz, has, (gz * a.ny + gy) * a.nx + gx) : 0.0f;
-            run[z] = y == 0 ? v : __fadd_rn(v, run[z]);
-            w[z] = run[z];
-#pragma unroll
-            for (int d = 1; d < 8; d <<= 1) {
-                const float n = __shfl_up_sync(0xffffffffu, w[z], d, 8);
-                if ((int)(lane & 7u) >= d) w[z] = __fadd_rn(w[z], n);
-            }
-        }
-#pragma unroll
-        for (int d = 1; d < 8; d <<= 1)
-#pragma unroll
-            for (int z = 7; z >= 1; z--)
-                if (z >= d) w[z] = __fadd_rn(w[z], w[z - d]);
-#pragma unroll
-        for (int z = 0; z < 8; z++) {
-            const uint32_t gz = z0 + z;
-            if (gx < a.nx && gy < a.ny && gz < a.nz) a.out[(gz * a.ny + gy) * a.nx + gx] = __fmul_rn(w[z], ebx2);
-        }
     }
 }
 
@@ -296,7 +225,7 @@ __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid
 #pragma unroll
             for (int d = 16; d >= 1; d >>= 1) s += __shfl_xor_sync(full, s, d);
             if (!(s + osum < kSumSlack)) {
-                exact_tile_1d(a, base, has, ebx2);
+                exact_tile_1d<ZZ>(a, base, rows, mode, ebx2);
                 continue;
             }
         }
@@ -354,16 +283,26 @@ __device__ __forceinline__ void stage_outliers(const InvArgs& a, uint32_t g0, ui
     }
 }
 
-// The x prefix of eight deltas, with the outliers staged at p when the row has
-// any.
+// Bit k: row r + 8k of a 2-D tile holds outliers.
+__device__ __forceinline__ uint32_t lane_rows(uint32_t rows, uint32_t r) {
+    return ((rows >> r) & 1u) | ((rows >> (r + 7u)) & 2u) | ((rows >> (r + 14u)) & 4u) | ((rows >> (r + 21u)) & 8u);
+}
+
+// Eight deltas, with the outliers staged at p when the row has any.
 template <bool ZZ>
-__device__ __forceinline__ void prefix8(const uint32_t (&w)[4], bool row, const float* p, float4& lo, float4& hi) {
+__device__ __forceinline__ void deltas8(const uint32_t (&w)[4], bool row, const float* p, float4& lo, float4& hi) {
     lo = deltas4<ZZ>(make_uint2(w[0], w[1]));
     hi = deltas4<ZZ>(make_uint2(w[2], w[3]));
     if (row) {
         lo = add4(lo, *reinterpret_cast<const float4*>(p));
         hi = add4(hi, *reinterpret_cast<const float4*>(p + 4));
     }
+}
+
+// Their x prefix.
+template <bool ZZ>
+__device__ __forceinline__ void prefix8(const uint32_t (&w)[4], bool row, const float* p, float4& lo, float4& hi) {
+    deltas8<ZZ>(w, row, p, lo, hi);
     lo.y = __fadd_rn(lo.y, lo.x);
     lo.z = __fadd_rn(lo.z, lo.y);
     lo.w = __fadd_rn(lo.w, lo.z);
@@ -371,6 +310,96 @@ __device__ __forceinline__ void prefix8(const uint32_t (&w)[4], bool row, const 
     hi.y = __fadd_rn(hi.y, hi.x);
     hi.z = __fadd_rn(hi.z, hi.y);
     hi.w = __fadd_rn(hi.w, hi.z);
+}
+
+// The add trees of a 2-D tile: its deltas go to the strip first (36 floats a row).
+template <bool ZZ>
+__device__ __noinline__ void exact_tile_2d(const InvArgs& a, float* strip, uint32_t x0, uint32_t y0, uint32_t rows,
+                                           int mode, float ebx2) {
+    const uint32_t lane = threadIdx.x & 31u, r = lane >> 2, x = x0 + 8u * (lane & 3u);
+    const int nv = x < a.nx ? (int)min(8u, a.nx - x) : 0, ny = (int)min(32u, a.ny - y0);
+    const uint32_t g0 = (y0 + r) * a.nx + x;
+    float* mine = strip + 36u * r + 8u * (lane & 3u);
+    const uint32_t lrows = lane_rows(rows, r);
+    if (rows) stage_outliers<4>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        uint32_t w[4];
+        load8(GlobalCodes{a.codes}, g0 + 8 * k * a.nx, (int)r + 8 * k < ny ? nv : 0, mode, w);
+        float4 lo, hi;
+        float* p = mine + 36 * 8 * k;
+        deltas8<ZZ>(w, (lrows >> k) & 1u, p, lo, hi);
+        *reinterpret_cast<float4*>(p) = lo;
+        *reinterpret_cast<float4*>(p + 4) = hi;
+    }
+    __syncwarp();
+    float* out = a.out + (size_t)y0 * a.nx + x0 + lane;  // the lane's column
+    float tot[4];
+#pragma unroll
+    for (int wy = 0; wy < 4; wy++) {  // the reference's four groups of 8 rows
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++) v[i] = strip[36 * (8 * wy + i) + lane];
+#pragma unroll
+        for (int i = 1; i < 8; i++) v[i] = __fadd_rn(v[i], v[i - 1]);
+        tot[wy] = v[7];
+        if (wy > 0) {
+            float add = tot[0];
+            if (wy > 1) add = __fadd_rn(add, tot[1]);
+            if (wy > 2) add = __fadd_rn(add, tot[2]);
+#pragma unroll
+            for (int i = 0; i < 8; i++) v[i] = __fadd_rn(v[i], add);
+        }
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1)
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                const float n = __shfl_up_sync(0xffffffffu, v[i], d);
+                if ((int)lane >= d) v[i] = __fadd_rn(v[i], n);
+            }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (x0 + lane < a.nx && 8 * wy + i < ny) out[(size_t)(8 * wy + i) * a.nx] = __fmul_rn(v[i], ebx2);
+    }
+    __syncwarp();
+}
+
+// The add trees of four 3-D tiles, whose deltas are in the brick (260 floats a
+// plane); tile lane % 4 starts at element base and has nv x ny x nz elements.
+__device__ __noinline__ void exact_brick_3d(const InvArgs& a, const float* brick, uint32_t base, int nv, int ny,
+                                            int nz, float ebx2) {
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu;
+    const uint32_t t = lane >> 3;  // the tile of the lane's column
+    float* out = a.out + __shfl_sync(full, base, t) + (lane & 7u);
+    const bool in = (int)(lane & 7u) < __shfl_sync(full, nv, t);
+    const int tny = __shfl_sync(full, ny, t), tnz = __shfl_sync(full, nz, t);
+    float run[8];
+#pragma unroll
+    for (int y = 0; y < 8; y++) {
+        float w[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            const float v = brick[260 * k + 32 * y + lane];
+            run[k] = y == 0 ? v : __fadd_rn(v, run[k]);
+            w[k] = run[k];
+        }
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1)
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                const float n = __shfl_up_sync(full, w[k], d, 8);
+                if ((int)(lane & 7u) >= d) w[k] = __fadd_rn(w[k], n);
+            }
+#pragma unroll
+        for (int d = 1; d < 8; d <<= 1)
+#pragma unroll
+            for (int k = 7; k >= 1; k--)
+                if (k >= d) w[k] = __fadd_rn(w[k], w[k - d]);
+#pragma unroll
+        for (int k = 0; k < 8; k++)
+            if (in && y < tny && k < tnz) out[(size_t)k * a.plane + y * a.nx] = __fmul_rn(w[k], ebx2);
+    }
+    __syncwarp();
 }
 
 // 2-D: a warp a 32x32 tile.  Rows of the shared tile are padded to 36 floats,
@@ -409,14 +438,12 @@ __global__ void __launch_bounds__(32 * kWarps)
 #pragma unroll
             for (int d = 16; d >= 1; d >>= 1) s += __shfl_xor_sync(full, s, d);
             if (!(s + osum < kSumSlack)) {
-                exact_tile_2d(a, x0, y0, has, ebx2);
+                exact_tile_2d<ZZ>(a, strip, x0, y0, rows, tmode, ebx2);
                 continue;
             }
         }
         float* mine = strip + 36u * r + 8u * c;
-        // bit k: the lane's k-th row (r + 8k) holds outliers
-        const uint32_t lrows = ((rows >> r) & 1u) | ((rows >> (r + 7u)) & 2u) | ((rows >> (r + 14u)) & 4u) |
-                               ((rows >> (r + 21u)) & 8u);
+        const uint32_t lrows = lane_rows(rows, r);
         if (rows) stage_outliers<4>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
@@ -501,6 +528,7 @@ __global__ void __launch_bounds__(32 * kWarps)
         uint32_t w[8][4];
 #pragma unroll
         for (int i = 0; i < 8; i++) load8(GlobalCodes{a.codes}, g0 + i * a.nx, i < ny ? nvz : 0, tmode, w[i]);
+        bool exact = true;
         if (__any_sync(full, osum != 0.0f)) {  // NaN counts
             uint32_t ors = 0;
 #pragma unroll
@@ -508,27 +536,33 @@ __global__ void __launch_bounds__(32 * kWarps)
 #pragma unroll
                 for (int j = 0; j < 4; j++) ors |= abs_bits<ZZ>(w[i][j]);
             ors = __reduce_or_sync(full, ors);
-            if (__any_sync(full, osum != 0.0f && !sums_exact(512.0f * code_bound(ors), osum))) {
+            exact = !__any_sync(full, osum != 0.0f && !sums_exact(512.0f * code_bound(ors), osum));
+            if (!exact) {
                 float s = 0.0f;
 #pragma unroll
                 for (int i = 0; i < 8; i++)
                     s += magnitudes<ZZ>(make_uint2(w[i][0], w[i][1])) + magnitudes<ZZ>(make_uint2(w[i][2], w[i][3]));
 #pragma unroll
                 for (int d = 16; d >= 4; d >>= 1) s += __shfl_xor_sync(full, s, d);
-                if (__any_sync(full, osum != 0.0f && !(s + osum < kSumSlack))) {
-                    for (uint32_t k = wt; k < min(wt + 4u, ntiles);) {
-                        const uint32_t kx = k % tx, cnt = min(tx - kx, min(wt + 4u, ntiles) - k);
-                        exact_brick_3d(a, kx * 8u, ((k / tx) % ty) * 8u, (k / (tx * ty)) * 8u, cnt, has, ebx2);
-                        k += cnt;
-                    }
-                    continue;
-                }
+                exact = !__any_sync(full, osum != 0.0f && !(s + osum < kSumSlack));
             }
+        }
+        float* p = brick + 260u * z + 8u * c;
+        if (__any_sync(full, rows != 0u)) stage_outliers<8>(a, g0, a.nx, nvz, rows, p, 32u);
+        if (!exact) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) {
+                float4 lo, hi;
+                deltas8<ZZ>(w[i], (rows >> i) & 1u, p + 32 * i, lo, hi);
+                *reinterpret_cast<float4*>(p + 32 * i) = lo;
+                *reinterpret_cast<float4*>(p + 32 * i + 4) = hi;
+            }
+            __syncwarp();
+            exact_brick_3d(a, brick, base, nv, ny, nz, ebx2);
+            continue;
         }
         {
             float4 ylo = make_float4(0.0f, 0.0f, 0.0f, 0.0f), yhi = ylo;
-            float* p = brick + 260u * z + 8u * c;
-            if (__any_sync(full, rows != 0u)) stage_outliers<8>(a, g0, a.nx, nvz, rows, p, 32u);
 #pragma unroll
             for (int i = 0; i < 8; i++) {
                 float4 lo, hi;

@@ -100,3 +100,30 @@ def test_outlier_sum_of_a_flat_tile_is_counted_once(cuda):
     t = least(400000), least(600000)
     print("us a call", [1e3 * v / 5 for v in t])
     assert t[1] < 1.2 * t[0]
+
+
+@pytest.mark.parametrize("dims", [(200, 200, 200), (1600, 1500, 1)])
+def test_large_outliers_cost_little_more(cuda, dims):
+    """Outliers past 2^24 send their tiles to the add trees: at most twice the time
+    of ones that do not (an element in a thousand is one)."""
+    from fzgpumodules_b200 import kernels as K
+    n = int(np.prod(dims))
+    codes = torch.zeros(n, dtype=torch.int16, device=cuda).view(torch.uint16)
+    idx = torch.arange(9, n, 997, dtype=torch.int32, device=cuda)
+    cnt = torch.tensor([idx.numel()], dtype=torch.int32, device=cuda)
+
+    def least(value):
+        err = torch.full((idx.numel(),), float(value), device=cuda)
+        times = []
+        for _ in range(10):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(10):
+                K.lq_inverse(codes, err, idx, cnt, idx.numel(), dims, 1.0, True)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        return min(times)
+    t = least(50000), least(1 << 25)
+    print("us a call", [100 * v for v in t])
+    assert t[1] < 2 * t[0]
