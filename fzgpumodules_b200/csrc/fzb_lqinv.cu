@@ -44,6 +44,7 @@ namespace {
 
 constexpr float kIntSum = 16777216.0f;      // 2^24
 constexpr float kSumSlack = 16700000.0f;    // a rounded sum of 1024 magnitudes below this is below 2^24
+constexpr int kFewOutliers = 8;             // a lane's outliers loaded one by one
 constexpr int kWarps = 4;                   // warps a CTA
 
 // The field's codes as load4 / load8 read them.
@@ -151,14 +152,20 @@ __device__ __forceinline__ float magnitudes(uint2 w) {
 template <bool ZZ>
 __device__ __noinline__ void exact_tile_1d(const InvArgs& a, uint32_t base, uint32_t rows, int mode, float ebx2) {
     const uint32_t lane = threadIdx.x & 31u;
+    auto deltas = [&](int vw) {
+        const uint32_t g = base + 128u * vw + 4u * lane;
+        const int valid = g < a.nfield ? (int)min(4u, a.nfield - g) : 0;
+        float4 d = deltas4<ZZ>(load4(GlobalCodes{a.codes}, g, valid, valid != 4 ? 2 : mode));
+        if ((rows >> vw) & 1u) d = with_outliers(d, a, g, valid);
+        return d;
+    };
     float tot[8];
+    float4 next = deltas(0);
 #pragma unroll
     for (int vw = 0; vw < 8; vw++) {  // the reference's eight warps of four elements a thread
         const uint32_t g0 = base + 128u * vw + 4u * lane;
-        const int valid = g0 < a.nfield ? (int)min(4u, a.nfield - g0) : 0;
-        float4 d = deltas4<ZZ>(load4(GlobalCodes{a.codes}, g0, valid, valid != 4 ? 2 : mode));
-        if ((rows >> vw) & 1u) d = with_outliers(d, a, g0, valid);
-        float v[4] = {d.x, d.y, d.z, d.w};
+        float v[4] = {next.x, next.y, next.z, next.w};
+        if (vw < 7) next = deltas(vw + 1);  // loaded before this step's stores
 #pragma unroll
         for (int i = 1; i < 4; i++) v[i] = __fadd_rn(v[i], v[i - 1]);
         float ts = v[3];
@@ -251,12 +258,43 @@ __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid
     }
 }
 
+// The outliers of a lane with many: whole rows of eight at out + step * i, those
+// flagged in byte i of m kept (VEC: by 16-byte loads), to p + pitch * i.
+template <int ROWS, bool VEC>
+__device__ __noinline__ void stage_rows(const float* out, uint32_t step, uint64_t m, float* p,
+                                        uint32_t pitch) {
+#pragma unroll
+    for (int i = 0; i < ROWS; i++) {
+        const uint32_t b = (uint32_t)(m >> (8 * i)) & 0xffu;
+        const float* o = out + i * step;
+        float v[8];
+        if (VEC) {
+            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            const float4 l = (b & 15u) ? __ldcg(reinterpret_cast<const float4*>(o)) : zero;
+            const float4 h = (b >> 4) ? __ldcg(reinterpret_cast<const float4*>(o) + 1) : zero;
+            v[0] = l.x, v[1] = l.y, v[2] = l.z, v[3] = l.w, v[4] = h.x, v[5] = h.y, v[6] = h.z, v[7] = h.w;
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = (b >> k) & 1u ? v[k] : 0.0f;
+        } else {
+#pragma unroll
+            for (int k = 0; k < 8; k++) v[k] = (b >> k) & 1u ? __ldcg(o + k) : 0.0f;
+        }
+        if (b) {
+            *reinterpret_cast<float4*>(p + pitch * i) = make_float4(v[0], v[1], v[2], v[3]);
+            *reinterpret_cast<float4*>(p + pitch * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
+        }
+    }
+}
+
 // Places the outliers of this lane's rows into its own part of the shared tile:
 // row i's eight floats at p + pitch * i, written for the rows flagged in `rows`
 // only.  The bitmap words and then the values of all rows are in flight
 // together (their latencies one after another were most of the time of a field
-// with 0.8 % outliers).
-template <int ROWS>
+// with 0.8 % outliers).  In 3-D, where a lane has more than kFewOutliers,
+// the warp loads whole rows instead (500 x 500 x 100 with 12 % outliers 163 us for the
+// inverse, now 132; in 2-D the call cost registers).  VEC: the output's rows start on
+// 16-byte boundaries.
+template <int ROWS, bool VEC>
 __device__ __forceinline__ void stage_outliers(const InvArgs& a, uint32_t g0, uint32_t step, int valid, uint32_t rows,
                                                float* p, uint32_t pitch) {
     uint64_t m = 0;
@@ -267,6 +305,10 @@ __device__ __forceinline__ void stage_outliers(const InvArgs& a, uint32_t g0, ui
             *reinterpret_cast<float4*>(p + pitch * i) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
             *reinterpret_cast<float4*>(p + pitch * i + 4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
+    }
+    if (ROWS == 8 && __any_sync(0xffffffffu, __popcll(m) > kFewOutliers)) {
+        stage_rows<ROWS, VEC>(a.out + g0, step, m, p, pitch);
+        return;
     }
     while (__any_sync(0xffffffffu, m != 0)) {
         float v[4];
@@ -321,7 +363,7 @@ __device__ __noinline__ void exact_tile_2d(const InvArgs& a, float* strip, uint3
     const uint32_t g0 = (y0 + r) * a.nx + x;
     float* mine = strip + 36u * r + 8u * (lane & 3u);
     const uint32_t lrows = lane_rows(rows, r);
-    if (rows) stage_outliers<4>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
+    if (rows) stage_outliers<4, false>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         uint32_t w[4];
@@ -444,7 +486,7 @@ __global__ void __launch_bounds__(32 * kWarps)
         }
         float* mine = strip + 36u * r + 8u * c;
         const uint32_t lrows = lane_rows(rows, r);
-        if (rows) stage_outliers<4>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
+        if (rows) stage_outliers<4, false>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             float4 lo, hi;
@@ -548,7 +590,7 @@ __global__ void __launch_bounds__(32 * kWarps)
             }
         }
         float* p = brick + 260u * z + 8u * c;
-        if (__any_sync(full, rows != 0u)) stage_outliers<8>(a, g0, a.nx, nvz, rows, p, 32u);
+        if (__any_sync(full, rows != 0u)) stage_outliers<8, AL>(a, g0, a.nx, nvz, rows, p, 32u);
         if (!exact) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
@@ -622,30 +664,46 @@ __global__ void __launch_bounds__(32 * kWarps)
 __global__ void mark_outliers_kernel(InvArgs a) {
     follow();
     if (inv_gated_off(a)) return;
-    const uint32_t n = min(*a.out_count, a.cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = a.out_idx[i];
-        if (k >= a.n_total) continue;
-        const float o = a.out_err[i];
-        a.out[k] = o;
-        if (k >= a.nfield) continue;
-        atomicOr(a.obits + (k >> 5), 1u << (k & 31u));
-        uint32_t tile, row;
-        if (a.nz > 1) {
-            const uint32_t z = k / a.plane, r = k - z * a.plane, y = r / a.nx, x = r - y * a.nx;
-            tile = ((z >> 3) * ((a.ny + 7u) >> 3) + (y >> 3)) * ((a.nx + 7u) >> 3) + (x >> 3);
-            row = 8u * (z & 7u) + (y & 7u);
-        } else if (a.ny > 1) {
-            const uint32_t y = k / a.nx, x = k - y * a.nx;
-            tile = (y >> 5) * ((a.nx + 31u) >> 5) + (x >> 5);
-            row = y & 31u;
-        } else {
-            tile = k >> 10;
-            row = (k >> 7) & 7u;
+    const uint32_t n = min(*a.out_count, a.cap), lane = threadIdx.x & 31u, full = 0xffffffffu;
+    for (uint32_t i0 = blockIdx.x * blockDim.x + threadIdx.x - lane; i0 < n; i0 += gridDim.x * blockDim.x) {
+        const uint32_t i = i0 + lane, k = i < n ? a.out_idx[i] : a.n_total;
+        const float o = i < n ? a.out_err[i] : 0.0f;
+        if (k < a.n_total) a.out[k] = o;
+        const bool in = k < a.nfield;
+        uint32_t tile = 0xffffffffu, row = 0;
+        if (in) {
+            if (a.nz > 1) {
+                const uint32_t z = k / a.plane, r = k - z * a.plane, y = r / a.nx, x = r - y * a.nx;
+                tile = ((z >> 3) * ((a.ny + 7u) >> 3) + (y >> 3)) * ((a.nx + 7u) >> 3) + (x >> 3);
+                row = 8u * (z & 7u) + (y & 7u);
+            } else if (a.ny > 1) {
+                const uint32_t y = k / a.nx, x = k - y * a.nx;
+                tile = (y >> 5) * ((a.nx + 31u) >> 5) + (x >> 5);
+                row = y & 31u;
+            } else {
+                tile = k >> 10;
+                row = (k >> 7) & 7u;
+            }
         }
-        const bool whole = fabsf(o) <= kIntSum && truncf(o) == o;  // false for NaN
-        atomicAdd(reinterpret_cast<float*>(a.otiles + 3u * tile), whole ? fabsf(o) : __int_as_float(0x7f800000));
-        atomicOr(a.otiles + 3u * tile + 1 + (row >> 5), 1u << (row & 31u));
+        // runs of lanes whose outliers are in one tile row add up first (a sorted list of
+        // many a tile: every one by itself took 21 us for 16.8 M values with 4 %)
+        const uint32_t before = __shfl_up_sync(full, tile, 1), brow = __shfl_up_sync(full, row, 1);
+        const uint32_t heads = __ballot_sync(full, lane == 0 || before != tile || brow != row);
+        const uint32_t later = lane < 31 ? heads >> (lane + 1) : 0u;
+        const uint32_t end = later ? lane + (uint32_t)__ffs(later) : 32u;  // the run's last lane + 1
+        const bool whole = fabsf(o) <= kIntSum && truncf(o) == o;          // false for NaN
+        uint32_t sum = in ? (whole ? (uint32_t)fabsf(o) : 1u << 25) : 0u;   // 2^25: past exactness
+#pragma unroll
+        for (uint32_t d = 1; d < 32; d <<= 1) {
+            const uint32_t s = __shfl_down_sync(full, sum, d);
+            if (lane + d < end) sum += s;
+        }
+        if (!in) continue;
+        atomicOr(a.obits + (k >> 5), 1u << (k & 31u));
+        if ((heads >> lane) & 1u) {
+            atomicAdd(reinterpret_cast<float*>(a.otiles + 3u * tile), (float)sum);
+            atomicOr(a.otiles + 3u * tile + 1 + (row >> 5), 1u << (row & 31u));
+        }
     }
 }
 

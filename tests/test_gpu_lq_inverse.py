@@ -127,3 +127,18 @@ def test_large_outliers_cost_little_more(cuda, dims):
     t = least(50000), least(1 << 25)
     print("us a call", [100 * v for v in t])
     assert t[1] < 2 * t[0]
+
+
+@pytest.mark.parametrize("dims", [(2000, 1, 1), (100, 70, 1), (101, 66, 1), (40, 33, 19), (41, 33, 19)])
+@pytest.mark.parametrize("size", [60000.0, 2.0 ** 25])
+def test_many_outliers(cuda, dims, size):
+    """Every second element an outlier, listed in order and not, with a repeat."""
+    n = int(np.prod(dims))
+    rng = np.random.default_rng(n)
+    idx = np.sort(rng.choice(n, n // 2, replace=False)).astype(np.uint32)
+    err = rng.integers(-size, size, idx.size).astype(np.float32)
+    codes = np.zeros(n, np.uint16)
+    _run(cuda, dims, codes, err, idx, True, 0)
+    order = rng.permutation(idx.size)
+    _run(cuda, dims, codes, err[order], idx[order], True, 1)
+    _run(cuda, dims, codes, np.append(err, err[-1]), np.append(idx, idx[-1]), False, 0)
