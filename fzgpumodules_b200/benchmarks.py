@@ -237,12 +237,22 @@ def _slab_field(f) -> bool:
             and f["x"].numel() == nx * ny * nz)
 
 
+def _walked_field(f) -> bool:
+    """Whether a 2-D or 3-D field fills so little of its tiles that it is walked by elements."""
+    nx, ny, nz = f["dims"]
+    t = 32 if nz == 1 else 8
+    cap = -(-nx // t) * t * (-(-ny // t) * t) * (1 if nz == 1 else -(-nz // t) * t)
+    return 16 * nx * ny * nz <= (9 if nz == 1 else 6) * cap
+
+
 def _batch_launches(fields) -> int:
     """Reset, value base and the two assembly kernels, a slab kernel per slab field, the
-    1-D chunk kernel, the tile and chunk kernels of the other 2-D and 3-D fields."""
+    1-D chunk kernel, the chunk kernel of the other 2-D and 3-D fields and the one or two
+    for their codes."""
     slab = [_slab_field(f) for f in fields]
     flat = [f["dims"][1] * f["dims"][2] == 1 for f in fields]
-    return 4 + sum(slab) + any(flat) + 2 * any(not a and not b for a, b in zip(slab, flat))
+    rest = [_walked_field(f) for f, a, b in zip(fields, slab, flat) if not a and not b]
+    return 4 + sum(slab) + any(flat) + bool(rest) + len(set(rest))
 
 
 def batch_summary(dev, steps: int, warmup: int) -> dict:

@@ -954,7 +954,7 @@ struct BatchPlan {
     BatchArgs args;
     uint32_t mm_grid_x;
     unsigned lq_grid;
-    uint32_t tile_blocks;
+    uint32_t tile_blocks, cell_blocks;
     std::vector<FwdArgs> slab;  // fields coded by a slab kernel (host copies of their arguments)
     unsigned sms = 148;
 };
@@ -1062,20 +1062,22 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
             mm_grid = std::max(mm_grid, 1 + std::min(b.a.obits_words / 4096u, 592u));
         }
     }
-    // field order of the unit ranges: the chunk kernels' fields first (1-D, then
-    // the others, in the tuned order), the slab kernels' fields after them
+    // field order of the unit ranges: the chunk kernels' fields first (1-D, then the
+    // others by tiles and those by elements, in the tuned order), the slab kernels'
+    // fields after them
     std::vector<uint32_t> order((size_t)nfields), begin((size_t)nfields), tiles((size_t)nfields);
     for (int i = 0; i < nfields; i++) order[i] = (uint32_t)i;
     if (tuning && tuning->order == 1)
         std::stable_sort(order.begin(), order.end(),
                          [&](uint32_t x, uint32_t y) { return hf[x].n_chunks > hf[y].n_chunks; });
-    std::stable_partition(order.begin(), order.end(), [&](uint32_t x) { return !is_slab[x]; });
-    std::stable_partition(order.begin(), order.end(), [&](uint32_t x) { return hf[x].kind == 0; });
-    uint64_t units = 0, lq_units = 0, one_units = 0, blocks = 0;
+    auto rank = [&](uint32_t x) { return is_slab[x] ? 3 : hf[x].a.cells ? 2 : hf[x].kind ? 1 : 0; };
+    std::stable_sort(order.begin(), order.end(), [&](uint32_t x, uint32_t y) { return rank(x) < rank(y); });
+    uint64_t units = 0, lq_units = 0, one_units = 0, blocks = 0, tile_blocks = 0;
     for (int i = 0; i < nfields; i++) {
         begin[i] = (uint32_t)units;
         tiles[i] = (uint32_t)blocks;
         if (hf[order[i]].a.obits) blocks += lq_tile_blocks(hf[order[i]].a);
+        if (rank(order[i]) < 2) tile_blocks = blocks;
         units += hf[order[i]].n_chunks;
         if (!is_slab[order[i]]) lq_units = units;
         if (hf[order[i]].kind == 0) one_units = units;
@@ -1116,7 +1118,8 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
     // room for
     const int pairs = (tuning && tuning->ctas_per_sm > 0) ? tuning->ctas_per_sm : 2;
     p->lq_grid = (unsigned)std::min<uint64_t>(2ull * (uint64_t)pairs * (uint64_t)sms, 0x7fffffffull);
-    p->tile_blocks = (uint32_t)blocks;
+    p->tile_blocks = (uint32_t)tile_blocks;
+    p->cell_blocks = (uint32_t)(blocks - tile_blocks);
     *st = FZB_OK;
     return p;
 }
@@ -1132,7 +1135,7 @@ int fzb_batch_launch(void* batch, void* stream) {
                                                                       : launch_lq3d_slab(a, 2 * p->sms, s);
         if (rc != 0) return FZB_E_CUDA;
     }
-    return launch_batch_code(p->args, p->lq_grid, p->tile_blocks, s) == 0 ? FZB_OK : FZB_E_CUDA;
+    return launch_batch_code(p->args, p->lq_grid, p->tile_blocks, p->cell_blocks, s) == 0 ? FZB_OK : FZB_E_CUDA;
 }
 
 void fzb_batch_destroy(void* batch) { delete static_cast<BatchPlan*>(batch); }

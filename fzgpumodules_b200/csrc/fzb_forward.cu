@@ -774,11 +774,9 @@ int launch_batch_scan(const BatchArgs& b, uint32_t mm_grid_x, cudaStream_t s) {
     return (int)cudaGetLastError();
 }
 
-int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks, cudaStream_t s) {
-    if (tile_blocks) {
-        const int rc = launch_batch_tiles(b, tile_blocks, s);
-        if (rc) return rc;
-    }
+int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks, uint32_t cell_blocks, cudaStream_t s) {
+    const int rc = launch_batch_tiles(b, tile_blocks, cell_blocks, s);
+    if (rc) return rc;
     const unsigned one = b.one_units, rest = b.lq_units - b.one_units;
     if (one) lq_batch_kernel<true><<<min(lq_grid, one), kThreads, kChunkSmem, s>>>(b);
     if (rest) lq_batch_kernel<false><<<min(lq_grid, rest), kThreads, kChunkSmem, s>>>(b);

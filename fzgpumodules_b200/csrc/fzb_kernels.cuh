@@ -323,8 +323,9 @@ struct BatchArgs {
 // the first lq_units units and the assembly of every field.  Fields that take
 // a slab kernel are launched between the two.
 int launch_batch_scan(const BatchArgs& b, uint32_t mm_grid_x, cudaStream_t s);
-int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks, cudaStream_t s);
-int launch_batch_tiles(const BatchArgs& b, uint32_t blocks, cudaStream_t s);  // fzb_tiles.cu
+int launch_batch_code(const BatchArgs& b, unsigned lq_grid, uint32_t tile_blocks, uint32_t cell_blocks, cudaStream_t s);
+// fzb_tiles.cu: the first `tiles` blocks of tile_begin's numbering and the `cells` after them
+int launch_batch_tiles(const BatchArgs& b, uint32_t tiles, uint32_t cells, cudaStream_t s);
 
 // Per-chunk coding with a learned selector (fzb_select.cu).
 constexpr int kSelCodes = 32768;            // codes per 64 KiB chunk

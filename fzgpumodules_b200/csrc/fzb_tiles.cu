@@ -395,11 +395,6 @@ __device__ __forceinline__ void tile_block(const FwdArgs& a, uint32_t block, Til
     const uint32_t warp = block * kTileWarps + (threadIdx.x >> 5);
     const float r = *a.ebx2_r;
     const int modes = tile_modes(a), smode = modes >> 1;
-    if (a.cells) {
-        if (modes & 1) a.nz > 1 ? cells<3, ZZ, 4>(a, warp, r) : cells<2, ZZ, 4>(a, warp, r);
-        else a.nz > 1 ? cells<3, ZZ, 1>(a, warp, r) : cells<2, ZZ, 1>(a, warp, r);
-        return;
-    }
     if (a.nz > 1) {
         const uint32_t n = ((a.nx + 7u) / 8u) * ((a.ny + 7u) / 8u) * ((a.nz + 7u) / 8u), wt = 4u * warp;
         if (wt >= n) return;
@@ -412,6 +407,14 @@ __device__ __forceinline__ void tile_block(const FwdArgs& a, uint32_t block, Til
     }
 }
 
+template <bool ZZ>
+__device__ __forceinline__ void cells_block(const FwdArgs& a, uint32_t block) {
+    const uint32_t warp = block * kTileWarps + (threadIdx.x >> 5);
+    const float r = *a.ebx2_r;
+    if (tile_modes(a) & 1) a.nz > 1 ? cells<3, ZZ, 4>(a, warp, r) : cells<2, ZZ, 4>(a, warp, r);
+    else a.nz > 1 ? cells<3, ZZ, 1>(a, warp, r) : cells<2, ZZ, 1>(a, warp, r);
+}
+
 __global__ void __launch_bounds__(32 * kTileWarps, 8) lq_tiles_kernel(const __grid_constant__ FwdArgs a) {
     follow();
     __shared__ TileSmem sm[kTileWarps];
@@ -419,21 +422,36 @@ __global__ void __launch_bounds__(32 * kTileWarps, 8) lq_tiles_kernel(const __gr
     else tile_block<false>(a, blockIdx.x, sm[threadIdx.x >> 5]);
 }
 
+// A kernel of its own: beside the tiles' code the tiles of 501 x 500 x 99 took 3 us
+// longer.
+__global__ void __launch_bounds__(32 * kTileWarps, 8) lq_cells_kernel(const __grid_constant__ FwdArgs a) {
+    follow();
+    if (a.zigzag) cells_block<true>(a, blockIdx.x);
+    else cells_block<false>(a, blockIdx.x);
+}
+
 // The tiles of a batch's 2-D and 3-D fields (eight CTAs an SM: 127 us for twenty
-// fields of 0.96 GB, 134 with six): CTAs [tile_begin[i], tile_begin[i + 1])
-// belong to the field of slot i of unit_order.
-__global__ void __launch_bounds__(32 * kTileWarps, 8) batch_tiles_kernel(BatchArgs b) {
-    __shared__ TileSmem sm[kTileWarps];
+// fields of 0.96 GB, 134 with six), or the elements of those that take cells():
+// block b of [tile_begin[i], tile_begin[i + 1]), `first` being the grid's, belongs to
+// the field of slot i of unit_order.
+template <bool CELLS>
+__global__ void __launch_bounds__(32 * kTileWarps, 8) batch_tiles_kernel(BatchArgs b, uint32_t first) {
+    __shared__ TileSmem sm[CELLS ? 1 : kTileWarps];
     uint32_t lo = 0, hi = b.nfields;
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
-        if (b.tile_begin[mid] <= blockIdx.x) lo = mid;
+        if (b.tile_begin[mid] <= first + blockIdx.x) lo = mid;
         else hi = mid;
     }
     const FwdArgs& a = b.fields[b.unit_order[lo]].a;
-    const uint32_t block = blockIdx.x - b.tile_begin[lo];
-    if (a.zigzag) tile_block<true>(a, block, sm[threadIdx.x >> 5]);
-    else tile_block<false>(a, block, sm[threadIdx.x >> 5]);
+    const uint32_t block = first + blockIdx.x - b.tile_begin[lo];
+    if (CELLS) {
+        if (a.zigzag) cells_block<true>(a, block);
+        else cells_block<false>(a, block);
+    } else {
+        if (a.zigzag) tile_block<true>(a, block, sm[threadIdx.x >> 5]);
+        else tile_block<false>(a, block, sm[threadIdx.x >> 5]);
+    }
 }
 
 }  // namespace
@@ -452,11 +470,12 @@ uint32_t lq_tile_blocks(const FwdArgs& a) {
 }
 
 int launch_lq_tiles(const FwdArgs& a, cudaStream_t s) {
-    return (int)launch_dependent(lq_tiles_kernel, lq_tile_blocks(a), 32 * kTileWarps, 0, s, a);
+    return (int)launch_dependent(a.cells ? lq_cells_kernel : lq_tiles_kernel, lq_tile_blocks(a), 32 * kTileWarps, 0, s, a);
 }
 
-int launch_batch_tiles(const BatchArgs& b, uint32_t blocks, cudaStream_t s) {
-    batch_tiles_kernel<<<blocks, 32 * kTileWarps, 0, s>>>(b);
+int launch_batch_tiles(const BatchArgs& b, uint32_t tiles, uint32_t cells, cudaStream_t s) {
+    if (tiles) batch_tiles_kernel<false><<<tiles, 32 * kTileWarps, 0, s>>>(b, 0);
+    if (cells) batch_tiles_kernel<true><<<cells, 32 * kTileWarps, 0, s>>>(b, tiles);
     return (int)cudaGetLastError();
 }
 

@@ -397,13 +397,15 @@ int fzb_status_from_bits(uint32_t bits, int* rerun_exact);
 
 /* ------------------------------------------------------------------------
  * Batched compression of many fields (no reference counterpart: it runs the
- * chain of fzb_lq_bs_rze_compress for every field in at most seven launches --
- * reset, one value-base scan over all fields, the codes of every 2-D and 3-D
- * field, one persistent chunk kernel over the 1-D fields' chunks and one over
- * the others', two assembly kernels -- plus one slab kernel launch per field
- * the single-field call codes with a slab kernel (3-D, nx a power of two in
- * [32, 1024], whole-row chunks), so a batch is one CUDA graph node group).  Each field's outputs are
- * byte-identical to its own fzb_lq_bs_rze_compress call.
+ * chain of fzb_lq_bs_rze_compress for every field in at most eight launches --
+ * reset, one value-base scan over all fields, the codes of the 2-D and 3-D
+ * fields by tiles, those of the fields that fill little of their tiles by
+ * elements, one persistent chunk kernel over the 1-D fields' chunks and one
+ * over the others', two assembly kernels -- plus one slab kernel launch per
+ * field the single-field call codes with a slab kernel (3-D, nx a power of two
+ * in [32, 1024], whole-row chunks), so a batch is one CUDA graph node group).
+ * Each field's outputs are byte-identical to its own fzb_lq_bs_rze_compress
+ * call.
  *
  * fzb_batch_create validates the fields, writes the descriptors into
  * d_work (synchronous copy) and returns a handle; fzb_batch_launch only
