@@ -40,3 +40,37 @@ def test_rle_tile_edges(cuda, dtype):
         assert np.array_equal(enc.cpu().numpy(), ref)
         dec = K.rle_decode(enc, a.size, TDT[dtype])
         assert np.array_equal(dec.cpu().numpy().view(dtype), a)
+
+
+@pytest.mark.parametrize("n", [1024 * 1024 - 1, 4 * 1024 * 1024 + 1, 9 * 1024 * 1024 + 5])
+def test_many_tiles_of_runs(cuda, n):
+    """A thread's share of the sums' scan: one to twelve sums, the last share partial."""
+    from fzgpumodules_b200 import kernels as K
+    t = (torch.arange(n, device=cuda) % 251).to(torch.uint8)
+    enc, _ = K.rle_encode(t)
+    assert enc.numel() == 4 + (n + 3) // 4 * 4 + 4 * n
+    assert torch.equal(K.rle_decode(enc, n, torch.uint8), t)
+    t[n // 3: n // 3 + 5000] = 9
+    enc, _ = K.rle_encode(t)
+    assert torch.equal(K.rle_decode(enc, n, torch.uint8), t)
+
+
+def test_long_runs_take_no_scan_of_all_tiles(cuda):
+    """One run over the whole stream: 2^25 bytes cost less than twice 2^24 16-bit codes."""
+    from fzgpumodules_b200 import kernels as K
+
+    def least(n, dtype):
+        enc, _ = K.rle_encode(torch.zeros(n, dtype=dtype, device=cuda))
+        times = []
+        for _ in range(12):
+            e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            e0.record()
+            for _ in range(5):
+                K.rle_decode(enc, n, dtype)
+            e1.record()
+            torch.cuda.synchronize()
+            times.append(e0.elapsed_time(e1))
+        return min(times)
+    t = least(1 << 24, torch.uint16), least(1 << 25, torch.uint8)
+    print("us a call", [200 * v for v in t])
+    assert t[1] < 1.8 * t[0]
