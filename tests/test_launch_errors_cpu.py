@@ -29,8 +29,8 @@ def test_tile_launch_reports_what_the_runtime_said(tmp_path, code):
     subprocess.run(["make", "-C", CSRC, obj], check=True, capture_output=True)
     (tmp_path / "runtime.c").write_text(RUNTIME % code)
     so = str(tmp_path / f"tiles{code}.so")
-    subprocess.run(["gcc", "-w", "-shared", "-fPIC", "-o", so, str(tmp_path / "runtime.c"), os.path.join(CSRC, obj),
-                    "-lstdc++"], check=True)
+    subprocess.run(["gcc", "-w", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-o", so, str(tmp_path / "runtime.c"),
+                    os.path.join(CSRC, obj), "-lstdc++"], check=True)  # its own runtime, whatever else is loaded
     launch = C.CDLL(so)["_ZN3fzb15launch_lq_tilesERKNS_7FwdArgsEP11CUstream_st"]
     launch.restype = C.c_int
     assert launch(C.create_string_buffer(4096), None) == code  # a field of no extents
