@@ -1,8 +1,7 @@
 // fzb_common.cuh -- device helpers shared by the sm_100a hot-path kernels.
 //
-// Rounding, code mapping, block scans, the 16x16 in-register bit transpose
-// used by Bitshuffle, byte-mask helpers used by RZE, and the bounded
-// decoupled look-back used to place variable-size chunk outputs.
+// Dependent launches, rounding, code mapping, block scans, the 16x16 in-register
+// bit transpose used by Bitshuffle, and byte-mask helpers used by RZE.
 #pragma once
 
 #include <cstdint>
@@ -55,7 +54,7 @@ constexpr int kChunkCodes = kChunkBytes / 2;  // u16 codes per chunk
 constexpr int kRzeAvail = kChunkBytes - 2;    // rze_stage.cu:369
 
 // Device error word bits (workspace[0]); read by the host after the launch.
-constexpr uint32_t kErrLookbackTimeout = 1u;
+constexpr uint32_t kErrLookbackTimeout = 1u;  // reported for it; no kernel sets it
 constexpr uint32_t kErrMalformed = 2u;
 constexpr uint32_t kErrInexact = 4u;      // fused inverse left the exact-integer regime
 constexpr uint32_t kErrUnsorted = 8u;     // outlier indices not ascending
@@ -70,18 +69,7 @@ __device__ __forceinline__ float round_half_away(float v) {
     return (fabsf(d) >= 0.5f) ? __fadd_rn(t, s) : t;
 }
 
-// Code of a quantizable delta: (TCode)(int)delta or its zigzag
-// (lorenzo_quant.cu:326-334, zigzag.h:70-74).
-__device__ __forceinline__ uint32_t encode_code(float c, bool zigzag) {
-    int iv = __float2int_rz(c);
-    if (zigzag) {
-        int s = (int)(int16_t)iv;
-        return (((uint32_t)s << 1) ^ (uint32_t)(s >> 15)) & 0xffffu;
-    }
-    return (uint32_t)iv & 0xffffu;
-}
-
-// Inverse of encode_code as the dequantize kernels read it (zigzag.h:80-84).
+// Delta of a code, plain int16 or zigzag (zigzag.h:80-84).
 __device__ __forceinline__ float decode_code(uint32_t u, bool zigzag) {
     if (zigzag) {
         int s = (int)((u >> 1) ^ (0u - (u & 1u)));
@@ -162,87 +150,6 @@ __device__ __forceinline__ uint32_t nz_nibble(uint32_t w) {
 
 __device__ __forceinline__ uint32_t nz_byte_mask64(uint64_t w) {
     return nz_nibble((uint32_t)w) | (nz_nibble((uint32_t)(w >> 32)) << 4);
-}
-
-// ---------------------------------------------------------------- look-back
-//
-// One u64 status word per chunk: bits 63..62 = 0 empty, 1 aggregate,
-// 2 inclusive prefix; bits 61..0 = value.  Chunks are taken in ticket
-// order, so a chunk only ever waits on chunks whose CTAs are running or
-// done; every wait is bounded and raises kErrLookbackTimeout instead of
-// spinning forever.
-
-constexpr uint64_t kFlagAgg = 1ull << 62;
-constexpr uint64_t kFlagPre = 2ull << 62;
-constexpr uint64_t kValMask = (1ull << 62) - 1;
-constexpr int kSpinLimit = 1 << 22;
-
-__device__ __forceinline__ void lb_store(unsigned long long* p, uint64_t v) {
-    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ uint64_t lb_load(const unsigned long long* p) {
-    uint64_t v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// Called by all kThreads threads of the CTA owning `chunk`: one round trip
-// inspects 256 predecessors.  Publishes `agg`, walks back to the nearest
-// inclusive prefix, publishes this chunk's inclusive prefix and returns the
-// exclusive prefix (identical in all threads).  `red` needs 2*(kThreads/32)+2
-// u64 of shared memory.
-__device__ __noinline__ static uint64_t lookback(unsigned long long* st, uint32_t chunk,
-                                                 uint64_t agg, uint32_t* err,
-                                                 unsigned long long* red) {
-    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    constexpr int W = kThreads / 32;
-    if (chunk == 0) {
-        if (t == 0) lb_store(st, kFlagPre | agg);
-        return 0;
-    }
-    if (t == 0) lb_store(st + chunk, kFlagAgg | agg);
-    uint64_t excl = 0;
-    int64_t base = (int64_t)chunk - 1;
-    bool timed_out = false;
-    while (true) {
-        const int64_t idx = base - t;
-        uint64_t s = kFlagPre;  // positions before chunk 0 read as an empty prefix
-        if (idx >= 0) {
-            int spins = 0;
-            while (true) {
-                s = lb_load(st + idx);
-                if ((s >> 62) != 0) break;
-                if (++spins > kSpinLimit) {
-                    timed_out = true;
-                    s = kFlagPre;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-        // nearest inclusive prefix: smallest t whose status carries one
-        const uint32_t pre = __ballot_sync(0xffffffffu, (s >> 62) == 2);
-        if (lane == 0) red[warp] = pre ? (unsigned long long)(warp * 32 + __ffs(pre) - 1) : 1000ull;
-        __syncthreads();
-        unsigned long long tmin = 1000ull;
-#pragma unroll
-        for (int w = 0; w < W; w++) tmin = min(tmin, red[w]);
-        uint64_t v = ((unsigned long long)t <= tmin) ? (s & kValMask) : 0ull;
-#pragma unroll
-        for (int d = 16; d >= 1; d >>= 1) v += __shfl_xor_sync(0xffffffffu, v, d);
-        if (lane == 0) red[W + warp] = v;
-        __syncthreads();
-        uint64_t sum = 0;
-#pragma unroll
-        for (int w = 0; w < W; w++) sum += red[W + w];
-        excl += sum;
-        __syncthreads();
-        if (tmin < 1000ull) break;
-        base -= kThreads;
-    }
-    if (timed_out) atomicOr(err, kErrLookbackTimeout);
-    if (t == 0) lb_store(st + chunk, kFlagPre | ((excl + agg) & kValMask));
-    return excl;
 }
 
 }  // namespace fzb

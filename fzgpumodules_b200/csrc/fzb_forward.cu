@@ -17,8 +17,7 @@ namespace fzb {
 // device, so REL/NOA need no host round trip.
 // ---------------------------------------------------------------------------
 
-// Grid-stride min/max with eight independent 16-byte loads in flight per
-// thread; the last block to finish reduces the partials and resolves
+// Grid-stride min/max by 16-byte loads; the last block to finish reduces the partials and resolves
 // abs_eb / ebx2_r into st (lorenzo_quant.cu:612-644).  st layout:
 // [0] value_base, [1] abs_eb, [2] ebx2_r, [3] ebx2.
 __device__ __forceinline__ void resolve_eb_store(float lo, float hi, int mode, float user_eb,
@@ -54,8 +53,8 @@ __device__ __forceinline__ void minmax_body(const float* __restrict__ x, uint64_
     const float4* x4 = reinterpret_cast<const float4*>(x);
     const uint64_t stride = (uint64_t)nblk * blockDim.x;
     uint64_t i = (uint64_t)blk * blockDim.x + threadIdx.x;
-    // sixteen 16-byte loads in flight per thread, streamed past L1 with a
-    // 256-byte L2 fetch (a read-once scan)
+    // sixteen 16-byte loads an iteration, as many in flight as the registers hold,
+    // streamed past L1 with a 256-byte L2 fetch (a read-once scan)
     for (; i + 15 * stride < nv; i += 16 * stride) {
         float4 v[16];
 #pragma unroll
@@ -144,8 +143,8 @@ __device__ __forceinline__ void zero_words(uint32_t* p, uint32_t n, uint32_t tid
     for (uint32_t i = tid; i < n; i += stride) p[i] = 0u;
 }
 
-// 32 registers: seven blocks an SM, which the scan's bandwidth needs (with 72,
-// three blocks, 512^3 took 190 us instead of 85).
+// 32 registers, so that eight blocks fit an SM and the seven of the grid are all
+// resident (with 72, three blocks, 512^3 took 190 us instead of 85).
 __global__ void __launch_bounds__(256, 8) minmax_kernel(const float* __restrict__ x, uint64_t n,
                                                      float* __restrict__ pmin, float* __restrict__ pmax,
                                                      unsigned int* __restrict__ done, int mode, float user_eb,
@@ -693,7 +692,8 @@ __global__ void __launch_bounds__(kThreads, kChunkCtas) lq_chunk_kernel(FwdArgs 
 // ONE_D: the units of the 1-D fields, the first b.one_units; else the 2-D and 3-D
 // fields' units after them.  One kernel for all of them was as large as its three
 // bodies and took 519 us for twenty fields of 0.96 GB with two CTAs an SM; these
-// take 158 + 147 with four an SM (159 + 150 with five, which spill).
+// take 158 + 147 with four an SM (159 + 150 with five; at four the 1-D kernel spills 8
+// bytes of its 64 registers).
 template <bool ONE_D>
 __global__ void __launch_bounds__(kThreads, 4) lq_batch_kernel(BatchArgs b) {
     extern __shared__ float4 Q[];
@@ -1139,8 +1139,8 @@ int launch_bitshuffle_wide(const uint8_t* in, uint8_t* out, uint64_t nfull, uint
 }
 
 // ---------------------------------------------------------------------------
-// Standalone RZE encode of a byte stream (rze_stage.cu:774-843 semantics,
-// one pass: chunk encode + look-back placement).
+// Standalone RZE encode of a byte stream (rze_stage.cu:774-843 semantics): chunks to
+// their slots, from where the assembly kernels place them.
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(kThreads) rze_encode_kernel(RzeEncArgs a) {
     extern __shared__ float4 Q[];

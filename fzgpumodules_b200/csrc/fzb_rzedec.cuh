@@ -1,5 +1,6 @@
-// fzb_rzedec.cuh -- block-level RZE chunk decoder (256 threads) and the pieces
-// it shares with the inverse slab kernel (fzb_slab_inv.cu).
+// fzb_rzedec.cuh -- block-level RZE chunk decoder (256 threads), and the staging of
+// a chunk and the pairing of codes, which it shares with the inverse slab kernel
+// (fzb_slab_inv.cu; that kernel decodes the levels in its own pipeline).
 //
 // Format of a chunk: fzb_rze.cuh (modules/coders/rze/rze_stage.cu:324-445;
 // decoding :871-994).  The decoder hands thread t the sixteen words

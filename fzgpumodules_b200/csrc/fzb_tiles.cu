@@ -11,7 +11,7 @@
 // through a shared strip in both directions, so that loads and stores stay
 // coalesced.  Codes leave in 16-byte stores: for the fused chain into the
 // chunk's 16 KiB slot of the workspace, where the chunk kernel
-// (code_chunk_kernel, fzb_forward.cu) picks them up.  Outliers get the code 0
+// (lq_chunk_kernel, fzb_forward.cu) picks them up.  Outliers get the code 0
 // and a bit in a.obits; their values are recomputed there.
 //
 // Bound by HBM on large 3-D fields (4 B read, 2 B written an element) and by
@@ -415,6 +415,7 @@ __device__ __forceinline__ void cells_block(const FwdArgs& a, uint32_t block) {
     else a.nz > 1 ? cells<3, ZZ, 1>(a, warp, r) : cells<2, ZZ, 1>(a, warp, r);
 }
 
+// Eight CTAs an SM leave 64 registers, 40 bytes of which the compiler spills.
 __global__ void __launch_bounds__(32 * kTileWarps, 8) lq_tiles_kernel(const __grid_constant__ FwdArgs a) {
     follow();
     __shared__ TileSmem sm[kTileWarps];
