@@ -245,11 +245,11 @@ def _walked_field(f) -> bool:
     return 16 * nx * ny * nz <= (9 if nz == 1 else 6) * cap
 
 
-def _batch_launches(fields) -> int:
-    """Reset, value base and the two assembly kernels, a slab kernel per slab field, the
-    1-D chunk kernel, the chunk kernel of the other 2-D and 3-D fields and the one or two
-    for their codes."""
-    slab = [_slab_field(f) for f in fields]
+def _batch_launches(fields, flat_tiles: bool) -> int:
+    """Reset, value base and the two assembly kernels, a slab kernel per slab field
+    (flat_tiles: none), the 1-D chunk kernel, the chunk kernel of the other 2-D and 3-D
+    fields and the one or two for their codes."""
+    slab = [_slab_field(f) and not flat_tiles for f in fields]
     flat = [f["dims"][1] * f["dims"][2] == 1 for f in fields]
     rest = [_walked_field(f) for f, a, b in zip(fields, slab, flat) if not a and not b]
     return 4 + sum(slab) + any(flat) + bool(rest) + len(set(rest))
@@ -291,7 +291,7 @@ def batch_summary(dev, steps: int, warmup: int) -> dict:
             "plain_gbs": total / t_plain / 1e6, "speedup_vs_plain": t_plain / t_batch, "bytes_identical": same,
             "tuning": {"ctas_per_sm": best.ctas_per_sm, "order": best.order, "flat_tiles": best.flat_tiles,
                        "scan_parts": best.scan_parts}, "autotune_best_ms": tune_ms,
-            "total_bytes": total, "ratio": total / comp, "launches_per_batch": _batch_launches(fields)}
+            "total_bytes": total, "ratio": total / comp, "launches_per_batch": _batch_launches(fields, bool(best.flat_tiles))}
 
 
 def run_batch(args, dev):

@@ -434,7 +434,8 @@ typedef struct fzb_batch_field {
 } fzb_batch_field;
 
 /* Launch shape of a batch (zero fields take the defaults):
- * ctas_per_sm  pairs of CTAs per SM of the persistent chunk kernels (default 2);
+ * ctas_per_sm  pairs of CTAs per SM of the persistent chunk kernels (default 2:
+ *              four CTAs, what their registers leave room for);
  * order        1: the chunk kernel dispenses the largest fields first;
  * flat_tiles   1: slab-shaped 3-D fields go through the chunk kernel's flat
  *              8192-element chunks instead of the slab kernel's R-row x
@@ -453,7 +454,7 @@ void* fzb_batch_create(const fzb_batch_field* fields, int nfields, const fzb_bat
                        size_t work_bytes, int* status);
 int fzb_batch_launch(void* batch, void* stream);
 void fzb_batch_destroy(void* batch);
-/* Times launch shapes with CUDA events and returns the fastest: every CTAs
+/* Times launch shapes with CUDA events and returns the fastest: pairs of CTAs
  * per SM (1-3) x dispatch order, then, from the best of those, the other
  * tile shape and scan granularities 1, 2 and 8. */
 int fzb_batch_autotune(const fzb_batch_field* fields, int nfields, void* d_work, size_t work_bytes, void* stream,
