@@ -134,4 +134,4 @@ def test_absolute_bound_costs_no_more_than_a_scan(cuda):
             times.append(e0.elapsed_time(e1))
         b.close()
         return min(times)
-    assert least(K().ABS) < least(K().REL)
+    assert least(K().ABS) < 1.1 * least(K().REL)  # 0.87; 1.28 with one block a bitmap

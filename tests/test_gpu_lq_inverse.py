@@ -99,7 +99,7 @@ def test_outlier_sum_of_a_flat_tile_is_counted_once(cuda):
         return min(times)
     t = least(400000), least(600000)
     print("us a call", [1e3 * v / 5 for v in t])
-    assert t[1] < 1.2 * t[0]
+    assert t[1] < 1.5 * t[0]  # 1.0; 2.0 when each lane counted it
 
 
 @pytest.mark.parametrize("dims", [(200, 200, 200), (1600, 1500, 1)])
@@ -126,7 +126,7 @@ def test_large_outliers_cost_little_more(cuda, dims):
         return min(times)
     t = least(50000), least(1 << 25)
     print("us a call", [100 * v for v in t])
-    assert t[1] < 2 * t[0]
+    assert t[1] < 2 * t[0]  # 1.0 to 1.15; 5.7 in 3-D code by code
 
 
 @pytest.mark.parametrize("dims", [(2000, 1, 1), (100, 70, 1), (101, 66, 1), (40, 33, 19), (41, 33, 19)])

@@ -56,7 +56,7 @@ def test_many_tiles_of_runs(cuda, n):
 
 
 def test_long_runs_take_no_scan_of_all_tiles(cuda):
-    """One run over the whole stream: 2^25 bytes cost less than twice 2^24 16-bit codes."""
+    """One run over the whole stream: 2^25 bytes cost little more than 2^24 16-bit codes."""
     from fzgpumodules_b200 import kernels as K
 
     def least(n, dtype):
@@ -73,4 +73,4 @@ def test_long_runs_take_no_scan_of_all_tiles(cuda):
         return min(times)
     t = least(1 << 24, torch.uint16), least(1 << 25, torch.uint8)
     print("us a call", [200 * v for v in t])
-    assert t[1] < 1.8 * t[0]
+    assert t[1] < 1.85 * t[0]  # 1.6; 2.1 with a scan of all tiles
