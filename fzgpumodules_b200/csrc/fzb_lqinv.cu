@@ -44,7 +44,7 @@ namespace {
 
 constexpr float kIntSum = 16777216.0f;      // 2^24
 constexpr float kSumSlack = 16700000.0f;    // a rounded sum of 1024 magnitudes below this is below 2^24
-constexpr int kFewOutliers = 8;             // a lane's outliers loaded one by one
+constexpr int kFewOutliers = 128;           // outliers of a warp's 2048 elements loaded one by one
 constexpr int kWarps = 4;                   // warps a CTA
 
 // The field's codes as load4 / load8 read them.
@@ -258,45 +258,37 @@ __global__ void __launch_bounds__(32 * kWarps) lq_inverse_1d_kernel(const __grid
     }
 }
 
-// The outliers of a lane with many: whole rows of eight at out + step * i, those
-// flagged in byte i of m kept (VEC: by 16-byte loads), to p + pitch * i.
-template <int ROWS, bool VEC>
-__device__ __noinline__ void stage_rows(const float* out, uint32_t step, uint64_t m, float* p,
-                                        uint32_t pitch) {
-#pragma unroll
-    for (int i = 0; i < ROWS; i++) {
-        const uint32_t b = (uint32_t)(m >> (8 * i)) & 0xffu;
-        const float* o = out + i * step;
+// The outliers of four 3-D tiles with many: a lane a column, row after row, so that a
+// load takes a line of the field and not eight floats of each of 32 rows.  m: byte y
+// flags those of row y of the lane's plane and tile (plane lane / 4, tile lane % 4);
+// out: the lane's tile's first element.
+__device__ __noinline__ void stage_columns(const float* out, uint32_t nx, uint32_t plane, uint64_t m, float* brick) {
+    const uint32_t lane = threadIdx.x & 31u, full = 0xffffffffu, t = lane >> 3, x = lane & 7u;
+    const float* col = reinterpret_cast<const float*>(__shfl_sync(full, reinterpret_cast<uint64_t>(out), t)) + x;
+    __syncwarp();  // the rows' zeros are in place
+    for (uint32_t z = 0; z < 8; z++, col += plane) {
+        const uint32_t lo = __shfl_sync(full, (uint32_t)m, 4 * z + t) >> x,
+                       hi = __shfl_sync(full, (uint32_t)(m >> 32), 4 * z + t) >> x;
         float v[8];
-        if (VEC) {
-            const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            const float4 l = (b & 15u) ? __ldcg(reinterpret_cast<const float4*>(o)) : zero;
-            const float4 h = (b >> 4) ? __ldcg(reinterpret_cast<const float4*>(o) + 1) : zero;
-            v[0] = l.x, v[1] = l.y, v[2] = l.z, v[3] = l.w, v[4] = h.x, v[5] = h.y, v[6] = h.z, v[7] = h.w;
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = (b >> k) & 1u ? v[k] : 0.0f;
-        } else {
+        for (uint32_t y = 0; y < 8; y++) v[y] = ((y < 4 ? lo : hi) >> (8u * (y & 3u))) & 1u ? __ldcg(col + y * nx) : 0.0f;
 #pragma unroll
-            for (int k = 0; k < 8; k++) v[k] = (b >> k) & 1u ? __ldcg(o + k) : 0.0f;
-        }
-        if (b) {
-            *reinterpret_cast<float4*>(p + pitch * i) = make_float4(v[0], v[1], v[2], v[3]);
-            *reinterpret_cast<float4*>(p + pitch * i + 4) = make_float4(v[4], v[5], v[6], v[7]);
-        }
+        for (uint32_t y = 0; y < 8; y++) brick[260u * z + 32u * y + lane] = v[y];
     }
+    __syncwarp();
 }
 
 // Places the outliers of this lane's rows into its own part of the shared tile:
 // row i's eight floats at p + pitch * i, written for the rows flagged in `rows`
 // only.  The bitmap words and then the values of all rows are in flight
 // together (their latencies one after another were most of the time of a field
-// with 0.8 % outliers).  In 3-D, where a lane has more than kFewOutliers,
-// the warp loads whole rows instead (500 x 500 x 100 with 12 % outliers 163 us for the
-// inverse, now 132; in 2-D the call cost registers).  VEC: the output's rows start on
-// 16-byte boundaries.
-template <int ROWS, bool VEC>
-__device__ __forceinline__ void stage_outliers(const InvArgs& a, uint32_t g0, uint32_t step, int valid, uint32_t rows,
-                                               float* p, uint32_t pitch) {
+// with 0.8 % outliers).  In 3-D, where a warp has more than kFewOutliers, it loads
+// none and returns their bits, for stage_columns (500 x 500 x 100 with 12 % outliers
+// 163 us for the inverse, now 105, but 91 instead of 84 with 3 % by columns; in 2-D such
+// a call cost registers).
+template <int ROWS>
+__device__ __forceinline__ uint64_t stage_outliers(const InvArgs& a, uint32_t g0, uint32_t step, int valid,
+                                                   uint32_t rows, float* p, uint32_t pitch) {
     uint64_t m = 0;
 #pragma unroll
     for (int i = 0; i < ROWS; i++) {
@@ -306,10 +298,7 @@ __device__ __forceinline__ void stage_outliers(const InvArgs& a, uint32_t g0, ui
             *reinterpret_cast<float4*>(p + pitch * i + 4) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         }
     }
-    if (ROWS == 8 && __any_sync(0xffffffffu, __popcll(m) > kFewOutliers)) {
-        stage_rows<ROWS, VEC>(a.out + g0, step, m, p, pitch);
-        return;
-    }
+    if (ROWS == 8 && __reduce_add_sync(0xffffffffu, __popcll(m)) > kFewOutliers) return m;
     while (__any_sync(0xffffffffu, m != 0)) {
         float v[4];
         int at[4];
@@ -323,6 +312,7 @@ __device__ __forceinline__ void stage_outliers(const InvArgs& a, uint32_t g0, ui
         for (int k = 0; k < 4; k++)
             if (at[k] >= 0) p[pitch * (at[k] >> 3) + (at[k] & 7)] = v[k];
     }
+    return 0;
 }
 
 // Bit k: row r + 8k of a 2-D tile holds outliers.
@@ -363,7 +353,7 @@ __device__ __noinline__ void exact_tile_2d(const InvArgs& a, float* strip, uint3
     const uint32_t g0 = (y0 + r) * a.nx + x;
     float* mine = strip + 36u * r + 8u * (lane & 3u);
     const uint32_t lrows = lane_rows(rows, r);
-    if (rows) stage_outliers<4, false>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
+    if (rows) stage_outliers<4>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
 #pragma unroll
     for (int k = 0; k < 4; k++) {
         uint32_t w[4];
@@ -486,7 +476,7 @@ __global__ void __launch_bounds__(32 * kWarps)
         }
         float* mine = strip + 36u * r + 8u * c;
         const uint32_t lrows = lane_rows(rows, r);
-        if (rows) stage_outliers<4, false>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
+        if (rows) stage_outliers<4>(a, g0, 8u * a.nx, nv, lrows, mine, 36u * 8u);
 #pragma unroll
         for (int k = 0; k < 4; k++) {
             float4 lo, hi;
@@ -590,7 +580,10 @@ __global__ void __launch_bounds__(32 * kWarps)
             }
         }
         float* p = brick + 260u * z + 8u * c;
-        if (__any_sync(full, rows != 0u)) stage_outliers<8, AL>(a, g0, a.nx, nvz, rows, p, 32u);
+        if (__any_sync(full, rows != 0u)) {
+            const uint64_t many = stage_outliers<8>(a, g0, a.nx, nvz, rows, p, 32u);
+            if (__any_sync(full, many != 0)) stage_columns(a.out + base, a.nx, a.plane, many, brick);
+        }
         if (!exact) {
 #pragma unroll
             for (int i = 0; i < 8; i++) {
