@@ -10,7 +10,7 @@
 
 #include <cuda_runtime.h>
 
-#ifdef __CUDACC__
+#ifdef __CUDA_ARCH__
 #define FZB_UNROLL _Pragma("unroll")
 #else
 #define FZB_UNROLL
